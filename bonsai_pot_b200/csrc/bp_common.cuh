@@ -53,6 +53,7 @@ struct bp_attn_ctx {
   __half *stage_q, *stage_k, *stage_v, *stage_out, *stage_wq, *stage_wk;
   uint32_t stage_rows;
   cudaStream_t host_stream;
+  struct bp_snap_lanes* snap_lanes;  // streams and pinned buffers of large snapshot copies, or null
   uint8_t stage_w_host[2][BP_HEAD_DIM * 2];  // the norm weights last uploaded by a host-buffer call (they rarely change)
   bool stage_w_valid;
   int sm_count;

@@ -7,7 +7,10 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
+#include <mutex>
 #include <new>
+#include <thread>
 #include <vector>
 
 #include "bp_common.cuh"
@@ -228,6 +231,9 @@ __global__ void __launch_bounds__(32) hold_sm_kernel(unsigned long long ns) {
 
 extern "C" {
 
+struct bp_snap_lanes;
+static void drop_snap_lanes(bp_snap_lanes* l);
+
 const char* bp_strerror(int status) {
   switch (status) {
     case BP_OK: return "ok";
@@ -383,6 +389,7 @@ void bp_attn_destroy(bp_attn_ctx* c) {
   cudaFree(c->stage_wq);
   cudaFree(c->stage_wk);
   drop_token_graph(c);
+  drop_snap_lanes(c->snap_lanes);
   if (c->host_stream) cudaStreamDestroy(c->host_stream);
   delete c;
 }
@@ -787,6 +794,134 @@ static cudaError_t shard_copy(void* host_row0, size_t pitch, size_t col, uint8_t
   return cudaMemcpy2D(dev, width, static_cast<uint8_t*>(host_row0) + col, pitch, width, rows, cudaMemcpyHostToDevice);
 }
 
+// ---- a snapshot's rows, moved by several lanes ----
+// A copy between the device and pageable memory is bound by the host: one thread touches fresh pages and copies at
+// a few GB/s, a fifth of the link. So the payload is cut into SNAP_LANES ranges; a lane is a thread with a stream
+// and two pinned buffers of SNAP_CHUNK, whose DMA runs under the host copy of the other buffer. The lanes are made
+// by the first large snapshot and belong to the context. Payloads below SNAP_LANES_MIN (a lane then has less than
+// one chunk, and starting the threads costs more than it saves) and sharded contexts (strided rows) take plain copies.
+constexpr uint32_t SNAP_LANES = 4;
+constexpr size_t SNAP_CHUNK = 1u << 20, SNAP_LANES_MIN = 2u << 20;
+struct bp_snap_lanes {
+  std::mutex busy;
+  cudaStream_t stream[SNAP_LANES] = {};
+  cudaEvent_t done[SNAP_LANES][2] = {};
+  uint8_t* pinned[SNAP_LANES][2] = {};
+};
+
+static void drop_snap_lanes(bp_snap_lanes* l) {
+  if (!l) return;
+  for (uint32_t t = 0; t < SNAP_LANES; t++) {
+    if (l->stream[t]) cudaStreamDestroy(l->stream[t]);
+    for (int i = 0; i < 2; i++) {
+      if (l->done[t][i]) cudaEventDestroy(l->done[t][i]);
+      if (l->pinned[t][i]) cudaFreeHost(l->pinned[t][i]);
+    }
+  }
+  delete l;
+}
+static bp_snap_lanes* make_snap_lanes() {
+  bp_snap_lanes* l = new (std::nothrow) bp_snap_lanes();
+  bool ok = l != nullptr;
+  for (uint32_t t = 0; ok && t < SNAP_LANES; t++) {
+    ok = cudaStreamCreateWithFlags(&l->stream[t], cudaStreamNonBlocking) == cudaSuccess;
+    for (int i = 0; ok && i < 2; i++)
+      ok = cudaEventCreateWithFlags(&l->done[t][i], cudaEventDisableTiming) == cudaSuccess &&
+           cudaMallocHost(&l->pinned[t][i], SNAP_CHUNK) == cudaSuccess;
+  }
+  if (ok) return l;
+  (void)cudaGetLastError();  // no lanes (no pinned memory left): plain copies
+  drop_snap_lanes(l);
+  return nullptr;
+}
+
+// Payload bytes [at, at + len) between the cache and `pin`, in as many copies as sections they span.
+static cudaError_t snap_pieces(bp_attn_ctx* c, uint32_t pos, uint64_t at, size_t len, uint8_t* pin, cudaStream_t s, bool to_host) {
+  const uint64_t d_layer = static_cast<uint64_t>(pos) * c->nb * 4u, q_layer = static_cast<uint64_t>(pos) * c->kv_dim;
+  while (len != 0) {
+    const uint64_t idx = at / (d_layer + q_layer), r = at % (d_layer + q_layer);
+    const uint32_t kind = static_cast<uint32_t>(idx / c->cfg.n_layer), il = static_cast<uint32_t>(idx % c->cfg.n_layer);
+    const bool scales = r < d_layer;
+    uint8_t* dev = c->kv[kind] + (scales ? bp_d_off(c, il) + r : bp_qs_off(c, il) + (r - d_layer));
+    const size_t n = static_cast<size_t>(std::min<uint64_t>(len, (scales ? d_layer : d_layer + q_layer) - r));
+    const cudaError_t e = to_host ? cudaMemcpyAsync(pin, dev, n, cudaMemcpyDeviceToHost, s) : cudaMemcpyAsync(dev, pin, n, cudaMemcpyHostToDevice, s);
+    if (e != cudaSuccess) return e;
+    at += n;
+    pin += n;
+    len -= n;
+  }
+  return cudaSuccess;
+}
+
+static cudaError_t snap_lane(bp_attn_ctx* c, bp_snap_lanes* l, uint32_t t, uint8_t* payload, uint32_t pos, uint64_t at, uint64_t end, bool to_host) {
+  cudaError_t e = cudaSetDevice(c->cfg.device);
+  cudaStream_t s = l->stream[t];
+  uint64_t before = at;   // to_host: the chunk whose DMA was requested last
+  size_t before_len = 0;
+  for (uint32_t i = 0; e == cudaSuccess && (at < end || before_len != 0); i++) {
+    const size_t len = static_cast<size_t>(std::min<uint64_t>(SNAP_CHUNK, end - at));
+    if (to_host) {
+      if (len != 0) {
+        e = snap_pieces(c, pos, at, len, l->pinned[t][i & 1], s, true);
+        if (e == cudaSuccess) e = cudaEventRecord(l->done[t][i & 1], s);
+      }
+      if (e == cudaSuccess && before_len != 0) {
+        e = cudaEventSynchronize(l->done[t][(i & 1) ^ 1]);
+        if (e == cudaSuccess) memcpy(payload + before, l->pinned[t][(i & 1) ^ 1], before_len);
+      }
+      before = at;
+      before_len = len;
+    } else {
+      if (i >= 2) e = cudaEventSynchronize(l->done[t][i & 1]);
+      if (e == cudaSuccess) {
+        memcpy(l->pinned[t][i & 1], payload + at, len);
+        e = snap_pieces(c, pos, at, len, l->pinned[t][i & 1], s, false);
+      }
+      if (e == cudaSuccess) e = cudaEventRecord(l->done[t][i & 1], s);
+    }
+    at += len;
+  }
+  const cudaError_t e_end = cudaStreamSynchronize(s);  // always: no copy may still use the buffers
+  return e != cudaSuccess ? e : e_end;
+}
+
+// All rows [0, pos) between the cache and `payload` (a context that holds every head). *done false: not taken.
+static cudaError_t snap_transfer(bp_attn_ctx* c, uint8_t* payload, uint32_t pos, bool to_host, bool* done) {
+  *done = false;
+  const uint64_t bytes = bp_snapshot_payload_bytes(c->cfg.n_layer, c->kv_dim, pos);
+  if (c->cfg.n_shards != 1 || bytes < SNAP_LANES_MIN) return cudaSuccess;
+  static std::mutex making;
+  {
+    std::lock_guard<std::mutex> g(making);
+    if (!c->snap_lanes) c->snap_lanes = make_snap_lanes();
+  }
+  bp_snap_lanes* l = c->snap_lanes;
+  if (!l) return cudaSuccess;
+  std::lock_guard<std::mutex> g(l->busy);
+  // Ordered as a plain copy on the default stream is: behind what the blocking streams hold.
+  cudaError_t e = cudaEventRecord(l->done[0][0], cudaStreamLegacy);
+  if (e == cudaSuccess) e = cudaEventSynchronize(l->done[0][0]);
+  if (e != cudaSuccess) return e;
+  const uint64_t per = ((bytes + SNAP_LANES - 1) / SNAP_LANES + 4095u) & ~static_cast<uint64_t>(4095u);
+  cudaError_t st[SNAP_LANES] = {};
+  std::thread th[SNAP_LANES];
+  auto lane = [&](uint32_t t) { st[t] = snap_lane(c, l, t, payload, pos, std::min<uint64_t>(bytes, t * per), std::min<uint64_t>(bytes, (t + 1) * per), to_host); };
+  for (uint32_t t = 1; t < SNAP_LANES; t++) {
+    try {
+      th[t] = std::thread(lane, t);
+    } catch (...) {  // no thread to be had: this one does the lane
+      lane(t);
+    }
+  }
+  lane(0);
+  for (uint32_t t = 1; t < SNAP_LANES; t++)
+    if (th[t].joinable()) th[t].join();
+  for (cudaError_t x : st)
+    if (x != cudaSuccess) e = x;
+  *done = e == cudaSuccess;
+  return e;
+}
+
 int bp_snapshot_capture(bp_attn_ctx* c, uint32_t pos, void* blob, uint64_t blob_bytes) {
   if (int s = enter_io(c)) return s;
   if (!blob) return fail(c, BP_ERR_NULL, "null pointer argument");
@@ -800,7 +935,9 @@ int bp_snapshot_capture(bp_attn_ctx* c, uint32_t pos, void* blob, uint64_t blob_
   memcpy(b + 8, hdr, 24);
   if (pos == 0) return BP_OK;
   uint8_t* payload = b + SNAP_HEADER;
-  for (uint32_t kind = 0; kind < 2; kind++) {
+  bool done = false;
+  BP_CUDA(c, snap_transfer(c, payload, pos, true, &done));
+  for (uint32_t kind = 0; kind < 2 && !done; kind++) {
     for (uint32_t il = 0; il < c->cfg.n_layer; il++) {
       uint8_t* d_dst = payload + bp_snapshot_payload_offset(c->cfg.n_layer, kv_dim_g, pos, kind, il, 0);
       uint8_t* q_dst = payload + bp_snapshot_payload_offset(c->cfg.n_layer, kv_dim_g, pos, kind, il, 1);
@@ -831,7 +968,9 @@ int bp_snapshot_apply(bp_attn_ctx* c, const void* blob, uint64_t blob_bytes, uin
   if (pos > c->cfg.max_seq) return fail_overflow(c, 0, pos, c->cfg.max_seq);
   if (int s = bind_device(c)) return s;
   uint8_t* payload = const_cast<uint8_t*>(b) + SNAP_HEADER;
-  for (uint32_t kind = 0; kind < 2 && pos; kind++) {
+  bool done = false;
+  if (pos) BP_CUDA(c, snap_transfer(c, payload, pos, false, &done));
+  for (uint32_t kind = 0; kind < 2 && pos && !done; kind++) {
     for (uint32_t il = 0; il < n_layer; il++) {
       uint8_t* d_src = payload + bp_snapshot_payload_offset(n_layer, kv_dim_g, pos, kind, il, 0);
       uint8_t* q_src = payload + bp_snapshot_payload_offset(n_layer, kv_dim_g, pos, kind, il, 1);

@@ -25,19 +25,40 @@ def payload_offset(n_layer, kv_dim, pos, kind, il, sect):
     return int(_lib.load().bp_snapshot_payload_offset(n_layer, kv_dim, pos, kind, il, sect))
 
 
+def new_blob(size):
+    """An uninitialised `bytes` object and the address of its bytes, for a call that fills it: a capture then
+    touches every page of the blob once (zeroing a buffer and copying it out took longer than the transfer)."""
+    new = C.pythonapi.PyBytes_FromStringAndSize
+    new.restype, new.argtypes = C.py_object, [C.c_char_p, C.c_ssize_t]
+    address = C.pythonapi.PyBytes_AsString
+    address.restype, address.argtypes = C.c_void_p, [C.py_object]
+    blob = new(None, size)
+    return blob, address(blob)
+
+
 class KvSnapshot:
+    """Holds the whole blob (header and payload): `to_bytes` and a restore hand it on without a copy."""
+
     def __init__(self, n_layer, kv_dim, max_seq, pos, payload: bytes):
         self._n_layer, self._kv_dim, self._max_seq, self._pos = n_layer, kv_dim, max_seq, pos
-        self.payload = bytes(payload)
+        self.payload = payload
 
     pos = property(lambda self: self._pos)
     n_layer = property(lambda self: self._n_layer)
     kv_dim = property(lambda self: self._kv_dim)
     max_seq = property(lambda self: self._max_seq)
 
+    @property
+    def payload(self) -> bytes:
+        return self._blob[HEADER_BYTES:]
+
+    @payload.setter
+    def payload(self, payload):
+        self._blob = MAGIC + struct.pack("<6I", VERSION, self._n_layer, self._kv_dim, self._max_seq, self._pos, 0) + bytes(payload)
+
     def to_bytes(self) -> bytes:
         """src/kv_snapshot.rs:69-80."""
-        return MAGIC + struct.pack("<6I", VERSION, self._n_layer, self._kv_dim, self._max_seq, self._pos, 0) + self.payload
+        return self._blob
 
     @classmethod
     def from_bytes(cls, blob: bytes) -> "KvSnapshot":
@@ -53,10 +74,15 @@ class KvSnapshot:
             raise ConfigError("invalid config: KvSnapshot blob has non-zero reserved field")
         if len(blob) - HEADER_BYTES != payload_bytes(n_layer, kv_dim, pos):
             raise ConfigError("invalid config: KvSnapshot blob payload length does not match header")
-        return cls(n_layer, kv_dim, max_seq, pos, blob[HEADER_BYTES:])
+        snap = cls.__new__(cls)
+        snap._n_layer, snap._kv_dim, snap._max_seq, snap._pos = n_layer, kv_dim, max_seq, pos
+        snap._blob = bytes(blob)  # (a `bytes` is kept as it is)
+        return snap
 
     def clone(self) -> "KvSnapshot":
-        return KvSnapshot(self._n_layer, self._kv_dim, self._max_seq, self._pos, bytes(self.payload))
+        snap = KvSnapshot.__new__(KvSnapshot)
+        snap.__dict__.update(self.__dict__)
+        return snap
 
     # -- device side ---------------------------------------------------------
     @classmethod
@@ -66,10 +92,12 @@ class KvSnapshot:
         ctxs = list(ctxs) if isinstance(ctxs, (list, tuple)) else [ctxs]
         lib = _lib.load()
         size = int(lib.bp_snapshot_size(ctxs[0]._h, pos))
-        buf = (C.c_uint8 * size)()
+        blob, address = new_blob(size)
+        if ctxs[0].cfg.n_shards != 1:
+            C.memset(address, 0, size)  # a shard that is not in the list leaves its columns zero
         for ctx in ctxs:
-            ctx._check(lib.bp_snapshot_capture(ctx._h, pos, buf, size))
-        return cls.from_bytes(bytes(buf))
+            ctx._check(lib.bp_snapshot_capture(ctx._h, pos, address, size))
+        return cls.from_bytes(blob)
 
     def apply(self, ctxs) -> int:
         """`Session::restore`: validate against the context(s) and write the rows back. Returns pos."""

@@ -14,7 +14,7 @@ import numpy as np
 from . import _lib
 from .attention import AttnContext
 from .errors import raise_for_status
-from .kv_snapshot import KvSnapshot
+from .kv_snapshot import KvSnapshot, new_blob
 
 TOPK_MAX = 32  # src/model.rs:279
 
@@ -230,9 +230,9 @@ class Session:
 
     def snapshot(self) -> KvSnapshot:
         size = int(self._lib.bp_session_snapshot_size(self._h))
-        buf = (C.c_uint8 * size)()
-        self.model._check(self._lib.bp_session_snapshot(self._h, buf, size))
-        return KvSnapshot.from_bytes(bytes(buf))
+        blob, address = new_blob(size)
+        self.model._check(self._lib.bp_session_snapshot(self._h, address, size))
+        return KvSnapshot.from_bytes(blob)
 
     def restore(self, snap: KvSnapshot):
         blob = snap.to_bytes()

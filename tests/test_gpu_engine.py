@@ -399,3 +399,29 @@ def test_session_behaviour_of_the_reference_integration_tests(tmp_path):
             with pytest.raises(bp.ContextOverflow) as e:
                 s7.generate(first, greedy_opts(8))
             assert e.value.max == 10 and e.value.n == 1
+
+
+@pytest.mark.parametrize("pos", [1, 455, 456, 1021])
+def test_large_snapshots_hold_the_cache_rows(pos):
+    """Below and above the size from which a snapshot is moved by several lanes (2 MB: 456 rows here), ranges that end
+    inside a section: the blob is the cache sections in order, and restoring it brings every byte back."""
+    with bp.AttnContext(n_layer=4, n_head=16, n_kv_head=4, max_seq=1024) as ctx, bp.AttnContext(n_layer=4, n_head=16, n_kv_head=4, max_seq=1024) as other:
+        g = torch.Generator(device="cuda").manual_seed(pos)
+        w = torch.ones(128, dtype=torch.float16, device="cuda")
+        for il in range(4):
+            k, v = (torch.randn(1024, 512, generator=g, device="cuda").half() for _ in range(2))
+            ctx.dispatch_kv_writeback_fused(il, k, v, w, 0, 1024)
+        snap = bp.KvSnapshot.capture(ctx, pos)  # (ordered behind the launches on the default stream)
+
+        def sections(c):
+            for kind in range(2):
+                for il in range(4):
+                    for sect, (dt, width) in enumerate(((np.float32, 16), (np.int8, 512))):
+                        a = np.empty((pos, width), dtype=dt)
+                        c.kv_export(kind, il, sect, pos, a)
+                        yield a.tobytes()
+
+        assert snap.payload == b"".join(sections(ctx))
+        assert snap.apply(other) == pos
+        assert snap.payload == b"".join(sections(other))
+        assert bp.KvSnapshot.from_bytes(snap.to_bytes()).clone().payload == snap.payload
