@@ -401,6 +401,42 @@ def test_session_behaviour_of_the_reference_integration_tests(tmp_path):
             assert e.value.max == 10 and e.value.n == 1
 
 
+@pytest.mark.parametrize("n", [32, 33, 511, 512, 2047, 4097, 30001, 151936])
+@pytest.mark.parametrize("kind", ["distinct", "few ties", "many ties", "one list", "specials"])
+def test_topk_reduce_selects_what_the_lists_select(n, kind):
+    """Distinct logits and ties across lists take the selection, ties inside a list the heaps: the shader's
+    values and indices either way. Not a number and infinities; all candidates in one list; signed zeros."""
+    rng = np.random.default_rng(n)
+    if kind == "distinct":
+        logits = (rng.permutation(n)[:n] % 60000).astype(np.uint16).view(np.float16).copy()
+        logits[~np.isfinite(logits)] = -1
+    elif kind == "one list":  # list 3: words 3, 259, ...
+        logits = rng.standard_normal(n).astype(np.float16)
+        at = [i for i in range(n) if (i >> 1) % 256 == 3][:40]
+        logits[at] = 100 + rng.permutation(len(at)).astype(np.float16)
+    else:
+        logits = (rng.standard_normal(n) * 3).astype(np.float16)
+    if kind == "few ties":
+        logits[rng.integers(0, n, 40)] = logits.max()
+    if kind == "many ties":
+        logits = np.round(logits)
+    if kind == "specials":
+        logits[rng.integers(0, n, n // 3)] = np.nan
+        logits[rng.integers(0, n, 3)] = -np.inf
+        logits[logits > 0] = np.float16(0.0)
+        logits[rng.integers(0, n, 2)] = np.float16(-0.0)
+    pd = dev(np.concatenate([logits, np.full(2, 1000, dtype=np.float16)]))
+    for k in (1, 5, 31, 32, 40):
+        vals = torch.zeros(32, dtype=torch.float32, device="cuda")
+        idx = torch.zeros(32, dtype=torch.int32, device="cuda")
+        assert _lib.load().bp_op_topk_reduce(None, pd.data_ptr(), n, k, vals.data_ptr(), idx.data_ptr()) == 0
+        torch.cuda.synchronize()
+        want_v, want_i = E.topk_reduce(logits, k)
+        kk = min(k, 32)
+        assert np.array_equal(vals.cpu().numpy()[:kk].view(np.uint32), want_v.view(np.uint32)), k
+        assert np.array_equal(idx.cpu().numpy()[:kk].astype(np.uint32), want_i), k
+
+
 @pytest.mark.parametrize("pos", [1, 455, 456, 1021])
 def test_large_snapshots_hold_the_cache_rows(pos):
     """Below and above the size from which a snapshot is moved by several lanes (2 MB: 456 rows here), ranges that end
