@@ -974,6 +974,53 @@ __device__ __forceinline__ float tk_sift_hole(TkEntry* heap, uint32_t j, uint32_
     i = right ? r : l;
   }
   heap[i * TK_LISTS + j] = e;
+  return root;
+}
+// The same walk on a FULL heap of TK_K = 32 entries (every insertion of the scan): the levels are unrolled, no
+// slot has to be checked against a limit above the last level (only slot 15 has a child there, slot 31), and
+// the four grandchildren of a node (slots 4 i + 3 .. 4 i + 6) are requested before its children are compared:
+// a level of the walk is then compare, select, compare instead of address, load, compare, select, compare.
+template <uint32_t TK_LISTS>
+__device__ __forceinline__ float tk_sift_full(TkEntry* heap, uint32_t j, TkEntry e) {
+  static_assert(TK_K == 32, "levels and slots below are those of a heap of 32");
+  TkEntry* E = heap + j;
+  uint32_t i = 0;
+  float root = e.v;
+  TkEntry cl = E[1 * TK_LISTS], cr = E[2 * TK_LISTS];
+#pragma unroll
+  for (uint32_t lvl = 0; lvl < 4; lvl++) {
+    TkEntry g0 = {}, g1 = {}, g2 = {}, g3 = {};
+    if (lvl < 3) {
+      const TkEntry* G = E + (4 * i + 3) * TK_LISTS;
+      g0 = G[0];
+      g1 = G[TK_LISTS];
+      g2 = G[2 * TK_LISTS];
+      g3 = G[3 * TK_LISTS];
+    }
+    const bool right = cr.v < cl.v;
+    const TkEntry m = right ? cr : cl;
+    if (!(m.v < e.v)) {
+      E[i * TK_LISTS] = e;
+      return root;
+    }
+    E[i * TK_LISTS] = m;
+    if (lvl == 0) root = m.v;
+    i = 2 * i + 1 + (right ? 1u : 0u);
+    if (lvl < 3) {
+      cl = right ? g2 : g0;
+      cr = right ? g3 : g1;
+    }
+  }
+  if (i == 15) {  // the one slot of the fourth level with a child
+    const TkEntry c = E[31 * TK_LISTS];
+    if (c.v < e.v) {
+      E[15 * TK_LISTS] = c;
+      i = 31;
+    }
+  }
+  E[i * TK_LISTS] = e;
+  return root;
+}
 // The result without the lists, wherever it does not depend on them. Let T be the k-th largest value. Elements below
 // T never take a place from one that is not, so where the elements >= T end up follows from their comparisons
 // among themselves: a list with DISTINCT values >= T has them in descending order whatever its heap did, and in
@@ -1105,63 +1152,6 @@ __device__ __forceinline__ bool tk_fast(TkFast& f, TkEntry* rows, const __half* 
   return true;
 }
 
-  return root;
-}
-// The same walk on a FULL heap of TK_K = 32 entries (every insertion of the scan): the levels are unrolled, no
-// slot has to be checked against a limit above the last level (only slot 15 has a child there, slot 31), and
-// the four grandchildren of a node (slots 4 i + 3 .. 4 i + 6) are requested before its children are compared:
-// a level of the walk is then compare, select, compare instead of address, load, compare, select, compare.
-template <uint32_t TK_LISTS>
-__device__ __forceinline__ float tk_sift_full(TkEntry* heap, uint32_t j, TkEntry e) {
-  static_assert(TK_K == 32, "levels and slots below are those of a heap of 32");
-  TkEntry* E = heap + j;
-  uint32_t i = 0;
-  float root = e.v;
-  TkEntry cl = E[1 * TK_LISTS], cr = E[2 * TK_LISTS];
-#pragma unroll
-  for (uint32_t lvl = 0; lvl < 4; lvl++) {
-    TkEntry g0 = {}, g1 = {}, g2 = {}, g3 = {};
-  cluster.barrier_arrive();
-    if (lvl < 3) {
-      const TkEntry* G = E + (4 * i + 3) * TK_LISTS;
-      g0 = G[0];
-  const uint32_t kk = k < TK_K ? k : TK_K;
-  __shared__ TkFast fast;
-  if (tk_fast<TK_CTAS>(fast, rows, logits, n, kk)) {
-    if (cluster.block_rank() == 0 && tid < kk) {
-      out_val[tid] = rows[tid].v;
-      out_idx[tid] = rows[tid].i;
-    }
-    return;
-  }
-      g1 = G[TK_LISTS];
-      g2 = G[2 * TK_LISTS];
-      g3 = G[3 * TK_LISTS];
-    }
-    const bool right = cr.v < cl.v;
-    const TkEntry m = right ? cr : cl;
-    if (!(m.v < e.v)) {
-      E[i * TK_LISTS] = e;
-      return root;
-    }
-    E[i * TK_LISTS] = m;
-    if (lvl == 0) root = m.v;
-    i = 2 * i + 1 + (right ? 1u : 0u);
-    if (lvl < 3) {
-      cl = right ? g2 : g0;
-      cr = right ? g3 : g1;
-    }
-  }
-  if (i == 15) {  // the one slot of the fourth level with a child
-    const TkEntry c = E[31 * TK_LISTS];
-    if (c.v < e.v) {
-      E[15 * TK_LISTS] = c;
-      i = 31;
-    }
-  }
-  E[i * TK_LISTS] = e;
-  return root;
-}
 __device__ __forceinline__ void tk_merge_sync() { asm volatile("bar.sync 1, %0;" ::"n"(TK_WG) : "memory"); }  // the merging threads only
 // One cluster of TK_CTAS CTAs. The 256 lists of the shader are independent until its merge rounds, and what
 // a list costs is a chain of about 130 dependent sifts (375 us per call at 151936 logits with 32 lists per
@@ -1178,9 +1168,19 @@ __global__ void __launch_bounds__(TK_THREADS) topk_kernel(const __half* logits, 
   TkEntry* heap = rows + TK_WG * TK_ROW;                      // [TK_K][TK_LISTS]
   __half2* stage_all = reinterpret_cast<__half2*>(heap + TK_K * TK_LISTS);
   cg::cluster_group cluster = cg::this_cluster();
+  cluster.barrier_arrive();
   pdl_launch_dependents();
   pdl_wait();
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t kk = k < TK_K ? k : TK_K;
+  __shared__ TkFast fast;
+  if (tk_fast<TK_CTAS>(fast, rows, logits, n, kk)) {
+    if (cluster.block_rank() == 0 && tid < kk) {
+      out_val[tid] = rows[tid].v;
+      out_idx[tid] = rows[tid].i;
+    }
+    return;
+  }
   const bool owner = lane < TK_LPW;                           // this lane scans a list
   const uint32_t jl = warp * TK_LPW + (owner ? lane : 0);     // the list's slot in this CTA
   const uint32_t j0 = cluster.block_rank() * TK_LISTS + warp * TK_LPW;  // the warp's first list
