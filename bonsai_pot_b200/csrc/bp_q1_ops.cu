@@ -307,6 +307,205 @@ __global__ void __launch_bounds__(MV_THREADS) matvec_q1_kernel(const MvParams p)
     *out_ptr[0] = silu_times_up(__float2half_rn(total[0]), __float2half_rn(total[MV_ROWS_PER_LANE - 1]));
 }
 
+// The same sums with a WARP per row, lane l taking the blocks l, l + 32, ...: the f16 sum of a block does not
+// depend on the others, so the eight chains of the shader (blocks tx, tx + 8, ... in order) only have to be formed
+// from the lanes' block results, four shuffles and additions per 32 blocks. Against 8 lanes per row a row has four
+// times the threads: the 4096-row tensors fill an SM with 28 warps instead of 7, a CTA's activations are staged by
+// 448 threads instead of 128, and the chain of a lane is k / 4096 blocks instead of k / 1024. The 8-lane kernel was
+// bound by latency there (36 % of the issue slots): one-token step at the 8B shape 1288 -> 1209 us (position 100).
+constexpr uint32_t MVW_WARPS = 14;  // warps of a CTA at most
+template <int MODE, uint32_t PASSES>
+constexpr uint32_t mvw_ctas() { return MODE == 3 || PASSES > 1 ? 2 : 3; }  // CTAs per SM that the registers of an instance allow
+template <int MODE, uint32_t PASSES>
+__global__ void __launch_bounds__(MVW_WARPS * 32, mvw_ctas<MODE, PASSES>()) matvec_q1_wide_kernel(const MvParams p) {
+  static_assert(MODE == 0 || MODE == 1 || MODE == 3, "modes of matvec_q1_kernel");
+  constexpr uint32_t RP = MODE == 3 ? 2 : 1;  // rows a warp computes together (gate and up), on one read of the activations
+  extern __shared__ __align__(16) uint8_t mv_smem[];
+  __shared__ float part[4];
+  __half* xs = reinterpret_cast<__half*>(mv_smem);
+  pdl_launch_dependents();
+  const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, n_thr = blockDim.x, nb = p.k / 128u;
+  const uint32_t items = MODE == 3 ? p.r[0].n : p.n_total, step = gridDim.x * (n_thr >> 5);
+  uint4 w[PASSES][RP];
+  __half d[PASSES][RP];
+  __half* out = nullptr;
+  auto fetch = [&](uint32_t item) {  // the item's signs and scales, and where its result goes
+#pragma unroll
+    for (uint32_t j = 0; j < RP; j++) {
+      uint32_t row = item;
+      const __half* dt = p.r[j].d;
+      const uint4* bt = p.r[j].bits;
+      __half* ot = p.r[j].out;
+      if (MODE != 3 && p.n_ranges > 1 && row >= p.r[0].n) {
+        row -= p.r[0].n;
+        const bool third = p.n_ranges > 2 && row >= p.r[1].n;
+        if (third) row -= p.r[1].n;
+        dt = third ? p.r[2].d : p.r[1].d;
+        bt = third ? p.r[2].bits : p.r[1].bits;
+        ot = third ? p.r[2].out : p.r[1].out;
+      }
+      if (j == 0) out = ot + row;
+#pragma unroll
+      for (uint32_t i = 0; i < PASSES; i++) {
+        const uint32_t b = lane + 32 * i;
+        if (b < nb) {
+          w[i][j] = __ldg(bt + static_cast<size_t>(row) * nb + b);
+          d[i][j] = __ldg(dt + static_cast<size_t>(row) * nb + b);
+        }
+      }
+    }
+  };
+  uint32_t item = blockIdx.x * (n_thr >> 5) + warp;
+  if (item < items) fetch(item);  // constants: requested while the kernel before this one still runs
+  pdl_wait();
+  float old = 0.0f;
+  if (MODE == 0 && p.accumulate && item < items) old = __half2float(*out);
+  float inv_rms = 1.0f;
+  // ---- stage the activations: block b at xs + b * XB_STRIDE ----
+  if (MODE == 1 || MODE == 3) {
+    constexpr uint32_t SB = 3;
+    for (uint32_t v0 = tid; v0 < p.k / 4u; v0 += n_thr * SB) {
+      uint2 raw_q[SB], wr_q[SB];
+#pragma unroll
+      for (uint32_t u = 0; u < SB; u++) {
+        const uint32_t v = v0 + u * n_thr;
+        if (v < p.k / 4u) {
+          raw_q[u] = *reinterpret_cast<const uint2*>(p.x + 4u * v);
+          wr_q[u] = __ldg(reinterpret_cast<const uint2*>(p.aux + 4u * v));
+        }
+      }
+#pragma unroll
+      for (uint32_t u = 0; u < SB; u++) {
+        const uint32_t v = v0 + u * n_thr;
+        if (v >= p.k / 4u) break;
+        const __half2 y01 = __hmul2(*reinterpret_cast<const __half2*>(&raw_q[u].x), *reinterpret_cast<const __half2*>(&wr_q[u].x));
+        const __half2 y23 = __hmul2(*reinterpret_cast<const __half2*>(&raw_q[u].y), *reinterpret_cast<const __half2*>(&wr_q[u].y));
+        uint2 o;
+        o.x = *reinterpret_cast<const uint32_t*>(&y01);
+        o.y = *reinterpret_cast<const uint32_t*>(&y23);
+        *reinterpret_cast<uint2*>(xs + (v >> 5) * XB_STRIDE + 4u * (v & 31u)) = o;
+      }
+    }
+    if (tid < 128) {  // the sum of squares of the shader's 128 invocations
+      float ssq = 0.0f;
+      constexpr uint32_t QB = 8;
+      for (uint32_t v0 = tid; v0 < p.k / 4u; v0 += 128 * QB) {
+        uint2 raw_q[QB];
+#pragma unroll
+        for (uint32_t u = 0; u < QB; u++)
+          if (v0 + u * 128 < p.k / 4u) raw_q[u] = *reinterpret_cast<const uint2*>(p.x + 4u * (v0 + u * 128));
+#pragma unroll
+        for (uint32_t u = 0; u < QB; u++) {
+          if (v0 + u * 128 >= p.k / 4u) break;
+          const float2 f01 = __half22float2(*reinterpret_cast<const __half2*>(&raw_q[u].x)), f23 = __half22float2(*reinterpret_cast<const __half2*>(&raw_q[u].y));
+          ssq = __fadd_rn(ssq, __fmul_rn(f01.x, f01.x));
+          ssq = __fadd_rn(ssq, __fmul_rn(f01.y, f01.y));
+          ssq = __fadd_rn(ssq, __fmul_rn(f23.x, f23.x));
+          ssq = __fadd_rn(ssq, __fmul_rn(f23.y, f23.y));
+        }
+      }
+      ssq = butterfly32(ssq);
+      if (lane == 0) part[warp] = ssq;
+    }
+    __syncthreads();
+    // workgroup_sum<4>: the butterfly of (part[0 .. 3], 0, ...)
+    const float total = __fadd_rn(__fadd_rn(part[0], part[2]), __fadd_rn(part[1], part[3]));
+    inv_rms = __frsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(p.k)), p.eps));
+  } else {
+    constexpr uint32_t SB = 4;
+    for (uint32_t v0 = tid; v0 < p.k / 8u; v0 += n_thr * SB) {
+      uint4 raw_q[SB];
+#pragma unroll
+      for (uint32_t u = 0; u < SB; u++)
+        if (v0 + u * n_thr < p.k / 8u) raw_q[u] = *reinterpret_cast<const uint4*>(p.x + 8u * (v0 + u * n_thr));
+#pragma unroll
+      for (uint32_t u = 0; u < SB; u++) {
+        const uint32_t v = v0 + u * n_thr;
+        if (v < p.k / 8u) *reinterpret_cast<uint4*>(xs + (v >> 4) * XB_STRIDE + 8u * (v & 15u)) = raw_q[u];
+      }
+    }
+    __syncthreads();
+  }
+  while (item < items) {
+    float acc[RP];
+#pragma unroll
+    for (uint32_t j = 0; j < RP; j++) acc[j] = 0.0f;
+    __half* const dst = out;
+    const uint32_t next = item + step;
+#pragma unroll
+    for (uint32_t i = 0; i < PASSES; i++) {
+      const uint32_t b = lane + 32 * i;
+      const bool mine = b < nb;
+      uint4 ww[RP];
+      float dd[RP], q[RP];
+#pragma unroll
+      for (uint32_t j = 0; j < RP; j++) {
+        ww[j] = w[i][j];
+        dd[j] = __half2float(d[i][j]);
+        q[j] = 0.0f;
+      }
+      if (i + 1 == PASSES && next < items) fetch(next);  // in flight under this item's last pass
+      if (mine) {
+        __half2 a01[RP], a23[RP];
+#pragma unroll
+        for (uint32_t j = 0; j < RP; j++) a01[j] = a23[j] = __float2half2_rn(0.0f);
+        const uint4* xb = reinterpret_cast<const uint4*>(xs + b * XB_STRIDE);
+#pragma unroll
+        for (uint32_t half = 0; half < 2; half++) {  // groups 0..15, then 16..31
+#pragma unroll
+          for (uint32_t g2 = 0; g2 < 8; g2++) {      // two groups per 16-byte read
+            const uint4 xv = xb[half * 8 + g2];
+#pragma unroll
+            for (uint32_t gg = 0; gg < 2; gg++) {
+              const uint32_t g = 2 * g2 + gg;
+              const uint32_t x01 = gg ? xv.z : xv.x, x23 = gg ? xv.w : xv.y;
+#pragma unroll
+              for (uint32_t j = 0; j < RP; j++) {
+                const uint32_t w01 = half ? ww[j].y : ww[j].x, w23 = half ? ww[j].w : ww[j].z;
+                const uint32_t s01 = x01 ^ ((w01 << g) & 0x80008000u);
+                const uint32_t s23 = x23 ^ ((w23 << g) & 0x80008000u);
+                a01[j] = __hadd2(a01[j], *reinterpret_cast<const __half2*>(&s01));
+                a23[j] = __hadd2(a23[j], *reinterpret_cast<const __half2*>(&s23));
+              }
+            }
+          }
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < RP; j++) {
+          const __half ls = __hadd(__hadd(__hadd(__low2half(a01[j]), __high2half(a01[j])), __low2half(a23[j])), __high2half(a23[j]));
+          q[j] = __fmul_rn(MODE != 0 ? __fmul_rn(dd[j], inv_rms) : dd[j], __half2float(ls));
+        }
+      }
+      __syncwarp();
+#pragma unroll
+      for (uint32_t c = 0; c < 4; c++) {  // chain tx: block 32 i + 8 c + tx
+        const uint32_t from = (lane & 7u) + 8 * c;
+#pragma unroll
+        for (uint32_t j = 0; j < RP; j++) {
+          const float v = __shfl_sync(FULL, q[j], from);
+          if (32 * i + from < nb) acc[j] = __fadd_rn(acc[j], v);
+        }
+      }
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < RP; j++) {
+      float a = acc[j];
+      a = __fadd_rn(a, __shfl_xor_sync(FULL, a, 1));
+      a = __fadd_rn(a, __shfl_xor_sync(FULL, a, 2));
+      acc[j] = __fadd_rn(a, __shfl_xor_sync(FULL, a, 4));
+    }
+    if (lane == 0) {
+      if (MODE == 3) {
+        *dst = silu_times_up(__float2half_rn(acc[0]), __float2half_rn(acc[RP - 1]));
+      } else {
+        *dst = __float2half_rn(MODE == 0 && p.accumulate ? __fadd_rn(old, acc[0]) : acc[0]);
+      }
+    }
+    item = next;
+    if (MODE == 0 && p.accumulate && item < items) old = __half2float(*out);
+  }
+}
+
 // rms_norm.wgsl:41-85: one CTA of 512 threads per group.
 __global__ void __launch_bounds__(512) rms_norm_kernel(const __half* in, __half* out, const __half* w, uint32_t n, float eps) {
   __shared__ float part[32];
@@ -1316,12 +1515,52 @@ cudaError_t launch_mv_r(bool pdl, cudaStream_t s, const MvParams& p) {
   return bp_launch(pdl, matvec_q1_kernel<MODE, R, KB>, dim3(ctas), dim3(MV_THREADS), smem, s, p);
 }
 
+// CTAs of a launch of the warp-per-row kernel: the rows of an SM spread over as few warps as keep it busy (42, or 28
+// where a lane holds more than one block), those over CTAs of equal size. 4096 rows: 2 CTAs of 14 warps per SM and
+// a row per warp; 6144: 3 of 14; 12288 pairs: 2 of 14, three pairs per warp.
+template <int MODE, uint32_t PASSES>
+cudaError_t launch_mv_wide(bool pdl, cudaStream_t s, const MvParams& p) {
+  static int sms = 0;
+  if (sms == 0) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 1;
+  }
+  constexpr uint32_t MAX_WARPS = mvw_ctas<MODE, PASSES>() * MVW_WARPS;
+  const uint32_t items = MODE == 3 ? p.r[0].n : p.n_total, n_sm = static_cast<uint32_t>(sms);
+  const uint32_t per_sm = (items + n_sm - 1) / n_sm, per_warp = (per_sm + MAX_WARPS - 1) / MAX_WARPS;
+  const uint32_t warps = (per_sm + per_warp - 1) / per_warp, ctas = (warps + MVW_WARPS - 1) / MVW_WARPS;
+  uint32_t w = (warps + ctas - 1) / ctas;
+  if (w < 4) w = 4;  // (the sum of squares is that of 128 invocations)
+  const uint32_t grid = (items + w * per_warp - 1) / (w * per_warp);
+  return bp_launch(pdl, matvec_q1_wide_kernel<MODE, PASSES>, dim3(grid), dim3(32 * w), mv_smem_bytes(p.k), s, p);
+}
+// Which calls take it: rows of at least 24 blocks (below, most lanes of a warp would have none), at most 128
+// (activations that fit a CTA's default shared memory; the paired mode at most 32: a lane's blocks of both rows have
+// to fit its registers), and no more rows than the two-rows-per-lane kernel is for.
+template <int MODE>
+bool mv_wide(const MvParams& p) {
+  const uint32_t nb = p.k / 128u;
+  return nb >= 24 && nb <= (MODE == 3 ? 32u : 128u) && p.n_total < 16384;
+}
+template <int MODE>
+cudaError_t launch_mv_wide(bool pdl, cudaStream_t s, const MvParams& p) {
+  const uint32_t passes = (p.k / 128u + 31) / 32;
+  if constexpr (MODE != 3) {
+    if (passes == 2) return launch_mv_wide<MODE, 2>(pdl, s, p);
+    if (passes == 3) return launch_mv_wide<MODE, 3>(pdl, s, p);
+    if (passes == 4) return launch_mv_wide<MODE, 4>(pdl, s, p);
+  }
+  return launch_mv_wide<MODE, 1>(pdl, s, p);
+}
+
 uint32_t g_mv_rows_override = 0;  // tuning aid (bp_op_set_matvec_rows): 0 = by tensor height
 bool g_mv_const_k = true;         // tuning aid: use the constant-block-count instances where one exists
 
 template <int MODE>
 cudaError_t launch_mv(bool pdl, cudaStream_t s, const MvParams& p) {
   uint32_t r = g_mv_rows_override;
+  if constexpr (MODE == 0 || MODE == 1)
+    if (r == 0 && g_mv_const_k && mv_wide<MODE>(p)) return launch_mv_wide<MODE>(pdl, s, p);
   // measured at Bonsai-8B shapes (us per call, R = 1 / 2 / 4): 4096 rows 4.9 / 5.9 / 9.2, 6144 rows 5.8 / 6.9 / 7.6,
   // 24576 rows 12.9 / 10.6 / 10.9, 151936 rows 50 / 45 / 54
   if (r == 0) r = p.n_total >= 16384 ? 2 : 1;
@@ -1388,6 +1627,7 @@ cudaError_t bp_q1_matvec_normed_silu(bool pdl, cudaStream_t s, const bp_q1_tenso
   p.x = x;
   p.aux = w_norm;
   p.eps = eps;
+  if (g_mv_rows_override == 0 && g_mv_const_k && mv_wide<3>(p)) return launch_mv_wide<3>(pdl, s, p);
   const size_t smem = mv_smem_bytes(p.k);
   static size_t configured = 0;
   if (smem > 48 * 1024 && smem > configured) {

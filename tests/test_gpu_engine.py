@@ -461,3 +461,34 @@ def test_large_snapshots_hold_the_cache_rows(pos):
         assert snap.apply(other) == pos
         assert snap.payload == b"".join(sections(other))
         assert bp.KvSnapshot.from_bytes(snap.to_bytes()).clone().payload == snap.payload
+
+
+@pytest.mark.parametrize("k,n", [(3072, 17), (4096, 4096), (4096 + 128, 600), (8192, 15), (12288, 4096), (16384, 301), (4096, 16383)])
+def test_warp_per_row_matvec_is_identical_to_eight_lanes_per_row(k, n):
+    """The warp-per-row kernel at its limits (24 and 128 blocks, a partly filled last pass, few rows, several rows per
+    warp) against the kernel it replaces there: plain, accumulating, and the normed ranges."""
+    rng = np.random.default_rng(k * 7 + n)
+    _, _, _, d_dev, _, bits = random_q1(rng, k, n)
+    n3 = (16, 48, 16)
+    parts = [random_q1(rng, k, r) for r in n3]
+    x, w_norm = dev(rng.standard_normal(k).astype(np.float16)), dev(rng.standard_normal(k).astype(np.float16))
+    y0 = rng.standard_normal(n).astype(np.float16)
+    lib = _lib.load()
+    got = []
+    try:
+        for rows in (0, 1):
+            lib.bp_op_set_matvec_rows(rows)
+            outs = []
+            for accumulate in (0, 1):
+                y = dev(y0.copy())
+                assert lib.bp_op_matvec_q1_0(None, d_dev.data_ptr(), bits.data_ptr(), k, n, x.data_ptr(), y.data_ptr(), accumulate) == 0
+                outs.append(y)
+            normed = [torch.zeros(r, dtype=torch.float16, device="cuda") for r in n3]
+            ds, bs, os_ = ((C.c_void_p * 3)(*v) for v in ([q[3].data_ptr() for q in parts], [q[5].data_ptr() for q in parts], [t.data_ptr() for t in normed]))
+            assert lib.bp_op_matvec_q1_0_fused_normed(None, k, x.data_ptr(), w_norm.data_ptr(), 1e-6, 3, ds, bs, (C.c_uint32 * 3)(*n3), os_) == 0
+            torch.cuda.synchronize()
+            got.append([t.cpu().numpy() for t in outs + normed])
+    finally:
+        lib.bp_op_set_matvec_rows(0)
+    for a, b in zip(*got):
+        assert np.array_equal(a.view(np.uint16), b.view(np.uint16))
