@@ -273,6 +273,8 @@ struct bp_model {
          *up = nullptr, *ffn_in = nullptr, *logits = nullptr, *q_roped = nullptr;
   float* a_d = nullptr;        // Q8_0 activations: scales [m_max][n_ff / 32]
   int8_t* a_qs = nullptr;      //                  quants [m_max][n_ff]
+  uint8_t* a_tiled = nullptr;  // Q8_0 activations of a batch as the tiled product reads them
+  float* a_tiled_d = nullptr;
   uint32_t* tokens_dev = nullptr;
   float* topk_val = nullptr;
   uint32_t* topk_idx = nullptr;
@@ -526,11 +528,36 @@ int step_topk_graph(bp_model* m, uint32_t token, uint32_t pos, uint32_t k, float
   return device_status(m);
 }
 
+// y[i] (+)= W[i] q8(act): the quantiser leaves the activations the way the product for this batch reads them, and
+// takes rms_norm (norm) or silu(act) * up with it where the product is the tiled one.
 int quantize_and_matmul(bp_model* m, const __half* act, uint32_t k, uint32_t mt, const bp_q1_tensor* w, __half* const* out, uint32_t n_w,
-                        bool accumulate) {
+                        bool accumulate, const __half* norm = nullptr, const __half* up = nullptr) {
   cudaStream_t s = m->stream;
+  uint32_t* err = m->attn->err_dev;
+  const uint32_t limit = m->attn->opt_wait_limit;
+  if (bp_q1_matmul_is_tiled(mt)) {
+    if (norm != nullptr && reinterpret_cast<uintptr_t>(norm) % 4u != 0) {  // (a manifest may place it at any f16)
+      M_CUDA(m, bp_q1_rms_norm(true, s, act, m->x_norm, norm, k, mt, m->cfg.rms_eps));
+      M_CUDA(m, bp_q1_quantize_tiled(true, s, m->x_norm, k, mt, m->a_tiled, m->a_tiled_d));
+    } else if (norm != nullptr) {
+      M_CUDA(m, bp_q1_rms_quantize_tiled(true, s, act, norm, m->cfg.rms_eps, k, mt, m->a_tiled, m->a_tiled_d));
+    } else if (up != nullptr) {
+      M_CUDA(m, bp_q1_silu_quantize_tiled(true, s, act, up, k, mt, m->a_tiled, m->a_tiled_d));
+    } else {
+      M_CUDA(m, bp_q1_quantize_tiled(true, s, act, k, mt, m->a_tiled, m->a_tiled_d));
+    }
+    M_CUDA(m, bp_q1_matmul_tiled(true, s, w, out, n_w, mt, m->a_tiled, m->a_tiled_d, accumulate, err, limit));
+    return BP_OK;
+  }
+  if (norm != nullptr) {
+    M_CUDA(m, bp_q1_rms_norm(true, s, act, m->x_norm, norm, k, mt, m->cfg.rms_eps));
+    act = m->x_norm;
+  } else if (up != nullptr) {
+    M_CUDA(m, bp_q1_silu_mul(true, s, act, up, m->ffn_in, static_cast<uint64_t>(mt) * k));
+    act = m->ffn_in;
+  }
   M_CUDA(m, bp_q1_quantize_q8(true, s, act, k, mt, m->a_d, m->a_qs));
-  M_CUDA(m, bp_q1_matmul_multi(true, s, w, out, n_w, mt, m->a_d, m->a_qs, accumulate, m->attn->err_dev, m->attn->opt_wait_limit));
+  M_CUDA(m, bp_q1_matmul_multi(true, s, w, out, n_w, mt, m->a_d, m->a_qs, accumulate, err, limit));
   return BP_OK;
 }
 
@@ -738,6 +765,8 @@ int bp_model_load(const char* dir, uint32_t max_seq, int32_t device, bp_model** 
   const uint32_t k_max = c.n_ff > c.q_dim ? (c.n_ff > c.n_embd ? c.n_ff : c.n_embd) : (c.q_dim > c.n_embd ? c.q_dim : c.n_embd);
   M_CUDA(m, cudaMalloc(&m->a_d, mm * (k_max / 32) * sizeof(float)));
   M_CUDA(m, cudaMalloc(&m->a_qs, mm * k_max));
+  M_CUDA(m, cudaMalloc(&m->a_tiled, bp_q1_tiled_bytes(M_MAX, k_max)));
+  M_CUDA(m, cudaMalloc(&m->a_tiled_d, bp_q1_tiled_scales(M_MAX, k_max) * sizeof(float)));
   M_CUDA(m, cudaMalloc(&m->tokens_dev, mm * sizeof(uint32_t)));
   M_CUDA(m, cudaMalloc(&m->topk_val, TOPK_MAX * sizeof(float)));
   M_CUDA(m, cudaMalloc(&m->topk_idx, TOPK_MAX * sizeof(uint32_t)));
@@ -757,7 +786,7 @@ void bp_model_free(bp_model* m) {
   for (auto p : m->dev_file) cudaFree(p);
   for (auto p : m->dev_bits) cudaFree(p);
   void* bufs[] = {m->x, m->x_norm, m->q, m->q_roped, m->k_cur, m->v_cur, m->attn_out, m->gate, m->up, m->ffn_in, m->logits,
-                  m->a_d, m->a_qs, m->tokens_dev, m->topk_val, m->topk_idx};
+                  m->a_d, m->a_qs, m->a_tiled, m->a_tiled_d, m->tokens_dev, m->topk_val, m->topk_idx};
   for (void* p : bufs) cudaFree(p);
   drop_step_graph(m);
   cudaFreeHost(m->token_pin);
@@ -849,11 +878,10 @@ int bp_model_prefill_topk(bp_model* m, const uint32_t* tokens, uint32_t n, uint3
   for (uint32_t il = 0; il < c.n_layer; il++) {  // layer_step_matmul_in_pass, src/forward.rs:1075-1253
     const LayerTensors& lt = m->layers[il];
     uint32_t launches = 0;
-    M_CUDA(m, bp_q1_rms_norm(pdl, s, m->x, m->x_norm, lt.attn_norm, c.n_embd, n, c.rms_eps));
     {
       const bp_q1_tensor w[3] = {lt.wq, lt.wk, lt.wv};
       __half* const out[3] = {m->q, m->k_cur, m->v_cur};
-      if (int st = quantize_and_matmul(m, m->x_norm, c.n_embd, n, w, out, 3, false)) return st;
+      if (int st = quantize_and_matmul(m, m->x, c.n_embd, n, w, out, 3, false, lt.attn_norm)) return st;
     }
     M_CUDA(m, bp_launch_q_norm_rope(m->attn, s, m->q, lt.q_norm, 0, n, &launches));
     M_CUDA(m, bp_launch_kv_writeback(m->attn, s, il, m->k_cur, m->v_cur, lt.k_norm, 0, n, &launches));
@@ -862,16 +890,14 @@ int bp_model_prefill_topk(bp_model* m, const uint32_t* tokens, uint32_t n, uint3
       __half* const out[1] = {m->x};
       if (int st = quantize_and_matmul(m, m->attn_out, c.q_dim, n, &lt.wo, out, 1, true)) return st;
     }
-    M_CUDA(m, bp_q1_rms_norm(pdl, s, m->x, m->x_norm, lt.ffn_norm, c.n_embd, n, c.rms_eps));
     {
       const bp_q1_tensor w[2] = {lt.wg, lt.wu};
       __half* const out[2] = {m->gate, m->up};
-      if (int st = quantize_and_matmul(m, m->x_norm, c.n_embd, n, w, out, 2, false)) return st;
+      if (int st = quantize_and_matmul(m, m->x, c.n_embd, n, w, out, 2, false, lt.ffn_norm)) return st;
     }
-    M_CUDA(m, bp_q1_silu_mul(pdl, s, m->gate, m->up, m->ffn_in, static_cast<uint64_t>(n) * c.n_ff));
     {
       __half* const out[1] = {m->x};
-      if (int st = quantize_and_matmul(m, m->ffn_in, c.n_ff, n, &lt.wd, out, 1, true)) return st;
+      if (int st = quantize_and_matmul(m, m->gate, c.n_ff, n, &lt.wd, out, 1, true, nullptr, m->up)) return st;
     }
   }
   return output_suffix(m, n - 1, k, logits, indices);

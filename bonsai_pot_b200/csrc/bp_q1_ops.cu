@@ -19,64 +19,17 @@
 
 #include "bp_common.cuh"
 #include "bp_ptx.cuh"
+#include "bp_q1_device.cuh"
 #include "bp_q1_ops.cuh"
 
 namespace {
 
 using namespace bp;
 namespace cg = cooperative_groups;
-constexpr unsigned FULL = 0xffffffffu;
 constexpr uint32_t MV_THREADS = 128;          // the invocation count of the fused shader: its sum of squares is per invocation
 // rows per lane (R): 4 for tall tensors (the activations a lane reads serve all of them), fewer for the
 // 4096-row ones, which would otherwise give the device only 64 CTAs
 constexpr uint32_t XB_STRIDE = 128 + 8;       // halves per staged block: 16 bytes of padding keep the 8 lanes of a row off each other's banks
-
-__device__ __forceinline__ float exp_det(float x) {  // the restatement's orc_exp_det, operation for operation
-  x = fminf(fmaxf(x, -87.3f), 88.7f);
-  const float n = rintf(__fmul_rn(x, 1.44269504088896341f));
-  float r = __fmaf_rn(n, -0.693359375f, x);
-  r = __fmaf_rn(n, 2.12194440e-4f, r);
-  float p = __fmaf_rn(r, 1.0f / 720.0f, 1.0f / 120.0f);
-  p = __fmaf_rn(r, p, 1.0f / 24.0f);
-  p = __fmaf_rn(r, p, 1.0f / 6.0f);
-  p = __fmaf_rn(r, p, 0.5f);
-  p = __fmaf_rn(r, p, 1.0f);
-  p = __fmaf_rn(r, p, 1.0f);
-  return ldexpf(p, static_cast<int>(n));
-}
-
-// f16(g / (1 + exp(-g))) * up, in f16 (silu_mul.wgsl:22-26)
-__device__ __forceinline__ __half silu_times_up(__half gate, __half up) {
-  const float g = __half2float(gate);
-  const float s = __fdiv_rn(g, __fadd_rn(1.0f, exp_det(-g)));
-  return __hmul(__float2half_rn(s), up);
-}
-
-// subgroupAdd of a 32-lane subgroup: xor butterfly 16, 8, 4, 2, 1
-__device__ __forceinline__ float butterfly32(float v) {
-#pragma unroll
-  for (int off = 16; off >= 1; off >>= 1) v = __fadd_rn(v, __shfl_xor_sync(FULL, v, off));
-  return v;
-}
-
-// Workgroup sum of rms_norm.wgsl:62-78 / matvec_q1_0_fused_normed.wgsl:131-146 for a CTA of NW warps:
-// per-warp butterfly, partial of warp s into lane s of warp 0 (zero elsewhere), butterfly again.
-template <uint32_t NW>
-__device__ __forceinline__ float workgroup_sum(float v, float* part /* shared, 32 floats */) {
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const float s = butterfly32(v);
-  if (lane == 0) part[warp] = s;
-  __syncthreads();
-  if (warp == 0) {
-    const float c = lane < NW ? part[lane] : 0.0f;
-    const float f = butterfly32(c);
-    if (lane == 0) part[0] = f;
-  }
-  __syncthreads();
-  const float total = part[0];
-  __syncthreads();
-  return total;
-}
 
 struct MvRange {
   const __half* d;        // block scales [n][nb]
@@ -1676,7 +1629,13 @@ cudaError_t bp_q1_quantize_q8(bool pdl, cudaStream_t s, const __half* x, uint32_
   return bp_launch(pdl, quantize_q8_kernel, dim3(static_cast<unsigned>((n_blocks + 255) / 256)), dim3(256), 0, s, x, n_blocks, d_out, qs_out);
 }
 
-static uint32_t g_matmul_variant = 0;  // 0 = by batch size; 1 dp4a, 2 mma.sync, 3 tcgen05; 4 / 5 = mma.sync with 64- / 128-token tiles only
+static uint32_t g_matmul_variant = 0;  // 0 = by batch size; 1 dp4a, 2 mma.sync, 3 tcgen05; 4 / 5 = mma.sync with 64- / 128-token tiles only; 6 .. 10 = a model's batches through the tiled product with 128, 112, 96, 64, 32 weight rows per tile
+
+// the kernel for the untiled activations of bp_op_quantize_q8_0
+static uint32_t op_variant(uint32_t m) {
+  if (g_matmul_variant == 0 || g_matmul_variant >= 6) return m > MMA_MIN_M ? 2u : 1u;
+  return g_matmul_variant >= 4 ? 2u : g_matmul_variant;
+}
 
 static cudaError_t launch_mma(bool pdl, cudaStream_t s, const bp_q1_tensor* w, __half* const* y, uint32_t n_w, uint32_t m, const float* a_d,
                               const int8_t* a_qs, uint32_t acc) {
@@ -1721,7 +1680,13 @@ static cudaError_t launch_mma(bool pdl, cudaStream_t s, const bp_q1_tensor* w, _
   return t_half < t_full ? launch(true, 0, tiles, pdl) : launch(false, 0, tiles, pdl);
 }
 
-void bp_q1_set_matmul_variant(uint32_t v) { g_matmul_variant = v <= 5 ? v : 0; }
+bool bp_q1_matmul_is_tiled(uint32_t m) { return m != 0 && (g_matmul_variant >= 6 || g_matmul_variant == 0); }
+uint32_t bp_q1_tile_width() {
+  constexpr uint32_t W[5] = {128, 112, 96, 64, 32};
+  return g_matmul_variant >= 6 ? W[g_matmul_variant - 6] : 0;
+}
+
+void bp_q1_set_matmul_variant(uint32_t v) { g_matmul_variant = v <= 10 ? v : 0; }
 
 cudaError_t bp_q1_take_error(uint32_t* code) {
   cudaError_t e = cudaMemcpyFromSymbol(code, g_q1_err, sizeof(uint32_t));
@@ -1738,7 +1703,7 @@ cudaError_t bp_q1_take_error(uint32_t* code) {
 // three give the same bits).
 cudaError_t bp_q1_matmul(bool pdl, cudaStream_t s, const bp_q1_tensor& w, uint32_t m, const float* a_d, const int8_t* a_qs, __half* y,
                          bool accumulate, uint32_t* err, uint32_t wait_limit) {
-  const uint32_t variant = g_matmul_variant >= 4 ? 2u : g_matmul_variant != 0 ? g_matmul_variant : (m > MMA_MIN_M ? 2u : 1u);
+  const uint32_t variant = op_variant(m);
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(matmul_q1_q8_mma_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(MMA_SMEM));
@@ -1768,7 +1733,7 @@ cudaError_t bp_q1_matmul(bool pdl, cudaStream_t s, const bp_q1_tensor& w, uint32
 // The same activations through up to three weight tensors of equal k: one launch where the kernel allows.
 cudaError_t bp_q1_matmul_multi(bool pdl, cudaStream_t s, const bp_q1_tensor* w, __half* const* y, uint32_t n_w, uint32_t m, const float* a_d,
                                const int8_t* a_qs, bool accumulate, uint32_t* err, uint32_t wait_limit) {
-  const uint32_t variant = g_matmul_variant >= 4 ? 2u : g_matmul_variant != 0 ? g_matmul_variant : (m > MMA_MIN_M ? 2u : 1u);
+  const uint32_t variant = op_variant(m);
   bool same_k = n_w >= 1 && n_w <= 3;
   for (uint32_t i = 1; i < n_w && same_k; i++) same_k = w[i].k == w[0].k;
   if (variant == 2 && same_k && n_w > 1) {

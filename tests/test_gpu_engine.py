@@ -492,3 +492,29 @@ def test_warp_per_row_matvec_is_identical_to_eight_lanes_per_row(k, n):
         lib.bp_op_set_matvec_rows(0)
     for a, b in zip(*got):
         assert np.array_equal(a.view(np.uint16), b.view(np.uint16))
+
+
+# heights that no tile width divides (n_ff = 640: 128 + 112 + .. leave remainders; K and V have 128 rows)
+RAGGED = dict(n_layer=1, n_embd=384, n_ff=640, n_head=4, n_kv_head=1, head_dim=128, n_vocab=512)
+
+
+@pytest.mark.parametrize("m", [1, 31, 33, 127, 128, 129, 300, 512])
+def test_tiled_product_is_identical_to_the_cuda_core_product(tmp_path, m):
+    """Every tile width of the tiled product (and the choice by size), one and several token tiles, partly filled
+    ones among them, with rms_norm and silu taken into the quantiser: hidden rows and logits as the dp4a path's."""
+    d = str(tmp_path / "m")
+    model_dir.write_synthetic_model(d, shape=RAGGED, seed=11)
+    prompt = [(13 * i + 5) % 500 for i in range(m)]
+    lib = _lib.load()
+    got = {}
+    try:
+        with bp.Model(d, max_seq=512) as gm:
+            for variant in (1, 0, 6, 7, 8, 9, 10):
+                lib.bp_op_set_matmul_variant(variant)
+                gm.prefill_topk(prompt)
+                got[variant] = [gm.logits().copy()] + [gm.hidden(r).copy() for r in {0, m // 2, m - 1}]
+    finally:
+        lib.bp_op_set_matmul_variant(0)
+    for variant, rows in got.items():
+        for a, b in zip(got[1], rows):
+            assert np.array_equal(a.view(np.uint8), b.view(np.uint8)), variant
