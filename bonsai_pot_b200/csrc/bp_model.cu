@@ -289,7 +289,7 @@ struct bp_model {
     std::vector<std::vector<bp_launch_record>> attn;  // per layer: the attention launches as captured
     bp_launch_recorder patch;                         // the recorder of the per-step pass
     bool valid = false;
-  } sg;
+  } sg, fill;                 // fill: the same without the output suffix (a token whose logits nobody asks for)
   bool step_graph = true;     // bp_model_set_step_graph
   uint64_t graph_steps = 0;   // steps that ran as a graph launch
   uint32_t* token_pin = nullptr;  // pinned: the token of the step (read by the graph's copy node)
@@ -446,51 +446,57 @@ int step_no_suffix(bp_model* m, uint32_t token, uint32_t pos) {
   return BP_OK;
 }
 
-void drop_step_graph(bp_model* m) {
-  if (m->sg.exec) cudaGraphExecDestroy(m->sg.exec);
-  if (m->sg.graph) cudaGraphDestroy(m->sg.graph);
-  m->sg = bp_model::StepGraph();
+void drop_step_graph(bp_model::StepGraph& g) {
+  if (g.exec) cudaGraphExecDestroy(g.exec);
+  if (g.graph) cudaGraphDestroy(g.graph);
+  g = bp_model::StepGraph();
+}
+void drop_step_graphs(bp_model* m) {
+  drop_step_graph(m->sg);
+  drop_step_graph(m->fill);
 }
 
 // The whole step (token copy, embed, layers, output norm, LM head, top-k of TOPK_MAX, result copies) captured
-// from the model's stream at position pos.
-int capture_step_graph(bp_model* m, uint32_t pos) {
+// from the model's stream at position pos. The fill graph begins with the embedding (several of its launches are
+// queued, each behind its own token copy) and ends with the last layer.
+int capture_step_graph(bp_model* m, bp_model::StepGraph& g, uint32_t pos) {
   const Config& c = m->cfg;
   cudaStream_t s = m->stream;
-  drop_step_graph(m);
-  m->sg.attn.resize(c.n_layer);
+  drop_step_graph(g);
+  const bool suffix = &g == &m->sg;
+  g.attn.resize(c.n_layer);
   M_CUDA(m, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   int st = BP_OK;
-  cudaError_t e = cudaMemcpyAsync(m->tokens_dev, m->token_pin, sizeof(uint32_t), cudaMemcpyHostToDevice, s);
+  cudaError_t e = suffix ? cudaMemcpyAsync(m->tokens_dev, m->token_pin, sizeof(uint32_t), cudaMemcpyHostToDevice, s) : cudaSuccess;
   if (e == cudaSuccess) e = bp_q1_embed(true, s, m->embed, m->tokens_dev, 1, m->x);
-  for (uint32_t il = 0; e == cudaSuccess && st == BP_OK && il < c.n_layer; il++) st = decode_layer(m, il, pos, true, &m->sg.attn[il]);
-  if (e == cudaSuccess && st == BP_OK) e = bp_q1_rms_norm(true, s, m->x, m->x, m->output_norm, c.n_embd, 1, c.rms_eps);
-  if (e == cudaSuccess && st == BP_OK) e = bp_q1_matvec(true, s, m->lm_head, m->x, m->logits, false);
-  if (e == cudaSuccess && st == BP_OK) e = bp_q1_topk(true, s, m->logits, c.n_vocab, TOPK_MAX, m->topk_val, m->topk_idx);
-  if (e == cudaSuccess && st == BP_OK) e = cudaMemcpyAsync(m->res_val_pin, m->topk_val, TOPK_MAX * sizeof(float), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess && st == BP_OK) e = cudaMemcpyAsync(m->res_idx_pin, m->topk_idx, TOPK_MAX * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-  const cudaError_t e_end = cudaStreamEndCapture(s, &m->sg.graph);  // always: the stream must leave capture mode
+  for (uint32_t il = 0; e == cudaSuccess && st == BP_OK && il < c.n_layer; il++) st = decode_layer(m, il, pos, true, &g.attn[il]);
+  if (suffix && e == cudaSuccess && st == BP_OK) e = bp_q1_rms_norm(true, s, m->x, m->x, m->output_norm, c.n_embd, 1, c.rms_eps);
+  if (suffix && e == cudaSuccess && st == BP_OK) e = bp_q1_matvec(true, s, m->lm_head, m->x, m->logits, false);
+  if (suffix && e == cudaSuccess && st == BP_OK) e = bp_q1_topk(true, s, m->logits, c.n_vocab, TOPK_MAX, m->topk_val, m->topk_idx);
+  if (suffix && e == cudaSuccess && st == BP_OK) e = cudaMemcpyAsync(m->res_val_pin, m->topk_val, TOPK_MAX * sizeof(float), cudaMemcpyDeviceToHost, s);
+  if (suffix && e == cudaSuccess && st == BP_OK) e = cudaMemcpyAsync(m->res_idx_pin, m->topk_idx, TOPK_MAX * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+  const cudaError_t e_end = cudaStreamEndCapture(s, &g.graph);  // always: the stream must leave capture mode
   if (st != BP_OK) return st;
   M_CUDA(m, e);
   M_CUDA(m, e_end);
-  M_CUDA(m, cudaGraphInstantiate(&m->sg.exec, m->sg.graph, 0));
-  m->sg.valid = true;
+  M_CUDA(m, cudaGraphInstantiate(&g.exec, g.graph, 0));
+  g.valid = true;
   return BP_OK;
 }
 
 // The attention nodes of the captured step, patched for position pos. False: the launches no longer have the
 // captured shape (another kernel instance, another number of launches): the step has to be captured again.
-int patch_step_graph(bp_model* m, uint32_t pos, bool* ok) {
+int patch_step_graph(bp_model* m, bp_model::StepGraph& g, uint32_t pos, bool* ok) {
   *ok = false;
   for (uint32_t il = 0; il < m->cfg.n_layer; il++) {
-    bp_launch_recorder& rec = m->sg.patch;  // its storage is reused from step to step
+    bp_launch_recorder& rec = g.patch;  // its storage is reused from step to step
     rec.mode = 1;
     rec.records.clear();
     bp_recorder() = &rec;
     const cudaError_t e = attention_call(m, il, pos);
     bp_recorder() = nullptr;
     M_CUDA(m, e);
-    const std::vector<bp_launch_record>& was = m->sg.attn[il];
+    const std::vector<bp_launch_record>& was = g.attn[il];
     if (rec.records.size() != was.size()) return BP_OK;
     for (size_t i = 0; i < was.size(); i++) {
       bp_launch_record& r = rec.records[i];
@@ -504,21 +510,27 @@ int patch_step_graph(bp_model* m, uint32_t pos, bool* ok) {
       kp.blockDim = r.block;
       kp.sharedMemBytes = static_cast<unsigned int>(r.smem);
       kp.kernelParams = argv;
-      M_CUDA(m, cudaGraphExecKernelNodeSetParams(m->sg.exec, was[i].node, &kp));
+      M_CUDA(m, cudaGraphExecKernelNodeSetParams(g.exec, was[i].node, &kp));
     }
   }
   *ok = true;
   return BP_OK;
 }
 
+// One step as a graph launch on the model's stream.
+int launch_step_graph(bp_model* m, bp_model::StepGraph& g, uint32_t pos) {
+  bool patched = false;
+  if (g.valid)
+    if (int st = patch_step_graph(m, g, pos, &patched)) return st;
+  if (!patched)
+    if (int st = capture_step_graph(m, g, pos)) return st;
+  M_CUDA(m, cudaGraphLaunch(g.exec, m->stream));
+  return BP_OK;
+}
+
 int step_topk_graph(bp_model* m, uint32_t token, uint32_t pos, uint32_t k, float* logits, uint32_t* indices) {
   *m->token_pin = token;
-  bool patched = false;
-  if (m->sg.valid)
-    if (int st = patch_step_graph(m, pos, &patched)) return st;
-  if (!patched)
-    if (int st = capture_step_graph(m, pos)) return st;
-  M_CUDA(m, cudaGraphLaunch(m->sg.exec, m->stream));
+  if (int st = launch_step_graph(m, m->sg, pos)) return st;
   M_CUDA(m, cudaStreamSynchronize(m->stream));
   m->graph_steps++;
   for (uint32_t i = 0; i < k; i++) {
@@ -788,7 +800,7 @@ void bp_model_free(bp_model* m) {
   void* bufs[] = {m->x, m->x_norm, m->q, m->q_roped, m->k_cur, m->v_cur, m->attn_out, m->gate, m->up, m->ffn_in, m->logits,
                   m->a_d, m->a_qs, m->a_tiled, m->a_tiled_d, m->tokens_dev, m->topk_val, m->topk_idx};
   for (void* p : bufs) cudaFree(p);
-  drop_step_graph(m);
+  drop_step_graphs(m);
   cudaFreeHost(m->token_pin);
   cudaFreeHost(m->res_val_pin);
   cudaFreeHost(m->res_idx_pin);
@@ -830,7 +842,7 @@ int bp_model_step_topk(bp_model* m, uint32_t token, uint32_t pos, uint32_t k, fl
 int bp_model_set_step_graph(bp_model* m, uint32_t enable) {
   if (int st = model_enter(m)) return st;
   m->step_graph = enable != 0;
-  if (!m->step_graph) drop_step_graph(m);
+  if (!m->step_graph) drop_step_graphs(m);
   return BP_OK;
 }
 uint64_t bp_model_graph_steps(const bp_model* m) { return m ? m->graph_steps : 0; }
@@ -848,8 +860,17 @@ int bp_model_prefill_loop_topk(bp_model* m, const uint32_t* tokens, uint32_t n, 
   for (uint32_t i = 0; i < n; i++)
     if (tokens[i] >= m->cfg.n_vocab) return mfail(m, BP_ERR_CONFIG, "invalid config: token id out of range");
   M_CUDA(m, cudaSetDevice(m->device));
+  // As graph launches, like the steps; a capture costs about two tokens' worth of stream launches, so a model that
+  // has none yet makes it for FILL_GRAPH_MIN tokens or more.
+  constexpr uint32_t FILL_GRAPH_MIN = 3;
+  const bool graph = m->step_graph && m->tap_mode == 0 && bp_use_umma(m->attn) && (m->fill.valid || n - 1 >= FILL_GRAPH_MIN);
   for (uint32_t i = 0; i + 1 < n; i++)  // KV-fill-only steps: no output suffix (src/forward.rs:947-965)
-    if (int st = step_no_suffix(m, tokens[i], pos_base + i)) return st;
+    if (graph) {
+      M_CUDA(m, cudaMemcpyAsync(m->tokens_dev, tokens + i, sizeof(uint32_t), cudaMemcpyHostToDevice, m->stream));
+      if (int st = launch_step_graph(m, m->fill, pos_base + i)) return st;
+    } else if (int st = step_no_suffix(m, tokens[i], pos_base + i)) {
+      return st;
+    }
   return bp_model_step_topk(m, tokens[n - 1], pos_base + n - 1, k, logits, indices);
 }
 

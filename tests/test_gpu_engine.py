@@ -518,3 +518,22 @@ def test_tiled_product_is_identical_to_the_cuda_core_product(tmp_path, m):
     for variant, rows in got.items():
         for a, b in zip(got[1], rows):
             assert np.array_equal(a.view(np.uint8), b.view(np.uint8)), variant
+
+
+def test_incremental_prefill_is_identical_as_graph_and_as_stream_launches(tmp_path):
+    d = str(tmp_path / "m")
+    model_dir.write_synthetic_model(d, seed=5)
+    toks = [(17 * i + 2) % 2000 for i in range(150)]
+    got = []
+    for graph in (True, False):
+        with bp.Model(d, max_seq=256) as gm:
+            gm.set_step_graph(graph)
+            s = gm.new_session()
+            rows = []
+            for a, b in ((0, 2), (2, 6), (6, 7), (7, 150)):  # below the length that makes the graph, at it, one token, across stages
+                s.prefill_one_at_a_time(toks[a:b], greedy())
+                rows.append(gm.logits().copy())
+            rows.append(np.frombuffer(s.snapshot().to_bytes(), dtype=np.uint8))
+            got.append(rows)
+    for a, b in zip(*got):
+        assert np.array_equal(a.view(np.uint8), b.view(np.uint8))
