@@ -647,9 +647,8 @@ __global__ void __launch_bounds__(256) matmul_q1_q8_kernel(const __half* w_d, co
   }
 }
 
-// The same product with warp-level MMAs (mma.sync m16n8k32, int8 x int8 -> int32), for batches of more than
-// MMA_MIN_M tokens: the integer dot of a sub-block of 32 is one MMA of the int8 activations with the weights
-// as +1 / -1 bytes. What the reference does in floating point, y += (a_d * w_d) * f32(sumi) per sub-block
+// The same product with warp-level MMAs (mma.sync m16n8k32, int8 x int8 -> int32), for batches of any size: the
+// integer dot of a sub-block of 32 is one MMA of the int8 activations with the weights as +1 / -1 bytes. What the reference does in floating point, y += (a_d * w_d) * f32(sumi) per sub-block
 // in ascending order, is done in the same order by the thread that holds the MMA's accumulator, so the result
 // has the same bits. A CTA of 16 warps owns 128 tokens x 128 weight rows, a warp 32 x 32 (2 x 4 MMA tiles
 // of m16 n8). Per block of 128 inputs the CTA stages the activations [128][128] and the weights as +-1
@@ -1631,9 +1630,14 @@ cudaError_t bp_q1_quantize_q8(bool pdl, cudaStream_t s, const __half* x, uint32_
 
 static uint32_t g_matmul_variant = 0;  // 0 = by batch size; 1 dp4a, 2 mma.sync, 3 tcgen05; 4 / 5 = mma.sync with 64- / 128-token tiles only; 6 .. 10 = a model's batches through the tiled product with 128, 112, 96, 64, 32 weight rows per tile
 
-// the kernel for the untiled activations of bp_op_quantize_q8_0
-static uint32_t op_variant(uint32_t m) {
-  if (g_matmul_variant == 0 || g_matmul_variant >= 6) return m > MMA_MIN_M ? 2u : 1u;
+// The kernel for the untiled activations of bp_op_quantize_q8_0. Up to MMA_MIN_M tokens the mma.sync kernel is taken
+// where its 16-byte reads are allowed (larger batches have always needed them): a pass of 21 tokens at the 8B shape
+// takes 13.5 ms with it and 53 ms with the CUDA-core kernel, one token 12.9 and 53.
+static uint32_t op_variant(uint32_t m, const float* a_d, const int8_t* a_qs, const uint8_t* w_qs) {
+  if (g_matmul_variant == 0 || g_matmul_variant >= 6) {
+    const bool aligned = ((reinterpret_cast<uintptr_t>(a_d) | reinterpret_cast<uintptr_t>(a_qs)) & 15u) == 0 && (reinterpret_cast<uintptr_t>(w_qs) & 3u) == 0;
+    return m > MMA_MIN_M || aligned ? 2u : 1u;
+  }
   return g_matmul_variant >= 4 ? 2u : g_matmul_variant;
 }
 
@@ -1695,15 +1699,13 @@ cudaError_t bp_q1_take_error(uint32_t* code) {
   return cudaMemcpyToSymbol(g_q1_err, &zero, sizeof zero);
 }
 
-// Batches of up to MMA_MIN_M tokens: CUDA cores (64 x 64 tiles fit them better than a 128-row MMA tile);
-// larger ones: the mma.sync kernel, which measured faster than the tcgen05 one (254 against 323 us for
-// 512 tokens x 4096 rows x 12288 inputs: both are bound by instruction issue, and what the tcgen05 kernel
-// saves on the arithmetic, 3 instead of 5 instructions per output and sub-block, it spends on staging f16
-// operands and on its barriers). Variant 1, 2, 3 forces dp4a, mma.sync, tcgen05 (tuning and tests: all
-// three give the same bits).
+// On untiled activations: the mma.sync kernel measured faster than the tcgen05 one that stages f16 operands (254
+// against 323 us for 512 tokens x 4096 rows x 12288 inputs: both are bound by instruction issue, and what the
+// latter saves on the arithmetic, 3 instead of 5 instructions per output and sub-block, it spends on staging and on
+// its barriers). Variant 1, 2, 3 forces dp4a, mma.sync, tcgen05 (tuning and tests: all three give the same bits).
 cudaError_t bp_q1_matmul(bool pdl, cudaStream_t s, const bp_q1_tensor& w, uint32_t m, const float* a_d, const int8_t* a_qs, __half* y,
                          bool accumulate, uint32_t* err, uint32_t wait_limit) {
-  const uint32_t variant = op_variant(m);
+  const uint32_t variant = op_variant(m, a_d, a_qs, w.qs);
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(matmul_q1_q8_mma_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(MMA_SMEM));
@@ -1733,7 +1735,7 @@ cudaError_t bp_q1_matmul(bool pdl, cudaStream_t s, const bp_q1_tensor& w, uint32
 // The same activations through up to three weight tensors of equal k: one launch where the kernel allows.
 cudaError_t bp_q1_matmul_multi(bool pdl, cudaStream_t s, const bp_q1_tensor* w, __half* const* y, uint32_t n_w, uint32_t m, const float* a_d,
                                const int8_t* a_qs, bool accumulate, uint32_t* err, uint32_t wait_limit) {
-  const uint32_t variant = op_variant(m);
+  const uint32_t variant = op_variant(m, a_d, a_qs, w[0].qs);
   bool same_k = n_w >= 1 && n_w <= 3;
   for (uint32_t i = 1; i < n_w && same_k; i++) same_k = w[i].k == w[0].k;
   if (variant == 2 && same_k && n_w > 1) {
