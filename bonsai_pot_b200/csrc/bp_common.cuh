@@ -77,6 +77,7 @@ struct bp_attn_ctx {
   struct bp_token_graph* tok_graph;  // the captured launches of bp_decode_token_host, or null
   uint32_t opt_pf_nq; // prefill: query tiles per work item (1 or 2), 0 = by batch size
   uint32_t opt_wait_limit;  // polls of an mbarrier / a meeting counter before a kernel gives up (BP_ERR_TIMEOUT)
+  uint32_t opt_mm_wait_limit;  // the same for a model's batched products
   uint32_t opt_poll_limit;  // polling rounds of the in-kernel merge before it gives up
   uint32_t opt_exclusive;   // 1: the caller's kernels have the device to themselves (all CTAs of a launch are co-resident)
   uint32_t umma_resident;   // tcgen05 decode: CTAs the device holds at once (occupancy query), the bound of a launch whose CTAs wait for one another

@@ -331,7 +331,7 @@ int bp_attn_create(const bp_attn_config* cfg, bp_attn_ctx** out) {
   c->opt_token_graph = 1;
   c->opt_umerge = 1;
   c->opt_uhpc = 1;  // one KV head per CTA measured faster than two at every context length tried
-  c->opt_wait_limit = 1u << 22;
+  c->opt_wait_limit = c->opt_mm_wait_limit = 1u << 22;
   c->opt_poll_limit = 1u << 18;
   c->opt_exclusive = 1;
   c->opt_vpre = 1;
@@ -1065,7 +1065,11 @@ int bp_set_option(bp_attn_ctx* c, const char* name, uint32_t value) {
     return BP_OK;
   } else if (strcmp(name, "wait_limit") == 0) {
     if (value == 0) return fail_config(c, "wait_limit must be > 0");
-    c->opt_wait_limit = value;
+    c->opt_wait_limit = c->opt_mm_wait_limit = value;
+    return BP_OK;
+  } else if (strcmp(name, "matmul_wait_limit") == 0) {
+    if (value == 0) return fail_config(c, "matmul_wait_limit must be > 0");
+    c->opt_mm_wait_limit = value;
     return BP_OK;
   } else if (strcmp(name, "merge_poll_limit") == 0) {
     if (value == 0) return fail_config(c, "merge_poll_limit must be > 0");

@@ -546,7 +546,7 @@ int quantize_and_matmul(bp_model* m, const __half* act, uint32_t k, uint32_t mt,
                         bool accumulate, const __half* norm = nullptr, const __half* up = nullptr) {
   cudaStream_t s = m->stream;
   uint32_t* err = m->attn->err_dev;
-  const uint32_t limit = m->attn->opt_wait_limit;
+  const uint32_t limit = m->attn->opt_mm_wait_limit;
   if (bp_q1_matmul_is_tiled(mt)) {
     if (norm != nullptr && reinterpret_cast<uintptr_t>(norm) % 4u != 0) {  // (a manifest may place it at any f16)
       M_CUDA(m, bp_q1_rms_norm(true, s, act, m->x_norm, norm, k, mt, m->cfg.rms_eps));

@@ -169,11 +169,14 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
 // mma.sync kernel, 29.2 now; 21 tokens: 53 ms with the CUDA-core kernel, 11.8 now. Slower (ms per 512-token pass): four
 // sets of one sub-block 32.6, the staging in four warps of its own 30.4, two issuing threads with the next
 // hand-over's first load before the last piece is added 30.8, scalar instead of packed sums and products: no change.
-// Every wait is bounded; a wait that gives up stores a code in the error word and the CTA winds down.
+// Every wait is bounded; a wait that gives up stores a code in the error word and the CTA winds down: it ends only
+// when its own copies have landed and its own MMAs are complete (waits of TT_DRAIN polls, whatever the caller's limit:
+// what is waited for there always comes), because the next CTA on the SM gets the same shared memory and TMEM.
+constexpr uint32_t TT_DRAIN = 1u << 20;
 template <uint32_t NC>
 __global__ void __launch_bounds__(TT_THREADS, 1) matmul_q1_tiled_kernel(const TiledTensors tensors, uint32_t k, uint32_t m, const uint8_t* __restrict__ a_t,
                                                                         const float* __restrict__ a_d, uint32_t accumulate, float one, uint32_t* err,
-                                                                        uint32_t wait_limit) {
+                                                                        uint32_t wait_limit, uint32_t poll_ns) {
   constexpr uint32_t N = 4 * NC, STAGE_B = 2 * TT_PART + N * 128;
   constexpr uint32_t G = NC > 16 ? 2 : 4, STEPS = 4 / G;      // sub-blocks per hand-over, hand-overs per block
   constexpr uint32_t BUFS = 2;                                                             // sets of G TMEM buffers
@@ -181,7 +184,7 @@ __global__ void __launch_bounds__(TT_THREADS, 1) matmul_q1_tiled_kernel(const Ti
   constexpr uint32_t W0 = NC < 16 ? NC : 16, W1 = NC - W0, PIECES = W1 != 0 ? 2 : 1;  // columns of a TMEM load
   static_assert(BUFS * G * COLS <= 512, "TMEM has 512 columns");
   extern __shared__ uint8_t tt_raw[];
-  __shared__ __align__(8) uint64_t full[TT_STAGES], a_full[TT_STAGES], empty[TT_STAGES], d_full[BUFS], d_empty[BUFS];
+  __shared__ __align__(8) uint64_t full[TT_STAGES], a_full[TT_STAGES], empty[TT_STAGES], d_full[BUFS], d_empty[BUFS], drained;
   __shared__ __align__(16) float s_wd[TT_WORKERS][2][32];
   __shared__ uint32_t tmem_base_s;
   __shared__ volatile uint32_t abort_s;
@@ -205,6 +208,7 @@ __global__ void __launch_bounds__(TT_THREADS, 1) matmul_q1_tiled_kernel(const Ti
       mbar_init(smem_u32(&d_full[i]), 1);
       mbar_init(smem_u32(&d_empty[i]), TT_WORKERS);
     }
+    mbar_init(smem_u32(&drained), 1);
     abort_s = 0;
     fence_barrier_init();
   }
@@ -218,7 +222,7 @@ __global__ void __launch_bounds__(TT_THREADS, 1) matmul_q1_tiled_kernel(const Ti
   // its loop without waiting, copying or writing results. (The flag is a register: a look at abort_s before every wait
   // and every MMA lengthened the chain from hand-over to hand-over by 7 % of the kernel.)
   bool dead = false;
-  auto waitb = [&](uint64_t* bar, uint32_t parity) {
+  auto waitb = [&](uint64_t* bar, uint32_t parity, uint32_t ns = 2000u) {  // ns: how long a poll may suspend its thread
     if (dead) return;
     const uint32_t addr = smem_u32(bar);
     for (uint32_t i = 0; i < wait_limit; i++) {
@@ -228,7 +232,7 @@ __global__ void __launch_bounds__(TT_THREADS, 1) matmul_q1_tiled_kernel(const Ti
           "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
           "selp.u32 %0, 1, 0, p;\n\t}"
           : "=r"(ok)
-          : "r"(addr), "r"(parity), "r"(2000u)
+          : "r"(addr), "r"(parity), "r"(ns)
           : "memory");
       if (ok) return;
       if (abort_s) {
@@ -246,9 +250,10 @@ __global__ void __launch_bounds__(TT_THREADS, 1) matmul_q1_tiled_kernel(const Ti
     if (lane == 0) {
       constexpr uint32_t IDESC = umma_idesc(1, 0, 0, 0, 0, TT_M, N);  // f32 = e4m3 (K-major) x e4m3 (K-major)
       const uint64_t dk = umma_desc_sw128(0, 16, 1024);
+      pdl_wait();  // the polls below count from here: the time of the kernel before this one is not theirs
       for (uint32_t b = 0; b < nb1; b++) {
         const uint32_t slot = b % TT_STAGES;
-        waitb(&a_full[slot], (b / TT_STAGES) & 1u);
+        waitb(&a_full[slot], (b / TT_STAGES) & 1u, poll_ns);
         waitb(&full[slot], (b / TT_STAGES) & 1u);
         const uint64_t ad = dk + ((smem_base + slot * STAGE_B) >> 4), bd = ad + (2u * TT_PART >> 4);
 #pragma unroll
@@ -264,6 +269,7 @@ __global__ void __launch_bounds__(TT_THREADS, 1) matmul_q1_tiled_kernel(const Ti
               umma_f8(tmem + (pb * G + g) * COLS, ad + part * (TT_PART >> 4) + (h * G + g) * 2u, bd + (h * G + g) * 2u, IDESC, part);
           umma_commit(smem_u32(&d_full[pb]));
         }
+        if (dead) break;  // no slot is given back any more: a copy into it could meet the previous one
         umma_commit(smem_u32(&empty[slot]));
       }
     }
@@ -378,7 +384,7 @@ __global__ void __launch_bounds__(TT_THREADS, 1) matmul_q1_tiled_kernel(const Ti
     }
     // no copy may still be on its way when the CTA ends (all have landed unless a wait gave up)
     if (wt == 0)
-      for (uint32_t b = copies > TT_STAGES ? copies - TT_STAGES : 0; b < copies; b++) (void)mbar_wait(smem_u32(&a_full[b % TT_STAGES]), (b / TT_STAGES) & 1u, wait_limit);
+      for (uint32_t b = copies > TT_STAGES ? copies - TT_STAGES : 0; b < copies; b++) (void)mbar_wait(smem_u32(&a_full[b % TT_STAGES]), (b / TT_STAGES) & 1u, TT_DRAIN);
     __syncwarp();
     if (row_ok && !dead) {
       __half* y = pick(tensors.y);
@@ -410,6 +416,13 @@ __global__ void __launch_bounds__(TT_THREADS, 1) matmul_q1_tiled_kernel(const Ti
   __syncwarp();  // the lanes of the one-thread roles meet again
   tc_fence_before();
   __syncthreads();
+  if (abort_s) {  // the workers have not seen the last MMAs complete
+    if (tid == 0) {  // (the thread that issued them)
+      umma_commit(smem_u32(&drained));
+      (void)mbar_wait(smem_u32(&drained), 0, TT_DRAIN);
+    }
+    __syncthreads();
+  }
   if (warp == 0) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);
@@ -443,8 +456,9 @@ cudaError_t launch_tiled(bool pdl, cudaStream_t s, const bp_q1_tensor* w, __half
     if (i < n_w) tiles += (w[i].n + 4 * NC - 1) / (4 * NC);
     t.tile_end[i] = tiles;
   }
+  // (a limit of a few polls is short in time too: the MMA issuer's polls for a copy suspend it for as many ns at most)
   return bp_launch(pdl, matmul_q1_tiled_kernel<NC>, dim3(tiles, (m + TT_M - 1) / TT_M), dim3(TT_THREADS), tt_smem<NC>(), s, t, w[0].k, m, a_t, a_d,
-                   accumulate ? 1u : 0u, 1.0f, err, wait_limit);
+                   accumulate ? 1u : 0u, 1.0f, err, wait_limit, wait_limit < 2000u ? wait_limit : 2000u);
 }
 
 }  // namespace

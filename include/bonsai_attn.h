@@ -279,7 +279,9 @@ int bp_set_variant(bp_attn_ctx* ctx, uint32_t variant);
  * start ends in BP_ERR_TIMEOUT after "merge_poll_limit" polling rounds (default
  * 2^18, about 0.2 us each). The peer exchange needs "exclusive_device" = 1.
  * Bounds of the device-side waits: "wait_limit" (polls of an mbarrier or of a
- * meeting counter before a kernel gives up, default 2^22) and "merge_poll_limit".
+ * meeting counter before a kernel gives up, default 2^22), "matmul_wait_limit"
+ * (the same for the batched matrix products of a model that owns the context;
+ * setting "wait_limit" sets it too) and "merge_poll_limit".
  * Peer exchange: "peer_meet_in_kernel" (see above, after bp_peer_sync). */
 int bp_set_option(bp_attn_ctx* ctx, const char* name, uint32_t value);
 /* Development aid: with the option "debug_counters" set to 1 the tcgen05 decode

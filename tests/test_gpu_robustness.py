@@ -9,7 +9,7 @@ import numpy as np
 import pytest
 
 import bonsai_pot_b200 as bp
-from bonsai_pot_b200 import _lib
+from bonsai_pot_b200 import _lib, model_dir
 from oracle import oracle as O
 from tests.helpers import build_decode_case, within_tolerance
 
@@ -278,3 +278,27 @@ def test_fused_tokens_in_one_graph_on_a_shallow_stack(n_layer):
     assert np.array_equal(results["plain"][0].view(np.uint16), results["graph"][0].view(np.uint16))
     for (d0, q0), (d1, q1) in zip(results["plain"][1], results["graph"][1]):
         assert np.array_equal(d0.view(np.uint32), d1.view(np.uint32)) and np.array_equal(q0, q1)
+
+
+@pytest.mark.parametrize("m", [1, 200, 512])
+def test_batched_product_whose_wait_runs_out_winds_down_and_latches(tmp_path, m):
+    """One poll of a nanosecond: the first wait of every CTA of every batched product gives up, with its copies in
+    flight. The launches behind it in the stream find shared memory and TMEM free, the model reports
+    BP_ERR_TIMEOUT from then on, and a fresh one on the same device gives the bits of an undisturbed one."""
+    d = str(tmp_path / "m")
+    model_dir.write_synthetic_model(d, seed=4)
+    prompt = [(11 * i + 1) % 2000 for i in range(m)]
+    rows = []
+    for disturbed in (False, True, False):
+        with bp.Model(d, max_seq=512) as gm:
+            if disturbed:
+                gm.attention().set_option("matmul_wait_limit", 1)
+                for _ in range(2):
+                    with pytest.raises(bp.DeviceTimeout):
+                        gm.prefill_topk(prompt)
+                assert gm.attention().status() == bp.errors.BP_ERR_TIMEOUT
+            else:
+                gm.prefill_topk(prompt)
+                rows.append((gm.logits(), gm.hidden(0), gm.hidden(m - 1)))
+    for a, b in zip(*rows):
+        assert np.array_equal(a.view(np.uint16), b.view(np.uint16))
