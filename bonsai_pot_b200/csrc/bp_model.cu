@@ -264,6 +264,7 @@ struct bp_model {
   bp_attn_ctx* attn = nullptr;
   cudaStream_t stream = nullptr;
   uint8_t* dev_file[5] = {};   // the weight files as they are on disk
+  std::map<std::string, uint64_t> f16_at;  // where an F16 tensor begins in its file's device copy: a multiple of 16
   void* dev_bits[4] = {};      // re-laid-out sign words: attn, gate_up, down, embed_lmhead (same offsets as the files' qs regions)
   std::vector<LayerTensors> layers;
   bp_q1_tensor embed, lm_head;
@@ -364,7 +365,7 @@ bp_q1_tensor q1_view(const bp_model* m, const std::string& name) {
 }
 const __half* f16_view(const bp_model* m, const std::string& name) {
   const TensorEntry& t = m->cfg.manifest.at(name);
-  return reinterpret_cast<const __half*>(m->dev_file[file_index(t.buffer)] + t.offset);
+  return reinterpret_cast<const __half*>(m->dev_file[file_index(t.buffer)] + m->f16_at.at(name));
 }
 
 // The attention call of layer il at position pos (Q norm + RoPE, cache write, attention: one launch by default).
@@ -548,10 +549,7 @@ int quantize_and_matmul(bp_model* m, const __half* act, uint32_t k, uint32_t mt,
   uint32_t* err = m->attn->err_dev;
   const uint32_t limit = m->attn->opt_mm_wait_limit;
   if (bp_q1_matmul_is_tiled(mt)) {
-    if (norm != nullptr && reinterpret_cast<uintptr_t>(norm) % 4u != 0) {  // (a manifest may place it at any f16)
-      M_CUDA(m, bp_q1_rms_norm(true, s, act, m->x_norm, norm, k, mt, m->cfg.rms_eps));
-      M_CUDA(m, bp_q1_quantize_tiled(true, s, m->x_norm, k, mt, m->a_tiled, m->a_tiled_d));
-    } else if (norm != nullptr) {
+    if (norm != nullptr) {
       M_CUDA(m, bp_q1_rms_quantize_tiled(true, s, act, norm, m->cfg.rms_eps, k, mt, m->a_tiled, m->a_tiled_d));
     } else if (up != nullptr) {
       M_CUDA(m, bp_q1_silu_quantize_tiled(true, s, act, up, k, mt, m->a_tiled, m->a_tiled_d));
@@ -727,8 +725,21 @@ int bp_model_load(const char* dir, uint32_t max_seq, int32_t device, bp_model** 
     Fail f = read_file(std::string(dir) + "/" + FILE_NAMES[fi], &bytes);
     if (f.status) return mfail(m, f.status, f.msg);
     for (const auto& kv : c.manifest)
-      if (kv.second.buffer == FILE_NAMES[fi] && kv.second.offset + kv.second.length > bytes.size())
+      if (kv.second.buffer == FILE_NAMES[fi] && (kv.second.length > bytes.size() || kv.second.offset > bytes.size() - kv.second.length))
         return mfail(m, BP_ERR_CONFIG, "invalid config: manifest: tensor extends past the end of its buffer file");
+    // The format lets an F16 tensor begin anywhere, the kernels read norm weights as 8-byte vectors: what is not
+    // aligned gets a second place behind the file's bytes.
+    for (const auto& kv : c.manifest) {
+      const TensorEntry& t = kv.second;
+      if (t.buffer != FILE_NAMES[fi] || t.dtype != "F16") continue;
+      uint64_t at = t.offset;
+      if (at % 16 != 0) {
+        at = (bytes.size() + 15u) & ~static_cast<uint64_t>(15u);
+        bytes.resize(at + t.length);
+        memcpy(bytes.data() + at, bytes.data() + t.offset, t.length);
+      }
+      m->f16_at[kv.first] = at;
+    }
     M_CUDA(m, cudaMalloc(&m->dev_file[fi], bytes.size() + 16));
     M_CUDA(m, cudaMemcpy(m->dev_file[fi], bytes.data(), bytes.size(), cudaMemcpyHostToDevice));
     if (FILE_OF_BITS[fi] >= 0) M_CUDA(m, cudaMalloc(&m->dev_bits[FILE_OF_BITS[fi]], bytes.size() + 16));
@@ -739,6 +750,7 @@ int bp_model_load(const char* dir, uint32_t max_seq, int32_t device, bp_model** 
     if (t.dtype != "Q1_0") continue;
     const int fi = file_index(t.buffer);
     if (t.qs_offset % 16 != 0) return mfail(m, BP_ERR_CONFIG, "invalid config: manifest: Q1_0 sign region is not 16-byte aligned");
+    if (t.d_offset % 2 != 0) return mfail(m, BP_ERR_CONFIG, "invalid config: manifest: Q1_0 scales are not 2-byte aligned");
     const uint64_t n_out = t.shape.size() > 1 ? t.shape[1] : 1;
     M_CUDA(m, bp_q1_relayout(m->stream, m->dev_file[fi] + t.qs_offset, static_cast<uint8_t*>(m->dev_bits[FILE_OF_BITS[fi]]) + t.qs_offset,
                              n_out * t.nb));

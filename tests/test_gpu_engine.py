@@ -4,12 +4,14 @@ the one-token forward pass with the GPU's attention outputs fed to the CPU pass 
 the residual stream and the logits is exact while attention keeps its own tolerance); and the session
 behaviour the reference tests in tests/gpu_integration.rs."""
 import ctypes as C
+import os
 
 import numpy as np
 import pytest
 
 import bonsai_pot_b200 as bp
 from bonsai_pot_b200 import _lib, model_dir
+from bonsai_pot_b200.model import check_dir
 from oracle import engine as E
 
 pytestmark = pytest.mark.gpu
@@ -537,3 +539,57 @@ def test_incremental_prefill_is_identical_as_graph_and_as_stream_launches(tmp_pa
             got.append(rows)
     for a, b in zip(*got):
         assert np.array_equal(a.view(np.uint8), b.view(np.uint8))
+
+
+def move_norms(path, shift, seed=3):
+    """Random norm weights, all of them `shift` bytes further in their file than the writer put them."""
+    rng = np.random.default_rng(seed)
+    f = os.path.join(path, "weights_norms.bin")
+    n = os.path.getsize(f) // 2
+    with open(f, "wb") as out:
+        out.write(b"\0" * shift + (1 + 0.3 * rng.standard_normal(n)).astype(np.float16).tobytes())
+    ini = os.path.join(path, "config.ini")
+    text, section_f16 = [], False
+    for line in open(ini).read().split("\n"):
+        if line.startswith("dtype = "):
+            section_f16 = line == "dtype = F16"
+        if section_f16 and line.startswith("offset = "):
+            line = "offset = %d" % (int(line[9:]) + shift)
+        text.append(line)
+    with open(ini, "w", newline="\n") as out:
+        out.write("\n".join(text))
+
+
+def test_norm_weights_may_begin_at_any_offset_of_their_file(tmp_path):
+    """The format asks for no alignment of an F16 tensor (validate_cfg, src/model.rs:658-837, looks at lengths only):
+    batched and one-token passes give the same bits wherever it begins. A Q1_0 tensor whose scales begin at an odd
+    byte is refused (no address of an f16)."""
+    rows = []
+    for shift in (0, 2, 4, 14):
+        d = str(tmp_path / ("m%d" % shift))
+        model_dir.write_synthetic_model(d, seed=21)
+        move_norms(d, shift)
+        with bp.Model(d, max_seq=128) as gm:
+            gm.prefill_topk(list(range(5, 45)))
+            got = [gm.logits(), gm.hidden(3)]
+            for pos in range(40, 44):
+                gm.step_topk(100 + pos, pos)
+                got.append(gm.logits())
+            gm.prefill_loop_topk(list(range(60, 66)), pos_base=44)
+            rows.append(got + [gm.logits(), gm.hidden(0)])
+    assert not np.isnan(rows[0][0].astype(np.float32)).any()
+    for got in rows[1:]:
+        for a, b in zip(rows[0], got):
+            assert np.array_equal(a.view(np.uint16), b.view(np.uint16))
+    odd = str(tmp_path / "odd")
+    model_dir.write_synthetic_model(odd, seed=21)
+    ini = os.path.join(odd, "config.ini")
+    head, name, tail = open(ini).read().partition("[blk.0.attn_q.weight]")
+    for a, b in (("d_offset = 0", "d_offset = 13"), ("qs_offset = 8192", "qs_offset = 8208"), ("length = 73728", "length = 73731")):
+        assert a in tail
+        tail = tail.replace(a, b, 1)
+    with open(ini, "w", newline="\n") as out:
+        out.write(head + name + tail)
+    check_dir(odd)  # (lengths and offsets add up)
+    with pytest.raises(bp.ConfigError, match="scales"):
+        bp.Model(odd, max_seq=64)
