@@ -648,13 +648,12 @@ __global__ void __launch_bounds__(256) matmul_q1_q8_kernel(const __half* w_d, co
 }
 
 // The same product with warp-level MMAs (mma.sync m16n8k32, int8 x int8 -> int32), for batches of any size: the
-// integer dot of a sub-block of 32 is one MMA of the int8 activations with the weights as +1 / -1 bytes. What the reference does in floating point, y += (a_d * w_d) * f32(sumi) per sub-block
-// in ascending order, is done in the same order by the thread that holds the MMA's accumulator, so the result
-// has the same bits. A CTA of 16 warps owns 128 tokens x 128 weight rows, a warp 32 x 32 (2 x 4 MMA tiles
+// integer dot of a sub-block of 32 is one MMA of the int8 activations with the weights as +1 / -1 bytes. What the
+// reference does in floating point, y += (a_d * w_d) * f32(sumi) per sub-block in ascending order, is done in the
+// same order by the thread that holds the MMA's accumulator, so the result has the same bits. A CTA of 16 warps owns 128 tokens x 128 weight rows, a warp 32 x 32 (2 x 4 MMA tiles
 // of m16 n8). Per block of 128 inputs the CTA stages the activations [128][128] and the weights as +-1
 // bytes [128][128] in shared memory (16-byte chunks xor-swizzled by the row, read back with ldmatrix); the
 // next block's global loads are in flight while the current one is multiplied.
-constexpr uint32_t MMA_MIN_M = 32;
 constexpr uint32_t MT = 128;                        // tile edge, tokens and weight rows
 constexpr uint32_t MMA_TILE_B = MT * 128;           // one operand tile: 128 rows of 128 int8
 constexpr uint32_t MMA_SMEM = 4 * MMA_TILE_B + 2 * (MT * 4 + MT) * 4 + 64;  // A, B double-buffered, scales, sign table
@@ -1630,15 +1629,19 @@ cudaError_t bp_q1_quantize_q8(bool pdl, cudaStream_t s, const __half* x, uint32_
 
 static uint32_t g_matmul_variant = 0;  // 0 = by batch size; 1 dp4a, 2 mma.sync, 3 tcgen05; 4 / 5 = mma.sync with 64- / 128-token tiles only; 6 .. 10 = a model's batches through the tiled product with 128, 112, 96, 64, 32 weight rows per tile
 
-// The kernel for the untiled activations of bp_op_quantize_q8_0. Up to MMA_MIN_M tokens the mma.sync kernel is taken
-// where its 16-byte reads are allowed (larger batches have always needed them): a pass of 21 tokens at the 8B shape
-// takes 13.5 ms with it and 53 ms with the CUDA-core kernel, one token 12.9 and 53.
-static uint32_t op_variant(uint32_t m, const float* a_d, const int8_t* a_qs, const uint8_t* w_qs) {
-  if (g_matmul_variant == 0 || g_matmul_variant >= 6) {
-    const bool aligned = ((reinterpret_cast<uintptr_t>(a_d) | reinterpret_cast<uintptr_t>(a_qs)) & 15u) == 0 && (reinterpret_cast<uintptr_t>(w_qs) & 3u) == 0;
-    return m > MMA_MIN_M || aligned ? 2u : 1u;
-  }
-  return g_matmul_variant >= 4 ? 2u : g_matmul_variant;
+// The kernel for the untiled activations of bp_op_quantize_q8_0: mma.sync wherever its 16-byte reads of a_d and a_qs
+// are allowed (a pass of 21 tokens at the 8B shape takes 13.5 ms with it and 53 ms with the CUDA-core kernel, one
+// token 12.9 and 53), else the CUDA-core kernel, which reads 32-bit words. 0: no kernel can read these buffers, or
+// not the one that was forced.
+static uint32_t op_variant(const bp_q1_tensor* w, __half* const* y, uint32_t n_w, const float* a_d, const int8_t* a_qs) {
+  const uintptr_t act = reinterpret_cast<uintptr_t>(a_d) | reinterpret_cast<uintptr_t>(a_qs);
+  if (act % 4u != 0) return 0;
+  for (uint32_t i = 0; i < n_w; i++)
+    if (reinterpret_cast<uintptr_t>(w[i].qs) % 4u != 0 || reinterpret_cast<uintptr_t>(w[i].d) % 2u != 0 || reinterpret_cast<uintptr_t>(y[i]) % 2u != 0) return 0;
+  if (g_matmul_variant == 0 || g_matmul_variant >= 6) return act % 16u == 0 ? 2u : 1u;
+  if (g_matmul_variant == 1) return 1;
+  if (act % 16u != 0) return 0;
+  return g_matmul_variant == 3 ? 3u : 2u;
 }
 
 static cudaError_t launch_mma(bool pdl, cudaStream_t s, const bp_q1_tensor* w, __half* const* y, uint32_t n_w, uint32_t m, const float* a_d,
@@ -1705,7 +1708,8 @@ cudaError_t bp_q1_take_error(uint32_t* code) {
 // its barriers). Variant 1, 2, 3 forces dp4a, mma.sync, tcgen05 (tuning and tests: all three give the same bits).
 cudaError_t bp_q1_matmul(bool pdl, cudaStream_t s, const bp_q1_tensor& w, uint32_t m, const float* a_d, const int8_t* a_qs, __half* y,
                          bool accumulate, uint32_t* err, uint32_t wait_limit) {
-  const uint32_t variant = op_variant(m, a_d, a_qs, w.qs);
+  const uint32_t variant = op_variant(&w, &y, 1, a_d, a_qs);
+  if (variant == 0) return cudaErrorMisalignedAddress;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(matmul_q1_q8_mma_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(MMA_SMEM));
@@ -1735,7 +1739,8 @@ cudaError_t bp_q1_matmul(bool pdl, cudaStream_t s, const bp_q1_tensor& w, uint32
 // The same activations through up to three weight tensors of equal k: one launch where the kernel allows.
 cudaError_t bp_q1_matmul_multi(bool pdl, cudaStream_t s, const bp_q1_tensor* w, __half* const* y, uint32_t n_w, uint32_t m, const float* a_d,
                                const int8_t* a_qs, bool accumulate, uint32_t* err, uint32_t wait_limit) {
-  const uint32_t variant = op_variant(m, a_d, a_qs, w[0].qs);
+  const uint32_t variant = op_variant(w, y, n_w, a_d, a_qs);
+  if (variant == 0) return cudaErrorMisalignedAddress;
   bool same_k = n_w >= 1 && n_w <= 3;
   for (uint32_t i = 1; i < n_w && same_k; i++) same_k = w[i].k == w[0].k;
   if (variant == 2 && same_k && n_w > 1) {

@@ -51,11 +51,12 @@ int bp_op_silu_mul(void* stream, const void* gate, const void* up, void* out, ui
 int bp_op_embed(void* stream, const void* d, const void* qs, uint32_t k, const void* tokens, uint32_t m, void* x);
 /* dispatch_quantize_act (src/forward.rs:415-441, quantize_q8_0.wgsl): d_out f32 [m][k/32], qs_out int8 [m][k] */
 int bp_op_quantize_q8_0(void* stream, const void* x, uint32_t k, uint32_t m, void* d_out, void* qs_out);
-/* dispatch_matmul_q1_0 (src/forward.rs:443-472, matmul_q1_0_q8_0.wgsl): y[m][n] (+)= A W^T */
+/* dispatch_matmul_q1_0 (src/forward.rs:443-472, matmul_q1_0_q8_0.wgsl): y[m][n] (+)= A W^T. qs, a_d and a_qs must be
+ * 4-byte aligned (BP_ERR_CUDA otherwise); a_d and a_qs should be 16-byte aligned, see the tuning aid. */
 int bp_op_matmul_q1_0_q8_0(void* stream, const void* d, const void* qs, uint32_t k, uint32_t n, uint32_t m, const void* a_d,
                            const void* a_qs, void* y, uint32_t accumulate);
 /* Tuning aid of the matmul: 0 = the default: a model's batches through the tiled tcgen05 product, this entry point
- * through mma.sync (CUDA cores up to 32 tokens if a_d or a_qs is not 16-byte aligned), 1 = CUDA cores (dp4a), 2 =
+ * through mma.sync (through the CUDA cores if a_d or a_qs is not 16-byte aligned), 1 = CUDA cores (dp4a), 2 =
  * mma.sync (int8; tiles of 128 tokens, of 64, or whole waves of the former and the rest as the latter, whichever fills
  * the device's waves best), 3 = tcgen05 (f16 operands), 4 / 5 = mma.sync with tiles of 64 / 128 tokens only, 6 .. 10 = as 0
  * with 128, 112, 96, 64, 32 weight rows per tile of the tiled product. Results do not depend on it. Process-wide. */

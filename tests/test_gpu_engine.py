@@ -173,6 +173,45 @@ def test_matmul_q1_0_q8_0_bit_exact(k, n, m, accumulate):
         lib.bp_op_set_matmul_variant(0)
 
 
+@pytest.mark.parametrize("m", [1, 20, 40, 130])
+def test_matmul_serves_any_buffer_it_can_read_and_refuses_the_others(m):
+    """Activations at 4 and 8 mod 16 bytes (a slice of a caller's arena) give the aligned result at every batch size;
+    below 4 bytes, and for a kernel forced to 16-byte reads, the call is refused on the host and nothing is written."""
+    lib = _lib.load()
+    k, n = 512, 200
+    rng = np.random.default_rng(m)
+    blob, d_off, qs_off, d_dev, qs_dev, _ = random_q1(rng, k, n)
+    act = (rng.standard_normal((m, k)) * 2).astype(np.float16)
+    a_d, a_qs = E.quantize_q8_0(act, k, m)
+    want = E.matmul(blob, d_off, qs_off, k, n, m, a_d, a_qs)
+
+    def at(a, off):  # the array `off` bytes into an allocation
+        raw = np.ascontiguousarray(a).view(np.uint8).reshape(-1)
+        return dev(np.concatenate([np.zeros(off, dtype=np.uint8), raw, np.zeros(16, dtype=np.uint8)]))
+
+    def call(off_d, off_q, off_w=0):
+        bd, bq, bw = at(a_d, off_d), at(a_qs, off_q), at(qs_dev.cpu().numpy(), off_w)
+        y = torch.zeros(m, n, dtype=torch.float16, device="cuda")
+        st = lib.bp_op_matmul_q1_0_q8_0(None, d_dev.data_ptr(), bw.data_ptr() + off_w, k, n, m, bd.data_ptr() + off_d, bq.data_ptr() + off_q,
+                                        y.data_ptr(), 0)
+        torch.cuda.synchronize()
+        return st, y
+
+    for offs in ((0, 0), (4, 0), (0, 4), (8, 12), (0, 0, 4), (4, 4, 12)):
+        st, y = call(*offs)
+        assert st == 0 and bits_equal(y, want), offs
+    for offs in ((0, 1), (0, 2), (2, 0), (0, 0, 2)):
+        st, y = call(*offs)
+        assert st == bp.errors.BP_ERR_CUDA and not y.any(), offs
+    try:
+        for variant in (2, 3, 4, 5):
+            lib.bp_op_set_matmul_variant(variant)
+            st, y = call(4, 0)
+            assert st == bp.errors.BP_ERR_CUDA and not y.any(), variant
+    finally:
+        lib.bp_op_set_matmul_variant(0)
+
+
 @pytest.mark.parametrize("k,n,m,accumulate", [(256, 24576, 512, True), (256, 6144, 512, False), (128, 6144, 300, True),
                                               (128, 19000, 450, False)])
 def test_matmul_tile_choices_agree(k, n, m, accumulate):
