@@ -1530,7 +1530,13 @@ void bp_q1_set_matvec_rows(uint32_t rows_per_lane) {
   g_mv_const_k = (rows_per_lane & 8u) == 0;  // + 8: the general instances only
 }
 
+// What a kernel reads or writes in vectors is checked here: an address that it cannot take is an error of the call.
+static bool aligned(uintptr_t to, const void* a, const void* b = nullptr) {
+  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & (to - 1u)) == 0;
+}
+
 cudaError_t bp_q1_relayout(cudaStream_t s, const uint8_t* qs, void* out, uint64_t n_blocks) {
+  if (!aligned(16, qs, out)) return cudaErrorMisalignedAddress;
   relayout_kernel<<<static_cast<unsigned>((n_blocks + 255) / 256), 256, 0, s>>>(qs, static_cast<uint4*>(out), n_blocks);
   return cudaGetLastError();
 }
@@ -1543,7 +1549,7 @@ cudaError_t bp_q1_matvec(bool pdl, cudaStream_t s, const bp_q1_tensor& w, const 
   p.k = w.k;
   p.x = x;
   p.accumulate = accumulate ? 1u : 0u;
-  if (reinterpret_cast<uintptr_t>(x) % 16u != 0) return cudaErrorMisalignedAddress;  // the activations are staged 16 bytes at a time
+  if (!aligned(16, x, w.bits) || !aligned(2, w.d, y)) return cudaErrorMisalignedAddress;
   return launch_mv<0>(pdl, s, p);
 }
 
@@ -1554,6 +1560,7 @@ cudaError_t bp_q1_matvec_normed(bool pdl, cudaStream_t s, const bp_q1_tensor* w,
   p.n_ranges = n_ranges;
   for (uint32_t r = 0; r < n_ranges; r++) {
     if (w[r].k != w[0].k || w[r].n % 16u != 0) return cudaErrorInvalidValue;  // the shader's range rule (ROWS_PER_WG = 16)
+    if (!aligned(16, w[r].bits) || !aligned(2, w[r].d, out[r])) return cudaErrorMisalignedAddress;
     p.r[r] = {w[r].d, static_cast<const uint4*>(w[r].bits), out[r], w[r].n};
     p.n_total += w[r].n;
   }
@@ -1561,6 +1568,7 @@ cudaError_t bp_q1_matvec_normed(bool pdl, cudaStream_t s, const bp_q1_tensor* w,
   p.x = x;
   p.aux = w_norm;
   p.eps = eps;
+  if (!aligned(8, x, w_norm)) return cudaErrorMisalignedAddress;
   return launch_mv<1>(pdl, s, p);
 }
 
@@ -1569,6 +1577,7 @@ cudaError_t bp_q1_matvec_normed(bool pdl, cudaStream_t s, const bp_q1_tensor* w,
 cudaError_t bp_q1_matvec_normed_silu(bool pdl, cudaStream_t s, const bp_q1_tensor& w_gate, const bp_q1_tensor& w_up, __half* out,
                                      const __half* x, const __half* w_norm, float eps) {
   if (w_gate.k != w_up.k || w_gate.n != w_up.n) return cudaErrorInvalidValue;
+  if (!aligned(16, w_gate.bits, w_up.bits) || !aligned(2, w_gate.d, w_up.d) || !aligned(2, out) || !aligned(8, x, w_norm)) return cudaErrorMisalignedAddress;
   MvParams p = {};
   p.n_ranges = 2;
   p.r[0] = {w_gate.d, static_cast<const uint4*>(w_gate.bits), out, w_gate.n};
@@ -1601,29 +1610,33 @@ cudaError_t bp_q1_matvec_silu(bool pdl, cudaStream_t s, const bp_q1_tensor& w, c
   p.k = w.k;
   p.x = gate;
   p.aux = up;
+  if (!aligned(16, w.bits) || !aligned(2, w.d, y) || !aligned(8, gate, up)) return cudaErrorMisalignedAddress;
   p.accumulate = accumulate ? 1u : 0u;
   return launch_mv<2>(pdl, s, p);
 }
 
 cudaError_t bp_q1_rms_norm(bool pdl, cudaStream_t s, const __half* in, __half* out, const __half* w, uint32_t group_size,
                            uint32_t n_groups, float eps) {
+  if (!aligned(2, in, out) || !aligned(2, w)) return cudaErrorMisalignedAddress;
   return bp_launch(pdl, rms_norm_kernel, dim3(n_groups), dim3(512), 0, s, in, out, w, group_size, eps);
 }
 
 cudaError_t bp_q1_silu_mul(bool pdl, cudaStream_t s, const __half* gate, const __half* up, __half* out, uint64_t n) {
-  const bool vec8 = n % 8u == 0 && (reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(up) | reinterpret_cast<uintptr_t>(out)) % 16u == 0;
+  if (!aligned(2, gate, up) || !aligned(2, out)) return cudaErrorMisalignedAddress;
+  const bool vec8 = n % 8u == 0 && aligned(16, gate, up) && aligned(16, out);
   if (vec8) return bp_launch(pdl, silu_mul_kernel<true>, dim3(static_cast<unsigned>((n / 8u + 255) / 256)), dim3(256), 0, s, gate, up, out, n);
   return bp_launch(pdl, silu_mul_kernel<false>, dim3(static_cast<unsigned>((n + 255) / 256)), dim3(256), 0, s, gate, up, out, n);
 }
 
 cudaError_t bp_q1_embed(bool pdl, cudaStream_t s, const bp_q1_tensor& w, const uint32_t* tokens, uint32_t m, __half* x) {
+  if (!aligned(2, w.d) || !aligned(4, tokens) || !aligned(16, x)) return cudaErrorMisalignedAddress;
   const uint64_t units = static_cast<uint64_t>(m) * (w.k / 8u);
   return bp_launch(pdl, embed_kernel, dim3(static_cast<unsigned>((units + 255) / 256)), dim3(256), 0, s, w.d, w.qs, w.k, tokens, m, x);
 }
 
 cudaError_t bp_q1_quantize_q8(bool pdl, cudaStream_t s, const __half* x, uint32_t k, uint32_t m, float* d_out, int8_t* qs_out) {
   const uint64_t n_blocks = static_cast<uint64_t>(m) * (k / 32u);
-  if (reinterpret_cast<uintptr_t>(x) % 16u != 0 || reinterpret_cast<uintptr_t>(qs_out) % 16u != 0) return cudaErrorMisalignedAddress;
+  if (!aligned(16, x, qs_out) || !aligned(4, d_out)) return cudaErrorMisalignedAddress;
   return bp_launch(pdl, quantize_q8_kernel, dim3(static_cast<unsigned>((n_blocks + 255) / 256)), dim3(256), 0, s, x, n_blocks, d_out, qs_out);
 }
 
@@ -1775,6 +1788,7 @@ static cudaError_t topk_launch(bool pdl, cudaStream_t s, const __half* logits, u
 }
 
 cudaError_t bp_q1_topk(bool pdl, cudaStream_t s, const __half* logits, uint32_t n, uint32_t k, float* out_val, uint32_t* out_idx) {
+  if (!aligned(4, logits, out_val) || !aligned(4, out_idx)) return cudaErrorMisalignedAddress;
   // Per device, once: 16 CTAs per cluster (beyond the portable 8) if the device can hold such a cluster.
   static int ctas_of_device[64] = {};
   int dev = 0;

@@ -26,7 +26,10 @@ extern "C" {
  * A Q1_0 tensor [n][k] is given by its two arrays as the model directory stores them
  * (manifest d_offset / qs_offset, src/model.rs:586-606): `d` = f16 block scales
  * [n][k/128], `qs` = sign bytes [n][k/128][16]. The one-token matvec kernels read the
- * signs in a layout of their own: `bits` = bp_op_q1_relayout(qs), same size as `qs`. */
+ * signs in a layout of their own: `bits` = bp_op_q1_relayout(qs), same size as `qs`.
+ * Alignment, checked before anything is launched (BP_ERR_CUDA): 16 bytes for `bits`, for bp_op_q1_relayout's arrays,
+ * x of bp_op_matvec_q1_0, x of bp_op_embed, x and qs_out of bp_op_quantize_q8_0; 8 for x, w_norm, gate and up of the
+ * other matvecs; 4 for the logits of bp_op_topk_reduce and every f32 / uint32 array; 2 for every other f16 array. */
 int bp_op_q1_relayout(void* stream, const void* qs, void* bits_out, uint64_t n_blocks);
 /* dispatch_matvec_q1_0 (src/forward.rs:212-248, matvec_q1_0.wgsl): y[n] (+)= W x */
 int bp_op_matvec_q1_0(void* stream, const void* d, const void* bits, uint32_t k, uint32_t n, const void* x, void* y,

@@ -93,6 +93,35 @@ def test_matvec_fused_normed_bit_exact(k, ns):
         lib.bp_op_set_matvec_rows(0)
 
 
+def test_operators_refuse_addresses_that_their_kernels_cannot_take():
+    """The alignment stated in include/bonsai_model.h is checked on the host: nothing is launched."""
+    lib = _lib.load()
+    p = torch.zeros(1 << 16, dtype=torch.uint8, device="cuda").data_ptr()
+    one = lambda v: (C.c_void_p * 1)(v)
+    n16 = (C.c_uint32 * 1)(16)
+    refused = [
+        lambda: lib.bp_op_q1_relayout(None, p + 8, p, 1),
+        lambda: lib.bp_op_q1_relayout(None, p, p + 8, 1),
+        lambda: lib.bp_op_matvec_q1_0(None, p, p, 128, 1, p + 8, p, 0),
+        lambda: lib.bp_op_matvec_q1_0(None, p, p + 8, 128, 1, p, p, 0),
+        lambda: lib.bp_op_matvec_q1_0(None, p + 1, p, 128, 1, p, p, 0),
+        lambda: lib.bp_op_matvec_q1_0_fused_normed(None, 128, p + 4, p, 1e-6, 1, one(p), one(p), n16, one(p)),
+        lambda: lib.bp_op_matvec_q1_0_fused_normed(None, 128, p, p + 2, 1e-6, 1, one(p), one(p), n16, one(p)),
+        lambda: lib.bp_op_matvec_q1_0_fused_normed(None, 128, p, p, 1e-6, 1, one(p), one(p + 4), n16, one(p)),
+        lambda: lib.bp_op_matvec_q1_0_silu(None, p, p, 128, 1, p + 4, p, p, 0),
+        lambda: lib.bp_op_matvec_q1_0_silu(None, p, p, 128, 1, p, p + 2, p, 0),
+        lambda: lib.bp_op_rms_norm(None, p + 1, p, p, 128, 1, 1e-6),
+        lambda: lib.bp_op_silu_mul(None, p + 1, p, p, 8),
+        lambda: lib.bp_op_embed(None, p, p, 128, p, 1, p + 8),
+        lambda: lib.bp_op_quantize_q8_0(None, p, 128, 1, p + 2, p),
+        lambda: lib.bp_op_quantize_q8_0(None, p, 128, 1, p, p + 8),
+        lambda: lib.bp_op_topk_reduce(None, p + 2, 64, 1, p, p),
+    ]
+    for i, call in enumerate(refused):
+        assert call() == bp.errors.BP_ERR_CUDA, i
+    torch.cuda.synchronize()  # (no error was left behind)
+
+
 @pytest.mark.parametrize("k,n", [(12288, 4096), (1536, 512), (9728, 24)])
 def test_matvec_silu_bit_exact(k, n):
     rng = np.random.default_rng(k)
