@@ -1232,12 +1232,45 @@ __device__ __forceinline__ bool tk_fast(TkFast& f, TkEntry* rows, const __half* 
   __syncthreads();
   const float bound = f.bound_k;  // NONE when fewer than k warps have an element: everything counts
   TkFast* f0 = cluster.map_shared_rank(&f, 0);
-  scan([&](float v, uint32_t i) {
-    if (v >= bound && v > NONE) {
-      const uint32_t at = atomicAdd(&f0->n_cand, 1u);
-      if (at < TK_CAND) f0->cand[at] = TkEntry{v, i};
+  // One addition to the first CTA's count per warp and batch, none once the count is over TK_CAND: with one per
+  // element, logits that are all equal sent 151936 of them to one address (49 us per call, 43 now, the lists alone 39; 600
+  // logits at the maximum 96.5, 92, 88).
+  for (uint32_t w0 = first; w0 - lane < n_words; w0 += BATCH * stride) {
+    __half2 p[BATCH];
+#pragma unroll
+    for (uint32_t u = 0; u < BATCH; u++) p[u] = w0 + u * stride < n_words ? __ldg(reinterpret_cast<const __half2*>(logits) + w0 + u * stride) : __half2();
+    uint32_t take = 0;
+#pragma unroll
+    for (uint32_t u = 0; u < BATCH; u++) {
+      const uint32_t i0 = 2 * (w0 + u * stride);
+      const float lo = __low2float(p[u]), hi = __high2float(p[u]);
+      if (i0 < n && lo >= bound && lo > NONE) take |= 1u << (2 * u);
+      if (i0 + 1 < n && hi >= bound && hi > NONE) take |= 2u << (2 * u);
     }
-  });
+    if (!__any_sync(FULL, take != 0)) continue;
+    uint32_t upto = __popc(take);  // elements of the lanes up to this one
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const uint32_t below = __shfl_up_sync(FULL, upto, off);
+      if (lane >= static_cast<uint32_t>(off)) upto += below;
+    }
+    uint32_t at = lane == 31 ? atomicAdd(&f0->n_cand, upto) : 0u;
+    at = __shfl_sync(FULL, at, 31);
+    if (at >= TK_CAND) break;  // (with this warp's the count is above it)
+    at += upto - __popc(take);
+#pragma unroll
+    for (uint32_t u = 0; u < BATCH; u++) {
+      const uint32_t i0 = 2 * (w0 + u * stride);
+      if (take >> (2 * u) & 1u) {
+        if (at < TK_CAND) f0->cand[at] = TkEntry{__low2float(p[u]), i0};
+        at++;
+      }
+      if (take >> (2 * u) & 2u) {
+        if (at < TK_CAND) f0->cand[at] = TkEntry{__high2float(p[u]), i0 + 1};
+        at++;
+      }
+    }
+  }
   cluster.sync();
   if (rank == 0) {
     const uint32_t c = f.n_cand;

@@ -472,7 +472,7 @@ def test_session_behaviour_of_the_reference_integration_tests(tmp_path):
 
 
 @pytest.mark.parametrize("n", [32, 33, 511, 512, 2047, 4097, 30001, 151936])
-@pytest.mark.parametrize("kind", ["distinct", "few ties", "many ties", "one list", "specials"])
+@pytest.mark.parametrize("kind", ["distinct", "few ties", "many ties", "one list", "specials", "equal", "512 at the top", "513 at the top"])
 def test_topk_reduce_selects_what_the_lists_select(n, kind):
     """Distinct logits and ties across lists take the selection, ties inside a list the heaps: the shader's
     values and indices either way. Not a number and infinities; all candidates in one list; signed zeros."""
@@ -490,6 +490,10 @@ def test_topk_reduce_selects_what_the_lists_select(n, kind):
         logits[rng.integers(0, n, 40)] = logits.max()
     if kind == "many ties":
         logits = np.round(logits)
+    if kind == "equal":
+        logits[:] = np.float16(0.75)
+    if kind.endswith("at the top"):  # as many candidates as are collected, and one more
+        logits[rng.permutation(n)[:int(kind[:3])]] = np.float16(30.0)
     if kind == "specials":
         logits[rng.integers(0, n, n // 3)] = np.nan
         logits[rng.integers(0, n, 3)] = -np.inf
