@@ -878,7 +878,10 @@ int bp_model_prefill_loop_topk(bp_model* m, const uint32_t* tokens, uint32_t n, 
   const bool graph = m->step_graph && m->tap_mode == 0 && bp_use_umma(m->attn) && (m->fill.valid || n - 1 >= FILL_GRAPH_MIN);
   for (uint32_t i = 0; i + 1 < n; i++)  // KV-fill-only steps: no output suffix (src/forward.rs:947-965)
     if (graph) {
-      M_CUDA(m, cudaMemcpyAsync(m->tokens_dev, tokens + i, sizeof(uint32_t), cudaMemcpyHostToDevice, m->stream));
+      // from a copy on the stack: out of the caller's array, if that is pinned, the token could still be read after an
+      // error has ended the call
+      const uint32_t token = tokens[i];
+      M_CUDA(m, cudaMemcpyAsync(m->tokens_dev, &token, sizeof token, cudaMemcpyHostToDevice, m->stream));
       if (int st = launch_step_graph(m, m->fill, pos_base + i)) return st;
     } else if (int st = step_no_suffix(m, tokens[i], pos_base + i)) {
       return st;
