@@ -292,7 +292,7 @@ struct bp_model {
     bool valid = false;
   } sg, fill;                 // fill: the same without the output suffix (a token whose logits nobody asks for)
   bool step_graph = true;     // bp_model_set_step_graph
-  uint64_t graph_steps = 0;   // steps that ran as a graph launch
+  uint64_t graph_steps = 0;   // steps that went to the device as a graph launch, of either graph
   uint32_t* token_pin = nullptr;  // pinned: the token of the step (read by the graph's copy node)
   float* res_val_pin = nullptr;   // pinned: top-k results of the step
   uint32_t* res_idx_pin = nullptr;
@@ -526,6 +526,7 @@ int launch_step_graph(bp_model* m, bp_model::StepGraph& g, uint32_t pos) {
   if (!patched)
     if (int st = capture_step_graph(m, g, pos)) return st;
   M_CUDA(m, cudaGraphLaunch(g.exec, m->stream));
+  m->graph_steps++;
   return BP_OK;
 }
 
@@ -533,7 +534,6 @@ int step_topk_graph(bp_model* m, uint32_t token, uint32_t pos, uint32_t k, float
   *m->token_pin = token;
   if (int st = launch_step_graph(m, m->sg, pos)) return st;
   M_CUDA(m, cudaStreamSynchronize(m->stream));
-  m->graph_steps++;
   for (uint32_t i = 0; i < k; i++) {
     logits[i] = m->res_val_pin[i];
     indices[i] = m->res_idx_pin[i];

@@ -108,7 +108,7 @@ int bp_model_step_topk(bp_model* m, uint32_t token, uint32_t pos, uint32_t k, fl
  * the stream launches; enable = 0 returns to those. The graph is used with the tcgen05 decode kernel
  * (4 query heads per KV head, kernel family 0) and while the attention tap is off. */
 int bp_model_set_step_graph(bp_model* m, uint32_t enable);
-/* Steps that ran as a graph launch since the model was loaded. */
+/* Steps that ran as a graph launch since the model was loaded (the tokens of bp_model_prefill_loop_topk among them). */
 uint64_t bp_model_graph_steps(const bp_model* m);
 /* prefill_matmul_topk (src/forward.rs:975-1073; layer_step_matmul_in_pass :1075-1253): n <= m_max tokens at positions 0 .. n - 1, batched. */
 int bp_model_prefill_topk(bp_model* m, const uint32_t* tokens, uint32_t n, uint32_t k, float* logits, uint32_t* indices);

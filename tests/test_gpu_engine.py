@@ -594,19 +594,28 @@ def test_tiled_product_is_identical_to_the_cuda_core_product(tmp_path, m):
             assert np.array_equal(a.view(np.uint8), b.view(np.uint8)), variant
 
 
-def test_incremental_prefill_is_identical_as_graph_and_as_stream_launches(tmp_path):
+@pytest.mark.parametrize("exclusive_device", [1, 0])
+def test_incremental_prefill_is_identical_as_graph_and_as_stream_launches(tmp_path, exclusive_device):
+    """The tokens whose logits nobody asks for as launches of the fill graph, the last one as the step graph. With
+    exclusive_device = 0 an attention call becomes two launches at 257 keys: the fill graph is then captured again
+    while its earlier launches are still queued."""
     d = str(tmp_path / "m")
     model_dir.write_synthetic_model(d, seed=5)
-    toks = [(17 * i + 2) % 2000 for i in range(150)]
+    n = 150 if exclusive_device else 330
+    toks = [(17 * i + 2) % 2000 for i in range(n)]
     got = []
     for graph in (True, False):
-        with bp.Model(d, max_seq=256) as gm:
+        with bp.Model(d, max_seq=512) as gm:
             gm.set_step_graph(graph)
+            gm.attention().set_option("exclusive_device", exclusive_device)
             s = gm.new_session()
             rows = []
-            for a, b in ((0, 2), (2, 6), (6, 7), (7, 150)):  # below the length that makes the graph, at it, one token, across stages
+            steps = 0
+            for a, b in ((0, 2), (2, 6), (6, 7), (7, n)):  # below the length that makes the graph, at it, one token, across stages
                 s.prefill_one_at_a_time(toks[a:b], greedy())
                 rows.append(gm.logits().copy())
+                steps += 1 if a == 0 else b - a
+                assert gm.graph_steps() == (steps if graph else 0)
             rows.append(np.frombuffer(s.snapshot().to_bytes(), dtype=np.uint8))
             got.append(rows)
     for a, b in zip(*got):
