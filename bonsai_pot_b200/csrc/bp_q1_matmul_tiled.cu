@@ -479,11 +479,7 @@ cudaError_t bp_q1_silu_quantize_tiled(bool pdl, cudaStream_t s, const __half* ga
 cudaError_t bp_q1_matmul_tiled(bool pdl, cudaStream_t s, const bp_q1_tensor* w, __half* const* y, uint32_t n_w, uint32_t m, const uint8_t* a_t,
                                const float* a_d, bool accumulate, uint32_t* err, uint32_t wait_limit) {
   if (n_w == 0 || n_w > 3) return cudaErrorInvalidValue;
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 1;
-  }
+  const uint32_t sms = bp_q1_sm_count();
   // The width of a tile: waves of one CTA per SM, times what a block of a tile of that width takes (us, measured).
   const uint32_t widths[5] = {32, 28, 24, 16, 8};
   const float cost[5] = {2.15f, 1.79f, 1.66f, 1.34f, 1.17f};

@@ -17,10 +17,25 @@
 #include <cuda_fp16.h>
 #include <math.h>
 
+#include <atomic>
+
 #include "bp_common.cuh"
 #include "bp_ptx.cuh"
 #include "bp_q1_device.cuh"
 #include "bp_q1_ops.cuh"
+
+// Asked once per device: a process may hold models on devices of different sizes.
+uint32_t bp_q1_sm_count() {
+  static std::atomic<int> count[64];
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1;
+  n = count[dev].load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 1;
+    count[dev].store(n, std::memory_order_relaxed);
+  }
+  return static_cast<uint32_t>(n);
+}
 
 namespace {
 
@@ -1504,13 +1519,8 @@ cudaError_t launch_mv_r(bool pdl, cudaStream_t s, const MvParams& p) {
 // a row per warp; 6144: 3 of 14; 12288 pairs: 2 of 14, three pairs per warp.
 template <int MODE, uint32_t PASSES>
 cudaError_t launch_mv_wide(bool pdl, cudaStream_t s, const MvParams& p) {
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 1;
-  }
   constexpr uint32_t MAX_WARPS = mvw_ctas<MODE, PASSES>() * MVW_WARPS;
-  const uint32_t items = MODE == 3 ? p.r[0].n : p.n_total, n_sm = static_cast<uint32_t>(sms);
+  const uint32_t items = MODE == 3 ? p.r[0].n : p.n_total, n_sm = bp_q1_sm_count();
   const uint32_t per_sm = (items + n_sm - 1) / n_sm, per_warp = (per_sm + MAX_WARPS - 1) / MAX_WARPS;
   const uint32_t warps = (per_sm + per_warp - 1) / per_warp, ctas = (warps + MVW_WARPS - 1) / MVW_WARPS;
   uint32_t w = (warps + ctas - 1) / ctas;
@@ -1707,12 +1717,7 @@ static cudaError_t launch_mma(bool pdl, cudaStream_t s, const bp_q1_tensor* w, _
   // the same), or full tiles for as many whole waves of one CTA per SM as there are and half tiles for the rest
   // in a second launch (gate + up at 512 tokens: 768 full tiles are 5.2 waves; 740 full tiles and 56 half tiles
   // are 5 waves and a short one): whichever needs the least time.
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 1;
-  }
-  const uint32_t n_sm = static_cast<uint32_t>(sms), m_full = (m + 127) / 128, m_half = (m + 63) / 64;
+  const uint32_t n_sm = bp_q1_sm_count(), m_full = (m + 127) / 128, m_half = (m + 63) / 64;
   auto waves = [&](uint32_t ctas) { return static_cast<float>((ctas + n_sm - 1) / n_sm); };
   constexpr float HALF_COST = 0.62f;
   const float t_full = waves(tiles * m_full), t_half = HALF_COST * waves(tiles * m_half);
