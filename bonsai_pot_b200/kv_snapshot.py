@@ -50,11 +50,14 @@ class KvSnapshot:
 
     @property
     def payload(self) -> bytes:
-        return self._blob[HEADER_BYTES:]
+        if self._payload is None:  # cut out of the blob at the first read and kept: it may be tens of megabytes
+            self._payload = self._blob[HEADER_BYTES:]
+        return self._payload
 
     @payload.setter
     def payload(self, payload):
-        self._blob = MAGIC + struct.pack("<6I", VERSION, self._n_layer, self._kv_dim, self._max_seq, self._pos, 0) + bytes(payload)
+        self._payload = bytes(payload)
+        self._blob = MAGIC + struct.pack("<6I", VERSION, self._n_layer, self._kv_dim, self._max_seq, self._pos, 0) + self._payload
 
     def to_bytes(self) -> bytes:
         """src/kv_snapshot.rs:69-80."""
@@ -76,7 +79,7 @@ class KvSnapshot:
             raise ConfigError("invalid config: KvSnapshot blob payload length does not match header")
         snap = cls.__new__(cls)
         snap._n_layer, snap._kv_dim, snap._max_seq, snap._pos = n_layer, kv_dim, max_seq, pos
-        snap._blob = bytes(blob)  # (a `bytes` is kept as it is)
+        snap._blob, snap._payload = bytes(blob), None  # (a `bytes` is kept as it is)
         return snap
 
     def clone(self) -> "KvSnapshot":

@@ -81,6 +81,7 @@ def test_kvsnapshot_value_type():
                    lambda b: b[:28] + b"\x01" + b[29:], lambda b: b[:16]):
         with pytest.raises(bp.ConfigError):
             bp.KvSnapshot.from_bytes(mutate(blob))
+    assert back.payload is back.payload and snap.payload is snap.payload  # reading it does not copy it
     clone = snap.clone()
     clone.payload = b"\x00" + clone.payload[1:]
     assert snap.payload[0:1] != b"\x00" or snap.payload == payload
