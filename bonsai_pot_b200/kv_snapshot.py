@@ -25,15 +25,16 @@ def payload_offset(n_layer, kv_dim, pos, kind, il, sect):
     return int(_lib.load().bp_snapshot_payload_offset(n_layer, kv_dim, pos, kind, il, sect))
 
 
+# Prototypes of this module's own: the attributes of `ctypes.pythonapi` are shared with everything else in the process.
+_bytes_new = C.PYFUNCTYPE(C.py_object, C.c_char_p, C.c_ssize_t)(("PyBytes_FromStringAndSize", C.pythonapi))
+_bytes_address = C.PYFUNCTYPE(C.c_void_p, C.py_object)(("PyBytes_AsString", C.pythonapi))
+
+
 def new_blob(size):
     """An uninitialised `bytes` object and the address of its bytes, for a call that fills it: a capture then
     touches every page of the blob once (zeroing a buffer and copying it out took longer than the transfer)."""
-    new = C.pythonapi.PyBytes_FromStringAndSize
-    new.restype, new.argtypes = C.py_object, [C.c_char_p, C.c_ssize_t]
-    address = C.pythonapi.PyBytes_AsString
-    address.restype, address.argtypes = C.c_void_p, [C.py_object]
-    blob = new(None, size)
-    return blob, address(blob)
+    blob = _bytes_new(None, size)
+    return blob, _bytes_address(blob)
 
 
 class KvSnapshot:

@@ -87,6 +87,15 @@ def test_kvsnapshot_value_type():
     assert snap.payload[0:1] != b"\x00" or snap.payload == payload
 
 
+def test_new_blob_leaves_the_shared_prototypes_alone():
+    shared = C.pythonapi.PyBytes_FromStringAndSize, C.pythonapi.PyBytes_AsString
+    before = [(f.restype, f.argtypes) for f in shared]
+    blob, address = kv_snapshot.new_blob(100)
+    assert [(f.restype, f.argtypes) for f in shared] == before
+    C.memmove(address, bytes(range(100)), 100)
+    assert type(blob) is bytes and blob == bytes(range(100))
+
+
 def test_strerror_and_null_handling():
     lib = _lib.load()
     assert lib.bp_strerror(0) == b"ok"
