@@ -290,9 +290,10 @@ def test_topk_reduce_identical_including_ties(n, k, ties):
 
 # ----------------------------------------------------------------- forward passes ----
 WIDE = dict(n_layer=2, n_embd=4096, n_ff=12288, n_head=32, n_kv_head=8, head_dim=128, n_vocab=151936)  # Bonsai-8B widths
+PARTLY = dict(n_layer=1, n_embd=3200, n_ff=6272, n_head=4, n_kv_head=1, head_dim=128, n_vocab=512)  # 25 and 49 blocks: last passes of 25 and 17 lanes
 
 
-@pytest.mark.parametrize("shape", [None, WIDE])
+@pytest.mark.parametrize("shape", [None, WIDE, PARTLY])
 def test_one_token_pass_matches_the_cpu_pass_bit_for_bit(tmp_path, shape):
     """Several decode steps. The GPU pass records its attention outputs; the CPU pass uses them in place of its
     own attention (both write the same cache rows), so every other operator must reproduce the residual stream,
@@ -537,10 +538,12 @@ def test_large_snapshots_hold_the_cache_rows(pos):
         assert bp.KvSnapshot.from_bytes(snap.to_bytes()).clone().payload == snap.payload
 
 
-@pytest.mark.parametrize("k,n", [(3072, 17), (4096, 4096), (4096 + 128, 600), (8192, 15), (12288, 4096), (16384, 301), (4096, 16383)])
+@pytest.mark.parametrize("k,n", [(3072, 17), (3200, 17), (4096, 4096), (4096 + 128, 600), (4096 + 128, 4096), (6272, 4096), (8192, 15),
+                                 (9344, 6144), (12288, 4096), (16384, 301), (4096, 16383)])
 def test_warp_per_row_matvec_is_identical_to_eight_lanes_per_row(k, n):
-    """The warp-per-row kernel at its limits (24 and 128 blocks, a partly filled last pass, few rows, several rows per
-    warp) against the kernel it replaces there: plain, accumulating, and the normed ranges."""
+    """The warp-per-row kernel at its limits (25 and 128 blocks, a partly filled last pass, few rows, several rows per
+    warp; 24 blocks and 33 blocks of many rows are left to the other) against the kernel it replaces there: plain,
+    accumulating, and the normed ranges."""
     rng = np.random.default_rng(k * 7 + n)
     _, _, _, d_dev, _, bits = random_q1(rng, k, n)
     n3 = (16, 48, 16)
