@@ -387,22 +387,23 @@ def test_free_running_passes_agree_on_the_top_candidates(tmp_path):
 
 
 def test_batched_prefill_is_identical_across_matmul_kernels(tmp_path):
-    """A 40-token prefill takes the tensor-core matmul (one launch for Q, K and V, one for gate and up); the
-    CUDA-core kernel and the tcgen05 kernel must give the same bits all the way to the logits."""
+    """A 40-token prefill takes the tiled product, or a forced kernel on untiled activations: the CUDA cores, mma.sync
+    (one launch for Q, K and V, one for gate and up; tiles by size, of 64 and of 128 tokens) or tcgen05 with f16
+    operands. The same bits all the way to the logits."""
     d = str(tmp_path / "m")
     model_dir.write_synthetic_model(d, seed=5)
     prompt = [(7 * i + 3) % 200 for i in range(40)]
     lib = _lib.load()
     got = {}
     try:
-        for variant in (1, 0, 3, 4, 5):
+        for variant in (1, 0, 2, 3, 4, 5):
             lib.bp_op_set_matmul_variant(variant)
             with bp.Model(d, max_seq=64) as gm:
                 lg, ix = gm.prefill_topk(prompt)
                 got[variant] = (lg.copy(), ix.copy(), gm.hidden(len(prompt) - 1).copy(), gm.logits().copy())
     finally:
         lib.bp_op_set_matmul_variant(0)
-    for variant in (0, 3):
+    for variant in (0, 2, 3, 4, 5):
         for a, b in zip(got[1], got[variant]):
             assert np.array_equal(a.view(np.uint8), b.view(np.uint8)), variant
 
@@ -595,6 +596,94 @@ def test_tiled_product_is_identical_to_the_cuda_core_product(tmp_path, m):
     for variant, rows in got.items():
         for a, b in zip(got[1], rows):
             assert np.array_equal(a.view(np.uint8), b.view(np.uint8)), variant
+
+
+def edit_tensors(path, change):
+    """Calls change(name, dtype, parts) for every tensor of a model directory and writes the arrays back: parts is
+    (values,) of an F16 tensor, (scales [n][blocks], signs [n][blocks][16]) of a Q1_0 tensor."""
+    entries, cur = {}, None
+    for line in open(os.path.join(path, "config.ini")).read().split("\n"):
+        if line.startswith("["):
+            cur = entries.setdefault(line[1:-1], {})
+        elif cur is not None and " = " in line:
+            key, _, value = line.partition(" = ")
+            cur[key] = value
+    for name, e in entries.items():
+        f = np.memmap(os.path.join(path, e["buffer"]), dtype=np.uint8, mode="r+")
+        shape = [int(v) for v in e["shape"].split(",")]
+        if e["dtype"] == "F16":
+            o = int(e["offset"])
+            change(name, "F16", (f[o:o + 2 * shape[0]].view(np.float16),))
+        else:
+            n, nb, o, q = shape[1], int(e["nb"]), int(e["d_offset"]), int(e["qs_offset"])
+            change(name, "Q1_0", (f[o:o + 2 * n * nb].view(np.float16).reshape(n, nb), f[q:q + 16 * n * nb].reshape(n, nb, 16)))
+        f.flush()
+
+
+def prefill_rows(path, prompt, variant, rows):
+    lib = _lib.load()
+    try:
+        lib.bp_op_set_matmul_variant(variant)
+        with bp.Model(path, max_seq=len(prompt)) as gm:
+            gm.prefill_topk(prompt)
+            return [gm.logits()] + [gm.hidden(r) for r in rows]
+    finally:
+        lib.bp_op_set_matmul_variant(0)
+
+
+@pytest.mark.parametrize("m", [5, 130])
+def test_tiled_product_at_the_largest_integer_dots_and_the_8b_block_counts(tmp_path, m):
+    """32 and 96 blocks of 128 inputs; activations of equal magnitude (every quant +-127) against weights of the same
+    and of the opposite signs, constant and mixed: the partial sums of the FP32 accumulators reach +-127 * 32."""
+    d = str(tmp_path / "m")
+    model_dir.write_synthetic_model(d, shape=dict(n_layer=1, n_embd=4096, n_ff=12288, n_head=32, n_kv_head=8, head_dim=128, n_vocab=512), seed=7)
+    pattern = np.random.default_rng(3).integers(0, 256, (32, 16), dtype=np.uint8)
+
+    def change(name, dtype, parts):
+        if dtype == "F16":
+            return
+        scales, signs = parts
+        scales[:] = np.float16(0.001 if "ffn_down" in name else 0.01)
+        if name == "blk.0.attn_v.weight":  # equal rows: attention outputs of equal magnitude
+            signs[:] = 0xFF
+        elif name in ("blk.0.ffn_gate.weight", "blk.0.ffn_up.weight"):  # as the residual stream's signs alternate behind Wo
+            signs[:] = 0x55
+        else:
+            signs[0::2], signs[1::2] = 0xFF, 0x00
+            if name != "token_embd.weight" and signs.shape[1] == 32:
+                signs[4], signs[5] = pattern, ~pattern
+            elif name == "token_embd.weight":
+                signs[2], signs[3] = pattern, ~pattern
+
+    edit_tensors(d, change)
+    prompt = [(i + 1) % 6 for i in range(m)]
+    want = prefill_rows(d, prompt, 1, (0, 1, 2, m - 1))
+    assert not np.isnan(np.array(want[1:], dtype=np.float32)).any() and all(len(np.unique(r)) > 1 for r in want)
+    for variant in (0, 6, 8, 10):
+        for a, b in zip(want, prefill_rows(d, prompt, variant, (0, 1, 2, m - 1))):
+            assert np.array_equal(a.view(np.uint16), b.view(np.uint16)), variant
+
+
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan])
+def test_tiled_product_with_infinite_and_undefined_activations(tmp_path, bad):
+    """A norm weight that is not finite puts one such value into a sub-block of every token (amax ignores NaN, an
+    infinite one makes the scale infinite): the bits of the CUDA-core path, for the last tokens of a partly filled
+    tile too. The rows of the tile that hold no token must not reach any output."""
+    d = str(tmp_path / "m")
+    model_dir.write_synthetic_model(d, shape=RAGGED, seed=13)
+
+    def change(name, dtype, parts):
+        if name == "blk.0.ffn_norm.weight":
+            parts[0][133] = bad
+
+    edit_tensors(d, change)
+    prompt = [(13 * i + 5) % 500 for i in range(131)]
+    rows = (0, 64, 127, 128, 130)
+    want = prefill_rows(d, prompt, 1, rows)
+    assert np.isfinite(np.array(want[1:], dtype=np.float32)).all() == np.isnan(bad)  # (NaN quantises to -127)
+    for variant in (0, 6, 7, 8, 9, 10):
+        for a, b in zip(want, prefill_rows(d, prompt, variant, rows)):
+            assert np.array_equal(a.view(np.uint16), b.view(np.uint16)), variant
 
 
 @pytest.mark.parametrize("exclusive_device", [1, 0])
