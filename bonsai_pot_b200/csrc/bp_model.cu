@@ -10,6 +10,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
 #include <limits>
 #include <map>
 #include <new>
@@ -270,12 +271,15 @@ struct bp_model {
   bp_q1_tensor embed, lm_head;
   const __half* output_norm = nullptr;
   // activations (ActLayout, src/model.rs:287-333), f16 [m_max][...] each
-  __half *x = nullptr, *x_norm = nullptr, *q = nullptr, *k_cur = nullptr, *v_cur = nullptr, *attn_out = nullptr, *gate = nullptr,
-         *up = nullptr, *ffn_in = nullptr, *logits = nullptr, *q_roped = nullptr;
-  float* a_d = nullptr;        // Q8_0 activations: scales [m_max][n_ff / 32]
-  int8_t* a_qs = nullptr;      //                  quants [m_max][n_ff]
+  __half *x = nullptr, *q = nullptr, *k_cur = nullptr, *v_cur = nullptr, *attn_out = nullptr, *gate = nullptr,
+         *up = nullptr, *logits = nullptr, *q_roped = nullptr;
+  __half* ffn_in = nullptr;    // one-token path: silu(gate) * up, [n_ff]
   uint8_t* a_tiled = nullptr;  // Q8_0 activations of a batch as the tiled product reads them
   float* a_tiled_d = nullptr;
+  // a batch through the other products (bp_op_set_matmul_variant): made by the first one, see untiled_buffers
+  __half *x_norm = nullptr, *silu_up = nullptr;
+  float* a_d = nullptr;        // Q8_0 activations: scales [m_max][k_max / 32]
+  int8_t* a_qs = nullptr;      //                  quants [m_max][k_max]
   uint32_t* tokens_dev = nullptr;
   float* topk_val = nullptr;
   uint32_t* topk_idx = nullptr;
@@ -541,6 +545,17 @@ int step_topk_graph(bp_model* m, uint32_t token, uint32_t pos, uint32_t k, float
   return device_status(m);
 }
 
+uint32_t k_max(const Config& c) { return std::max(c.n_embd, std::max(c.n_ff, c.q_dim)); }
+
+int untiled_buffers(bp_model* m) {
+  const size_t mm = M_MAX, k = k_max(m->cfg);
+  if (!m->x_norm) M_CUDA(m, cudaMalloc(&m->x_norm, mm * m->cfg.n_embd * 2));
+  if (!m->silu_up) M_CUDA(m, cudaMalloc(&m->silu_up, mm * m->cfg.n_ff * 2));
+  if (!m->a_d) M_CUDA(m, cudaMalloc(&m->a_d, mm * (k / 32) * sizeof(float)));
+  if (!m->a_qs) M_CUDA(m, cudaMalloc(&m->a_qs, mm * k));
+  return BP_OK;
+}
+
 // y[i] (+)= W[i] q8(act): the quantiser leaves the activations the way the product for this batch reads them, and
 // takes rms_norm (norm) or silu(act) * up with it where the product is the tiled one.
 int quantize_and_matmul(bp_model* m, const __half* act, uint32_t k, uint32_t mt, const bp_q1_tensor* w, __half* const* out, uint32_t n_w,
@@ -559,12 +574,13 @@ int quantize_and_matmul(bp_model* m, const __half* act, uint32_t k, uint32_t mt,
     M_CUDA(m, bp_q1_matmul_tiled(true, s, w, out, n_w, mt, m->a_tiled, m->a_tiled_d, accumulate, err, limit));
     return BP_OK;
   }
+  if (int st = untiled_buffers(m)) return st;
   if (norm != nullptr) {
     M_CUDA(m, bp_q1_rms_norm(true, s, act, m->x_norm, norm, k, mt, m->cfg.rms_eps));
     act = m->x_norm;
   } else if (up != nullptr) {
-    M_CUDA(m, bp_q1_silu_mul(true, s, act, up, m->ffn_in, static_cast<uint64_t>(mt) * k));
-    act = m->ffn_in;
+    M_CUDA(m, bp_q1_silu_mul(true, s, act, up, m->silu_up, static_cast<uint64_t>(mt) * k));
+    act = m->silu_up;
   }
   M_CUDA(m, bp_q1_quantize_q8(true, s, act, k, mt, m->a_d, m->a_qs));
   M_CUDA(m, bp_q1_matmul_multi(true, s, w, out, n_w, mt, m->a_d, m->a_qs, accumulate, err, limit));
@@ -776,7 +792,6 @@ int bp_model_load(const char* dir, uint32_t max_seq, int32_t device, bp_model** 
   m->output_norm = f16_view(m, "output_norm.weight");
   const size_t mm = M_MAX;
   M_CUDA(m, cudaMalloc(&m->x, mm * c.n_embd * 2));
-  M_CUDA(m, cudaMalloc(&m->x_norm, mm * c.n_embd * 2));
   M_CUDA(m, cudaMalloc(&m->q, mm * c.q_dim * 2));
   M_CUDA(m, cudaMalloc(&m->q_roped, static_cast<size_t>(c.q_dim) * 2));
   M_CUDA(m, cudaMalloc(&m->k_cur, mm * c.kv_dim * 2));
@@ -784,13 +799,10 @@ int bp_model_load(const char* dir, uint32_t max_seq, int32_t device, bp_model** 
   M_CUDA(m, cudaMalloc(&m->attn_out, mm * c.q_dim * 2));
   M_CUDA(m, cudaMalloc(&m->gate, mm * c.n_ff * 2));
   M_CUDA(m, cudaMalloc(&m->up, mm * c.n_ff * 2));
-  M_CUDA(m, cudaMalloc(&m->ffn_in, mm * c.n_ff * 2));
+  M_CUDA(m, cudaMalloc(&m->ffn_in, static_cast<size_t>(c.n_ff) * 2));
   M_CUDA(m, cudaMalloc(&m->logits, (static_cast<size_t>(c.n_vocab) + 2) * 2));
-  const uint32_t k_max = c.n_ff > c.q_dim ? (c.n_ff > c.n_embd ? c.n_ff : c.n_embd) : (c.q_dim > c.n_embd ? c.q_dim : c.n_embd);
-  M_CUDA(m, cudaMalloc(&m->a_d, mm * (k_max / 32) * sizeof(float)));
-  M_CUDA(m, cudaMalloc(&m->a_qs, mm * k_max));
-  M_CUDA(m, cudaMalloc(&m->a_tiled, bp_q1_tiled_bytes(M_MAX, k_max)));
-  M_CUDA(m, cudaMalloc(&m->a_tiled_d, bp_q1_tiled_scales(M_MAX, k_max) * sizeof(float)));
+  M_CUDA(m, cudaMalloc(&m->a_tiled, bp_q1_tiled_bytes(M_MAX, k_max(c))));
+  M_CUDA(m, cudaMalloc(&m->a_tiled_d, bp_q1_tiled_scales(M_MAX, k_max(c)) * sizeof(float)));
   M_CUDA(m, cudaMalloc(&m->tokens_dev, mm * sizeof(uint32_t)));
   M_CUDA(m, cudaMalloc(&m->topk_val, TOPK_MAX * sizeof(float)));
   M_CUDA(m, cudaMalloc(&m->topk_idx, TOPK_MAX * sizeof(uint32_t)));
@@ -809,7 +821,7 @@ void bp_model_free(bp_model* m) {
   }
   for (auto p : m->dev_file) cudaFree(p);
   for (auto p : m->dev_bits) cudaFree(p);
-  void* bufs[] = {m->x, m->x_norm, m->q, m->q_roped, m->k_cur, m->v_cur, m->attn_out, m->gate, m->up, m->ffn_in, m->logits,
+  void* bufs[] = {m->x, m->x_norm, m->silu_up, m->q, m->q_roped, m->k_cur, m->v_cur, m->attn_out, m->gate, m->up, m->ffn_in, m->logits,
                   m->a_d, m->a_qs, m->a_tiled, m->a_tiled_d, m->tokens_dev, m->topk_val, m->topk_idx};
   for (void* p : bufs) cudaFree(p);
   drop_step_graphs(m);
