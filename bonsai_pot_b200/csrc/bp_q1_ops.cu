@@ -1692,21 +1692,24 @@ cudaError_t bp_q1_quantize_q8(bool pdl, cudaStream_t s, const __half* x, uint32_
   return bp_launch(pdl, quantize_q8_kernel, dim3(static_cast<unsigned>((n_blocks + 255) / 256)), dim3(256), 0, s, x, n_blocks, d_out, qs_out);
 }
 
-static uint32_t g_matmul_variant = 0;  // 0 = by batch size; 1 dp4a, 2 mma.sync, 3 tcgen05; 4 / 5 = mma.sync with 64- / 128-token tiles only; 6 .. 10 = a model's batches through the tiled product with 128, 112, 96, 64, 32 weight rows per tile
+// 0 = the default: a model's batches through the tiled product, untiled activations by alignment (op_variant); 1 dp4a,
+// 2 mma.sync, 3 tcgen05; 4 / 5 = mma.sync with 64- / 128-token tiles only; 6 .. 10 = as 0, the tiled product with 128,
+// 112, 96, 64, 32 weight rows per tile
+static uint32_t g_matmul_variant = 0;
 
 // The kernel for the untiled activations of bp_op_quantize_q8_0: mma.sync wherever its 16-byte reads of a_d and a_qs
 // are allowed (a pass of 21 tokens at the 8B shape takes 13.5 ms with it and 53 ms with the CUDA-core kernel, one
-// token 12.9 and 53), else the CUDA-core kernel, which reads 32-bit words. 0: no kernel can read these buffers, or
-// not the one that was forced.
+// token 12.9 and 53), else the CUDA-core kernel, which reads 32-bit words. Signs are read as 32-bit words, by the
+// tcgen05 kernel as 16-bit ones. 0: no kernel can read these buffers, or not the one that was forced.
 static uint32_t op_variant(const bp_q1_tensor* w, __half* const* y, uint32_t n_w, const float* a_d, const int8_t* a_qs) {
   const uintptr_t act = reinterpret_cast<uintptr_t>(a_d) | reinterpret_cast<uintptr_t>(a_qs);
-  if (act % 4u != 0) return 0;
-  for (uint32_t i = 0; i < n_w; i++)
-    if (reinterpret_cast<uintptr_t>(w[i].qs) % 4u != 0 || reinterpret_cast<uintptr_t>(w[i].d) % 2u != 0 || reinterpret_cast<uintptr_t>(y[i]) % 2u != 0) return 0;
-  if (g_matmul_variant == 0 || g_matmul_variant >= 6) return act % 16u == 0 ? 2u : 1u;
-  if (g_matmul_variant == 1) return 1;
-  if (act % 16u != 0) return 0;
-  return g_matmul_variant == 3 ? 3u : 2u;
+  const uint32_t variant = g_matmul_variant == 0 || g_matmul_variant >= 6 ? (act % 16u == 0 ? 2u : 1u) : g_matmul_variant >= 4 ? 2u : g_matmul_variant;
+  if (act % (variant == 1 ? 4u : 16u) != 0) return 0;
+  for (uint32_t i = 0; i < n_w; i++) {
+    if (reinterpret_cast<uintptr_t>(w[i].qs) % (variant == 3 ? 2u : 4u) != 0) return 0;
+    if (reinterpret_cast<uintptr_t>(w[i].d) % 2u != 0 || reinterpret_cast<uintptr_t>(y[i]) % 2u != 0) return 0;
+  }
+  return variant;
 }
 
 static cudaError_t launch_mma(bool pdl, cudaStream_t s, const bp_q1_tensor* w, __half* const* y, uint32_t n_w, uint32_t m, const float* a_d,

@@ -237,6 +237,9 @@ def test_matmul_serves_any_buffer_it_can_read_and_refuses_the_others(m):
             lib.bp_op_set_matmul_variant(variant)
             st, y = call(4, 0)
             assert st == bp.errors.BP_ERR_CUDA and not y.any(), variant
+        lib.bp_op_set_matmul_variant(3)  # (reads the signs as 16-bit words)
+        st, y = call(0, 0, 2)
+        assert st == 0 and bits_equal(y, want)
     finally:
         lib.bp_op_set_matmul_variant(0)
 
