@@ -387,7 +387,8 @@ cudaError_t attention_call(bp_model* m, uint32_t il, uint32_t pos) {
 // Which launches carry programmatic stream serialization was measured per kernel on the 8B shape (us per layer,
 // stream launches / graph replay): all four matvecs 55.0 / 53.2, all but the down projection 48.8 / 44.8, gate + up
 // only 49.9 / 41.1, none 51.2 / 42.3. The down projection's CTAs, resident early, take the SM slots that the
-// second wave of the gate + up launch is waiting for.
+// second wave of the gate + up launch is waiting for. (Measured with the 8-lane matvecs; the warp-per-row kernels that
+// these launches now run at that shape come in one wave, and the combinations have not been measured again.)
 int decode_layer(bp_model* m, uint32_t il, uint32_t pos, bool in_graph = false, std::vector<bp_launch_record>* attn_nodes = nullptr) {
   const Config& c = m->cfg;
   const LayerTensors& lt = m->layers[il];

@@ -165,7 +165,7 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
 //   warp 0, lane 0    issues the MMAs, G sub-blocks per hand-over, into one of two sets of G TMEM buffers
 // What bounds it (128 x 112 tile, cycles per sub-block, stamps in the kernel): 855, of them 510 the scaling and adding
 // (336 if only the FMA pipe counted), 220 the staging (its proxy fence above all), 120 waiting for the MMAs; the
-// tensor pipe is 13 % busy, the issue slots 60 %. A pass of 512 tokens at the Bonsai-8B shape: 37.9 ms with the
+// tensor pipe is 13 % busy, the issue slots 58 % (gate + up of 512 tokens under ncu). A pass of 512 tokens at the Bonsai-8B shape: 37.9 ms with the
 // mma.sync kernel, 29.2 now; 21 tokens: 53 ms with the CUDA-core kernel, 11.8 now. Slower (ms per 512-token pass): four
 // sets of one sub-block 32.6, the staging in four warps of its own 30.4, two issuing threads with the next
 // hand-over's first load before the last piece is added 30.8, scalar instead of packed sums and products: no change.
@@ -480,7 +480,9 @@ cudaError_t bp_q1_matmul_tiled(bool pdl, cudaStream_t s, const bp_q1_tensor* w, 
                                const float* a_d, bool accumulate, uint32_t* err, uint32_t wait_limit) {
   if (n_w == 0 || n_w > 3) return cudaErrorInvalidValue;
   const uint32_t sms = bp_q1_sm_count();
-  // The width of a tile: waves of one CTA per SM, times what a block of a tile of that width takes (us, measured).
+  // The width of a tile: waves of one CTA per SM, times what a block of a tile of that width takes: us, 512 tokens through
+  // the 8B shape's tensors, 96 blocks (down) to 32 (Q/K/V): 2.11 - 2.28, 1.79 - 1.96, 1.58 - 1.71, 1.23 - 1.36, 1.14 - 1.21.
+  // The choice was the fastest of the five widths for Q/K/V, Wo, gate + up and down at 21, 128, 173, 300 and 512 tokens.
   const uint32_t widths[5] = {32, 28, 24, 16, 8};
   const float cost[5] = {2.15f, 1.79f, 1.66f, 1.34f, 1.17f};
   float best = 1e30f;

@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(MV_THREADS) matvec_q1_kernel(const MvParams p)
 // from the lanes' block results, four shuffles and additions per 32 blocks. Against 8 lanes per row a row has four
 // times the threads: the 4096-row tensors fill an SM with 28 warps instead of 7, a CTA's activations are staged by
 // 448 threads instead of 128, and the chain of a lane is k / 4096 blocks instead of k / 1024. The 8-lane kernel was
-// bound by latency there (36 % of the issue slots): one-token step at the 8B shape 1288 -> 1209 us (position 100).
+// bound by latency there (36 % of the issue slots): one-token step at the 8B shape 1288 -> 1225 us (position 100).
 constexpr uint32_t MVW_WARPS = 14;  // warps of a CTA at most
 template <int MODE, uint32_t PASSES>
 constexpr uint32_t mvw_ctas() { return MODE == 3 || PASSES > 1 ? 2 : 3; }  // CTAs per SM that the registers of an instance allow

@@ -14,7 +14,7 @@ struct bp_q1_tensor {
   uint32_t k, n;
 };
 
-uint32_t bp_q1_sm_count();  // of the current device: what the grids of the persistent-style launches are cut for
+uint32_t bp_q1_sm_count();  // of the current device: what the grids are cut for
 void bp_q1_set_matvec_rows(uint32_t rows_per_lane);  // tuning aid: 0 = by tensor height, else 1, 2 or 4
 cudaError_t bp_q1_relayout(cudaStream_t s, const uint8_t* qs, void* out, uint64_t n_blocks);
 cudaError_t bp_q1_matvec(bool pdl, cudaStream_t s, const bp_q1_tensor& w, const __half* x, __half* y, bool accumulate);
@@ -46,6 +46,6 @@ cudaError_t bp_q1_rms_quantize_tiled(bool pdl, cudaStream_t s, const __half* x, 
 cudaError_t bp_q1_silu_quantize_tiled(bool pdl, cudaStream_t s, const __half* gate, const __half* up, uint32_t k, uint32_t m, uint8_t* a_t, float* a_d);
 cudaError_t bp_q1_matmul_tiled(bool pdl, cudaStream_t s, const bp_q1_tensor* w, __half* const* y, uint32_t n_w, uint32_t m, const uint8_t* a_t,
                                const float* a_d, bool accumulate, uint32_t* err, uint32_t wait_limit);
-void bp_q1_set_matmul_variant(uint32_t variant);  // tuning aid: 0 = by batch size (1 or 2), 1 = dp4a, 2 = mma.sync, 3 = tcgen05
+void bp_q1_set_matmul_variant(uint32_t variant);  // tuning aid, see bp_op_set_matmul_variant
 cudaError_t bp_q1_take_error(uint32_t* code);     // synchronous; 0 = no wait gave up since the last call
 cudaError_t bp_q1_topk(bool pdl, cudaStream_t s, const __half* logits, uint32_t n, uint32_t k, float* out_val, uint32_t* out_idx);

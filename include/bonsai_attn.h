@@ -220,7 +220,10 @@ uint64_t bp_snapshot_size(const bp_attn_ctx* ctx, uint32_t pos);
 /* `Session::snapshot` -> `KvSnapshot::to_bytes`: writes bp_snapshot_size bytes.
  * On a sharded context the blob is written in the GLOBAL row order: header
  * kv_dim = n_shards * local kv_dim, and only this shard's columns of each row
- * are touched, so n_shards calls on the same buffer assemble the full blob. */
+ * are touched, so n_shards calls on the same buffer assemble the full blob.
+ * The first blob of 2 MB or more that an unsharded context captures or applies
+ * makes four streams and 8 MB of pinned host memory that stay with the context
+ * until it is destroyed (without them, plain copies); four threads then copy. */
 int bp_snapshot_capture(bp_attn_ctx* ctx, uint32_t pos, void* blob, uint64_t blob_bytes);
 /* `KvSnapshot::from_bytes` + `validate_against` + `kv_snapshot::apply`
  * (src/kv_snapshot.rs:104-140, 184-199, 312-372). Returns the restored `pos`
