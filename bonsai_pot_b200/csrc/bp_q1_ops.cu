@@ -1534,16 +1534,16 @@ cudaError_t launch_mv_wide(bool pdl, cudaStream_t s, const MvParams& p) {
 // us per call, warp per row / 8 lanes, weights from HBM, back to back in a graph, plain: 24 blocks 3.6 / 3.4 (4096 rows)
 // and 6.4 / 5.8 (12288), 26 blocks 3.7 / 3.8 and 6.5 / 6.9; 36 blocks 4.8 / 4.4 and 9.7 / 8.3, 56 blocks 5.1 / 5.7 and
 // 10.0 / 10.8; 72 blocks 6.3 / 6.6 and 13.6 / 12.8, 80 blocks 6.4 / 7.2 and 13.7 / 14.0; 104 blocks 7.9 / 8.9 and
-// 17.5 / 18.6. So of `passes` passes fewer than `passes` groups of eight lanes may be idle in the last one. Up to 20
-// rows per SM the 8-lane kernel has too few warps to be the better one: 36 blocks and 1024 rows 2.5 / 3.0, 2560
-// rows 93 % of its time, from 3072 on 100 % and more. The paired mode at 32 blocks is no faster back to back (12288
-// pairs 10.3 / 10.3, 6144 pairs 7.1 / 6.7) but in a step, where a warp's first row is requested under the kernel
-// before: 1.212 / 1.228 ms per token at the 8B shape.
+// 17.5 / 18.6. So of `passes` passes fewer than `passes` groups of eight lanes may be idle in the last one. Up to 21
+// rows per SM (28 with three passes and more: a row per warp) the 8-lane kernel has too few warps to be the better one:
+// 36 blocks and 1024 rows 2.5 / 3.0, 2560 rows 94 % of its time, 3072 rows 100 %; 72 blocks and 3072 rows 86 %, 4096
+// rows 96 %. The paired mode at 32 blocks is no faster back to back (12288 pairs 10.3 / 10.3, 6144 pairs 7.1 / 6.7) but
+// in a step, where a warp's first row is requested under the kernel before: 1.212 / 1.228 ms per token at the 8B shape.
 template <int MODE>
 bool mv_wide(const MvParams& p) {
   const uint32_t nb = p.k / 128u, passes = (nb + 31) / 32, rounds = (nb + 7) / 8;
   if (nb < 25 || nb > (MODE == 3 ? 32u : 128u) || p.n_total >= 16384) return false;
-  return p.n_total <= 20 * bp_q1_sm_count() || 4 * passes - rounds < passes;
+  return p.n_total <= (passes > 2 ? 28 : 21) * bp_q1_sm_count() || 4 * passes - rounds < passes;
 }
 template <int MODE>
 cudaError_t launch_mv_wide(bool pdl, cudaStream_t s, const MvParams& p) {
