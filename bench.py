@@ -676,7 +676,7 @@ def prefill_exchange_bench(torch, dist, bp, stream, args, world, rank, local_ran
 
 
 def extras(torch, bp, stream, hbm_peak, tflops_peak, peak_kind, args):
-    """The 36-layer decode stack at ctx 4096 (BASELINE config 1) and the prefill pass (pp 512 / 2048) on one GPU."""
+    """The 36-layer decode stack at ctx 4096 and the prefill pass (pp 512 / 2048) on one GPU."""
     out = {}
     gen = torch.Generator(device="cuda")
     gen.manual_seed(99)
@@ -722,7 +722,7 @@ def extras(torch, bp, stream, hbm_peak, tflops_peak, peak_kind, args):
 
 
 def engine_bench(torch, bp, n_tokens=128, reps=3):
-    """a Bonsai-8B-shaped random-init model (Q1_0 signs Bernoulli(0.5), f16 block scales
+    """Whole engine: a Bonsai-8B-shaped random-init model (Q1_0 signs Bernoulli(0.5), f16 block scales
     |N(0, 0.02)|, norms 1.0) written to a temporary model directory, loaded, prefilled with 512 tokens through
     the batched path and decoded greedily for 128 tokens through Session::generate, this library's attention
     inside. Tokens per second, whole engine (the CPU restatement of this size is hours of CPU time: the

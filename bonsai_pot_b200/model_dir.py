@@ -6,7 +6,7 @@ files. A Q1_0 tensor [n_in, n_out] is stored as an array of f16 block scales [n_
 followed (4-byte padded) by an array of 16-byte sign blocks [n_out][n_in/128][16], bit e of a
 block = weight e. No real checkpoint exists where this repository is built, so this module
 WRITES directories of that format from a seed: sign bits Bernoulli(0.5), block scales
-|N(0, 0.02)| as f16, norm weights 1.0 (the random-init model BASELINE.json describes).
+|N(0, 0.02)| as f16, norm weights 1.0.
 Reading and validating a directory is the library's job (bp_model_load / bp_model_check_dir).
 """
 from __future__ import annotations

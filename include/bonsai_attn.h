@@ -315,7 +315,7 @@ uint32_t bp_decode_num_splits(const bp_attn_ctx* ctx, uint32_t cur_pos);
  * It runs the plain CUDA-core kernels, not the tcgen05 kernel of
  * bp_attn_decode: its result agrees with bp_attn_decode's within the attention
  * tolerance (|x - ref| <= 2e-3 + 1e-2 |ref|), not bit for bit, and a call is
- * several times slower (DESIGN.md gives the measured times). Limits: n_head <=
+ * several times slower. Limits: n_head <=
  * 64 (BP_ERR_CONFIG beyond that; use bp_attn_decode), head_dim 128, at most 32
  * splits (longer contexts get longer splits). The CURRENT device must be the one
  * that holds the cache, the other buffers and the stream (a cache on another

@@ -142,7 +142,7 @@ def test_decode_every_small_position(variant):
 
 @pytest.mark.parametrize("seed", [0, 1, 2])
 def test_decode_config0_end_to_end(seed):
-    """BASELINE config 0: 512 past tokens, the new token goes through
+    """512 past tokens, the new token goes through
     q_norm_rope + kv_writeback on the GPU, then decode over 513 keys."""
     sh = O.Shape(n_layer=1, max_seq=1024)
     case = build_decode_case(sh, seed=seed, cfg_id=0, layer=0, n_past=512)
@@ -246,7 +246,7 @@ def test_peer_exchange_epilogue_on_one_rank():
 
 @pytest.mark.parametrize("ctx_len,layer", [(4096, 1), (32768, 1)])
 def test_decode_long_context(ctx_len, layer):
-    """BASELINE configs 1 and 3 at full context length (two layers allocated,
+    """4096 and 32768 keys at full context length (two layers allocated,
     the second one used so that the layer offset is exercised)."""
     sh = O.Shape(n_layer=2, max_seq=ctx_len)
     case = build_decode_case(sh, seed=0, cfg_id=3, layer=layer, n_past=ctx_len - 1)
@@ -306,7 +306,7 @@ def prefill_case(sh, seed, layer, m):
 @pytest.mark.parametrize("m", [1, 5, 33, 64, 100, 512])
 @pytest.mark.parametrize("variant", [0, 1])
 def test_prefill_pass_matches_oracle(m, variant):
-    """BASELINE config 2 for one layer: q_norm_rope, kv_writeback and the causal
+    """A prefill pass of one layer: q_norm_rope, kv_writeback and the causal
     attention in one pass, as layer_step_matmul_in_pass issues them."""
     sh = O.Shape(n_layer=2, max_seq=2048)
     c = prefill_case(sh, seed=0, layer=1, m=m)
