@@ -1529,8 +1529,8 @@ cudaError_t launch_mv_wide(bool pdl, cudaStream_t s, const MvParams& p) {
   return bp_launch(pdl, matvec_q1_wide_kernel<MODE, PASSES>, dim3(grid), dim3(32 * w), mv_smem_bytes(p.k), s, p);
 }
 // Which calls take it: at most 128 blocks (activations that fit a CTA's default shared memory; the paired mode at most
-// 32: a lane's blocks of both rows have to fit its registers), no more rows than the two-rows-per-lane kernel is for,
-// and from 25 blocks on. A row costs a warp its passes of 32 blocks, full or not, and the 8-lane kernel its rounds of 8.
+// 32: a lane's blocks of both rows have to fit its registers), no more rows than the two-rows-per-lane kernel is for
+// (4096 inputs: 16384 rows 8.1 us against its 7.0, 24576 rows 10.5 against 8.8), and from 25 blocks on. A row costs a warp its passes of 32 blocks, full or not, and the 8-lane kernel its rounds of 8.
 // us per call, warp per row / 8 lanes, weights from HBM, back to back in a graph, plain: 24 blocks 3.6 / 3.4 (4096 rows)
 // and 6.4 / 5.8 (12288), 26 blocks 3.7 / 3.8 and 6.5 / 6.9; 36 blocks 4.8 / 4.4 and 9.7 / 8.3, 56 blocks 5.1 / 5.7 and
 // 10.0 / 10.8; 72 blocks 6.3 / 6.6 and 13.6 / 12.8, 80 blocks 6.4 / 7.2 and 13.7 / 14.0; 104 blocks 7.9 / 8.9 and
