@@ -6,6 +6,7 @@
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
+#include <sys/mman.h>
 
 #include <algorithm>
 #include <mutex>
@@ -794,16 +795,17 @@ static cudaError_t shard_copy(void* host_row0, size_t pitch, size_t col, uint8_t
   return cudaMemcpy2D(dev, width, static_cast<uint8_t*>(host_row0) + col, pitch, width, rows, cudaMemcpyHostToDevice);
 }
 
-// ---- a snapshot's rows, moved by several lanes ----
+// ---- a snapshot's rows, moved by lanes ----
 // A copy between the device and pageable memory is bound by the host: one thread touches fresh pages and copies at
-// a few GB/s, a fifth of the link. So the payload is cut into SNAP_LANES ranges; a lane is a thread with a stream
-// and two pinned buffers of SNAP_CHUNK, whose DMA runs under the host copy of the other buffer. The lanes are made
-// by the first large snapshot and belong to the context. Sharded contexts (strided rows) and payloads below
-// SNAP_LANES_MIN, where a lane has less than half a chunk, take plain copies. 36 layers, capture / restore in us: 25 rows
-// (2.0 MB) plain 1960 / 1812, 26 rows in lanes 637 / 648; 512 rows (42 MB) 5331 / 6555 and 2149 / 1844, from and to
-// pinned memory 2483 / 9551 and 2059 / 1857. So the lanes would pay below the line too; how far was not measured.
+// a few GB/s, a fifth of the link, and a plain copy per section costs some 13 us whatever its size. So the payload is cut
+// into a range per SNAP_PER_LANE bytes, SNAP_LANES at most; a lane is a thread (the first is the caller's) with a stream
+// and two pinned buffers of SNAP_CHUNK, whose DMA runs under the host copy of the other buffer. A lane is made when a
+// snapshot first needs it and belongs to the context. Sharded contexts (strided rows) and the smallest payloads take
+// plain copies. 36 layers, capture / restore in us: 16 rows (1.3 MB) 607 / 590 (plain copies 1900 / 1800), 100 rows
+// 921 / 823, 512 rows (42 MB) 2575 / 1907; the capture 5800 before its fresh pages were asked for as huge ones. Eight
+// lanes: 512 rows 2206 / 1814, 100 rows 919 / 907.
 constexpr uint32_t SNAP_LANES = 4;
-constexpr size_t SNAP_CHUNK = 1u << 20, SNAP_LANES_MIN = 2u << 20;
+constexpr size_t SNAP_CHUNK = 1u << 20, SNAP_LANES_MIN = 64u << 10, SNAP_PER_LANE = 1u << 20;
 struct bp_snap_lanes {
   std::mutex busy;
   cudaStream_t stream[SNAP_LANES] = {};
@@ -822,19 +824,17 @@ static void drop_snap_lanes(bp_snap_lanes* l) {
   }
   delete l;
 }
-static bp_snap_lanes* make_snap_lanes() {
-  bp_snap_lanes* l = new (std::nothrow) bp_snap_lanes();
-  bool ok = l != nullptr;
-  for (uint32_t t = 0; ok && t < SNAP_LANES; t++) {
-    ok = cudaStreamCreateWithFlags(&l->stream[t], cudaStreamNonBlocking) == cudaSuccess;
+// The first `n` lanes, as far as they are not there already.
+static bool make_snap_lanes(bp_snap_lanes* l, uint32_t n) {
+  bool ok = true;
+  for (uint32_t t = 0; ok && t < n; t++) {
+    ok = l->stream[t] || cudaStreamCreateWithFlags(&l->stream[t], cudaStreamNonBlocking) == cudaSuccess;
     for (int i = 0; ok && i < 2; i++)
-      ok = cudaEventCreateWithFlags(&l->done[t][i], cudaEventDisableTiming) == cudaSuccess &&
-           cudaMallocHost(&l->pinned[t][i], SNAP_CHUNK) == cudaSuccess;
+      ok = (l->done[t][i] || cudaEventCreateWithFlags(&l->done[t][i], cudaEventDisableTiming) == cudaSuccess) &&
+           (l->pinned[t][i] || cudaMallocHost(&l->pinned[t][i], SNAP_CHUNK) == cudaSuccess);
   }
-  if (ok) return l;
-  (void)cudaGetLastError();  // no lanes (no pinned memory left): plain copies
-  drop_snap_lanes(l);
-  return nullptr;
+  if (!ok) (void)cudaGetLastError();  // no lanes (no pinned memory left): plain copies
+  return ok;
 }
 
 // Payload bytes [at, at + len) between the cache and `pin`, in as many copies as sections they span.
@@ -892,23 +892,30 @@ static cudaError_t snap_transfer(bp_attn_ctx* c, uint8_t* payload, uint32_t pos,
   *done = false;
   const uint64_t bytes = bp_snapshot_payload_bytes(c->cfg.n_layer, c->kv_dim, pos);
   if (c->cfg.n_shards != 1 || bytes < SNAP_LANES_MIN) return cudaSuccess;
+  const uint32_t lanes = static_cast<uint32_t>(std::min<uint64_t>(SNAP_LANES, 1 + bytes / SNAP_PER_LANE));
   static std::mutex making;
   {
     std::lock_guard<std::mutex> g(making);
-    if (!c->snap_lanes) c->snap_lanes = make_snap_lanes();
+    if (!c->snap_lanes) c->snap_lanes = new (std::nothrow) bp_snap_lanes();
   }
   bp_snap_lanes* l = c->snap_lanes;
   if (!l) return cudaSuccess;
   std::lock_guard<std::mutex> g(l->busy);
+  if (!make_snap_lanes(l, lanes)) return cudaSuccess;
+  if (to_host) {  // a capture fills a fresh buffer: whole huge pages of it in one fault each (a wish: no matter if it fails)
+    constexpr uintptr_t HUGE = 2u << 20;
+    const uintptr_t from = (reinterpret_cast<uintptr_t>(payload) + HUGE - 1) & ~(HUGE - 1), to = (reinterpret_cast<uintptr_t>(payload) + bytes) & ~(HUGE - 1);
+    if (from < to) (void)madvise(reinterpret_cast<void*>(from), to - from, MADV_HUGEPAGE);
+  }
   // Ordered as a plain copy on the default stream is: behind what the blocking streams hold.
   cudaError_t e = cudaEventRecord(l->done[0][0], cudaStreamLegacy);
   if (e == cudaSuccess) e = cudaEventSynchronize(l->done[0][0]);
   if (e != cudaSuccess) return e;
-  const uint64_t per = ((bytes + SNAP_LANES - 1) / SNAP_LANES + 4095u) & ~static_cast<uint64_t>(4095u);
+  const uint64_t per = ((bytes + lanes - 1) / lanes + 4095u) & ~static_cast<uint64_t>(4095u);
   cudaError_t st[SNAP_LANES] = {};
   std::thread th[SNAP_LANES];
   auto lane = [&](uint32_t t) { st[t] = snap_lane(c, l, t, payload, pos, std::min<uint64_t>(bytes, t * per), std::min<uint64_t>(bytes, (t + 1) * per), to_host); };
-  for (uint32_t t = 1; t < SNAP_LANES; t++) {
+  for (uint32_t t = 1; t < lanes; t++) {
     try {
       th[t] = std::thread(lane, t);
     } catch (...) {  // no thread to be had: this one does the lane
@@ -916,7 +923,7 @@ static cudaError_t snap_transfer(bp_attn_ctx* c, uint8_t* payload, uint32_t pos,
     }
   }
   lane(0);
-  for (uint32_t t = 1; t < SNAP_LANES; t++)
+  for (uint32_t t = 1; t < lanes; t++)
     if (th[t].joinable()) th[t].join();
   for (cudaError_t x : st)
     if (x != cudaSuccess) e = x;

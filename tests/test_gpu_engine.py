@@ -769,3 +769,9 @@ def test_norm_weights_may_begin_at_any_offset_of_their_file(tmp_path):
     check_dir(odd)  # (lengths and offsets add up)
     with pytest.raises(bp.ConfigError, match="scales"):
         bp.Model(odd, max_seq=64)
+
+
+@pytest.mark.parametrize("pos", [14, 15, 227, 228])
+def test_snapshots_at_the_edges_of_the_lanes(pos):
+    """14 rows here are the last that go by plain copies (64 KB), 15 take one lane; 228 the second (1 MB)."""
+    test_large_snapshots_hold_the_cache_rows(pos)
