@@ -319,9 +319,9 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
   const CUtensorMap &map_kq = maps[0], &map_kd = maps[1], &map_vq = maps[2], &map_vd = maps[3];
   using L = ULayout<HPC>;
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t full_bar[U_MAX_STAGES], k_empty[U_MAX_STAGES], v_full[U_MAX_STAGES], v_empty[U_MAX_STAGES];
+  __shared__ __align__(8) uint64_t full_bar[2 * U_MAX_STAGES], k_empty[U_MAX_STAGES], v_full[2 * U_MAX_STAGES], v_empty[2 * U_MAX_STAGES];
   __shared__ __align__(8) uint64_t s_ready[4], s_free[4], p_ready[4], p_free[4], o_ready[4], o_free[4];
-  __shared__ __align__(8) uint64_t q_bar, patched_bar, patched_v;
+  __shared__ __align__(8) uint64_t q_bar, patched_bar, patched_v, v_last;
   __shared__ uint32_t tmem_base_s;
   __shared__ volatile uint32_t abort_s;
 
@@ -355,8 +355,14 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
   Misc* misc = reinterpret_cast<Misc*>(smem_gen + ring_b + L::Q_B + L::P_B);
 
   // One K stage: K tiles of the HPC heads and both scale rows, 128 tokens from `it * UT`.
+  // Barriers that an issuer waits for: two per stage and slot, used in turn. Job j belongs to issuer j mod NISS, so in a
+  // ring of odd size an issuer meets every other use of a stage, and on ONE barrier a wait for use u returned as soon as
+  // use u - 2 was complete: it was right only as long as the loads in between happened to land first. With the barrier
+  // chosen by the job modulo twice the ring every use that completes it is waited for by the same issuer, in order.
+  auto bar2 = [](uint64_t* bars, uint32_t i, uint32_t ring) { return bars + i % (2 * ring); };
+  auto phase2 = [](uint32_t i, uint32_t ring) { return (i / (2 * ring)) & 1u; };
   auto issue_stage = [&](uint32_t it, uint32_t s) {
-    const uint32_t bar = smem_u32(&full_bar[s]);
+    const uint32_t bar = smem_u32(bar2(full_bar, it, ns));
     const uint32_t stage = smem_base + s * L::KSTAGE_B;
     const int row = static_cast<int>(p.row_base + tok_begin + it * UT);
     // Older rows were written by launches that have long completed; rows from fresh_from on (the
@@ -369,9 +375,11 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
     tma_load_2d(stage + HPC * TILE_B + L::SCALE_B, &map_vd, bar, static_cast<int>(g0 * 16), row);
     for (uint32_t g = 0; g < HPC; g++) tma_load_3d(stage + g * TILE_B, &map_kq, bar, 0, static_cast<int>(g0 + g), row);
   };
-  // The V tile of job j (stage j / HPC, head j % HPC) into V slot j % nv.
+  const bool new_row = p.fused && tok_end == p.cur_pos;  // this CTA's last stage holds the new token's row
+  // The V tile of job j (stage j / HPC, head j % HPC) into V slot j % nv. The new row's tiles complete a barrier of
+  // their own: who patches the row in has not followed the slot's phases, and one phase looks like the next but one.
   auto issue_v = [&](uint32_t j) {
-    const uint32_t v = j % nv, bar = smem_u32(&v_full[v]);
+    const uint32_t v = j % nv, bar = smem_u32(new_row && j / HPC == n_iter - 1 ? &v_last : bar2(v_full, j, nv));
     const int row = static_cast<int>(p.row_base + tok_begin + (j / HPC) * UT);
     mbar_arrive_expect_tx(bar, L::VSLOT_B);
     tma_load_3d(v_ring + v * L::VSLOT_B, &map_vq, bar, 0, static_cast<int>(g0 + j % HPC), row);
@@ -393,8 +401,11 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
     issue_stage(0, 0);
     prefetch_tensormap(&map_vq);
   } else if (warp == 3) {
-    if (lane >= 1 && lane < ns) mbar_init(smem_u32(&full_bar[lane]), 1);
-    if (lane >= 8 && lane - 8 < nv) mbar_init(smem_u32(&v_full[lane - 8]), 1);
+    if (lane >= 1 && lane < 2 * U_MAX_STAGES) mbar_init(smem_u32(&full_bar[lane]), 1);
+    if (lane >= 2 * U_MAX_STAGES) mbar_init(smem_u32(&v_full[lane - 2 * U_MAX_STAGES]), 1);
+    fence_barrier_init();
+  } else if (warp == 4) {
+    if (lane < 2 * U_MAX_STAGES) mbar_init(smem_u32(&v_empty[lane]), 1);  // the tcgen05.commit behind the job's P V
     fence_barrier_init();
   } else if (warp == 2) {
     if (lane < 4) {
@@ -410,10 +421,9 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
       mbar_init(smem_u32(&q_bar), 4);  // the four accumulate warps prepare Q
       mbar_init(smem_u32(&patched_bar), 1);
       mbar_init(smem_u32(&patched_v), 1);
+      mbar_init(smem_u32(&v_last), HPC);
     } else if (lane < 21) {
       if (lane - 13 < ns) mbar_init(smem_u32(&k_empty[lane - 13]), HPC * 4);  // the 4 warps of each job's softmax group
-    } else if (lane < 29) {
-      if (lane - 21 < nv) mbar_init(smem_u32(&v_empty[lane - 21]), 1);  // the tcgen05.commit behind the job's P V
     }
     fence_barrier_init();
   }
@@ -527,7 +537,6 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
     __syncwarp();
     // Fused step, last split: the whole warp first quantises the new token's K / V rows of this
     // CTA's heads (the arithmetic of kv_writeback_kernel) and stores them to the cache.
-    const bool new_row = p.fused && tok_end == p.cur_pos;
     uint32_t pk[HPC], pv[HPC];
     float dk[HPC], dv[HPC];
     if (new_row) {
@@ -569,7 +578,7 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
       // rows, scale rows). K side first (the last Q K^T waits for it and only then requests its V
       // tile), V side when that tile is there (the last P V waits for it).
       const uint32_t it_last = n_iter - 1, s_last = it_last % ns;
-      wait(&full_bar[s_last], (it_last / ns) & 1);
+      wait(bar2(full_bar, it_last, ns), phase2(it_last, ns));
       const uint32_t r = p.cur_pos - 1 - (tok_begin + it_last * UT);
       uint8_t* stage = smem_gen + s_last * L::KSTAGE_B;
 #pragma unroll
@@ -583,10 +592,10 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
       fence_proxy_async();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&patched_bar));
+      wait(&v_last, 0);
 #pragma unroll
       for (uint32_t g = 0; g < HPC; g++) {
-        const uint32_t j = it_last * HPC + g, v = j % nv;
-        wait(&v_full[v], (j / nv) & 1);
+        const uint32_t v = (it_last * HPC + g) % nv;
         *reinterpret_cast<uint32_t*>(smem_gen + ns * L::KSTAGE_B + v * L::VSLOT_B + swz128(r * 128 + 4 * lane)) = pv[g];
       }
       fence_proxy_async();
@@ -621,9 +630,9 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
       const uint32_t q = warp - 1;
       wait(&q_bar, 0);
       for (uint32_t j = q; j < n_jobs; j += NISS) {
-        const uint32_t it = j / HPC, g = j % HPC, bi = j % NGRP, k = j / NGRP, s = it % ns, use = it / ns;
-        wait(&full_bar[s], use & 1);
-        if (p.fused && tok_end == p.cur_pos && it == n_iter - 1) wait(&patched_bar, 0);  // the new row is in place
+        const uint32_t it = j / HPC, g = j % HPC, bi = j % NGRP, k = j / NGRP, s = it % ns;
+        wait(bar2(full_bar, it, ns), phase2(it, ns));
+        if (new_row && it == n_iter - 1) wait(&patched_bar, 0);  // the new row is in place
         if (k > 0) wait(&s_free[bi], (k - 1) & 1);
         tc_fence_after();
         const uint64_t ka = dbase + ((smem_base + s * L::KSTAGE_B + g * TILE_B) >> 4);
@@ -634,7 +643,7 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
         // Now request the job's V tile (unless set-up did): it arrives while the softmax group works,
         // and its slot is occupied for one load latency instead of the load latency plus the whole job.
         if (j >= v_pre) {
-          if (j >= nv) wait(&v_empty[j % nv], (j / nv - 1) & 1);
+          if (j >= nv) wait(bar2(v_empty, j - nv, nv), phase2(j - nv, nv));
           if (!abort_s) issue_v(j);
         }
       }
@@ -651,8 +660,11 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
       for (uint32_t j = q; j < n_jobs; j += NISS) {
         const uint32_t it = j / HPC, bi = j % NGRP, k = j / NGRP;
         const uint32_t v = j % nv;
-        wait(&v_full[v], (j / nv) & 1);
-        if (p.fused && tok_end == p.cur_pos && it == n_iter - 1) wait(&patched_v, 0);  // the new row is in place
+        if (new_row && it == n_iter - 1) {
+          wait(&patched_v, 0);  // the tile is there and the new row in it
+        } else {
+          wait(bar2(v_full, j, nv), phase2(j, nv));
+        }
         wait(&p_ready[bi], k & 1);
         if (k > 0) wait(&o_free[bi], (k - 1) & 1);
         tc_fence_after();
@@ -663,7 +675,7 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
           umma_i8(tmem + NGRP * 64 + bi * 64, va + kk * (32 * 128 >> 4), pb + 2 * kk, IDESC_PV, kk);
         umma_commit(smem_u32(&o_ready[bi]));
         umma_commit(smem_u32(&p_free[bi]));
-        umma_commit(smem_u32(&v_empty[v]));  // the V slot is free once this P V has run
+        umma_commit(smem_u32(bar2(v_empty, j, nv)));  // the V slot is free once this P V has run
       }
     }
   }
