@@ -624,7 +624,7 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
     // ---------------- QK issuers: S^T[token][(block, byte row, head)] = K tile x Q^T ----------------
     // One UMMA per Q8_0 block (K = 32 dims). Issuer q takes the jobs j = q (mod NISS); issuing is
     // serial scalar work (about 100 instructions per job), hence more than one issuer.
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t IDESC_QK = umma_idesc(2, 1, 1, 0, 0, 128, 16);  // s32 = s8 (K-major) x s8
       const uint64_t dbase = umma_desc_sw128(0, 16, 1024);               // + (shared address >> 4)
       const uint32_t q = warp - 1;
@@ -653,7 +653,7 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
     // The four blocks' P' tiles are 16 consecutive rows each of one 64-row K-major operand, so one
     // N = 64 UMMA per 32 tokens serves all of them and the V tile is read once; only the
     // (dims of block b) x (columns of block b) part of the result is used.
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t IDESC_PV = umma_idesc(2, 1, 0, 1, 0, 128, 64);  // s32 += s8 (MN-major) x u8
       const uint64_t dbase = umma_desc_sw128(0, 16, 1024);
       const uint32_t q = warp - 1 - NISS;

@@ -318,7 +318,7 @@ prefill_umma_kernel(const CUtensorMap* __restrict__ maps, const PrefillParams p)
       // and query tile (polls, four MMAs at 115 cycles each, three commits), so a P tile waited some 1400
       // cycles for its turn and the softmax groups then waited as long for the next S. With one query
       // tile per CTA warp 0 does all of it.
-      if (lane == 0) {
+      if (elect_one()) {
         constexpr uint32_t IDESC_PV = umma_idesc(1, 0, 0, 0, 1, BM, 128);  // f32 += f16 (TMEM) x f16 (MN-major), N = 128 dims
         const uint64_t dmn = umma_desc_sw128(0, 8192, 1024);    // V: next 64 dims 8 KB away, 8 key rows 1 KB apart
         const bool do_k = L::N_LOADERS == 1 || warp == 1, do_v = warp == 0;
@@ -390,7 +390,7 @@ prefill_umma_kernel(const CUtensorMap* __restrict__ maps, const PrefillParams p)
       // for all P V (4 per key tile and query tile).
       const uint32_t x = warp - L::N_LOADERS;
       const uint32_t n_mine = nx[x], c0 = gx[x];
-      if (lane == 0 && n_mine > 0) {
+      if (n_mine > 0 && elect_one()) {
         constexpr uint32_t IDESC_QK = umma_idesc(1, 0, 0, 0, 0, BM, BN);   // f32 = f16 (K-major) x f16 (K-major), N = 64 keys
         const uint64_t dk = umma_desc_sw128(0, 16, 1024);       // K-major operands
         const uint64_t qa = dk + ((smem_base + L::OFF_Q + x * OPER_B) >> 4);
