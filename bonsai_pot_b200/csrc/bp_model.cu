@@ -285,7 +285,7 @@ struct bp_model {
   uint32_t* topk_idx = nullptr;
   uint32_t tap_mode = 0;
   uint8_t* tap_buf = nullptr;
-  // The one-token step as a CUDA graph (token copy, embed, layers, output suffix, result copies). The only
+  // The one-token step as a CUDA graph (embed, layers, output suffix). The only
   // launches whose arguments depend on the position are the attention calls: their nodes are patched per step
   // with what the attention library's launcher produces for the new position.
   struct StepGraph {
@@ -297,8 +297,8 @@ struct bp_model {
   } sg, fill;                 // fill: the same without the output suffix (a token whose logits nobody asks for)
   bool step_graph = true;     // bp_model_set_step_graph
   uint64_t graph_steps = 0;   // steps that went to the device as a graph launch, of either graph
-  uint32_t* token_pin = nullptr;  // pinned: the token of the step (read by the graph's copy node)
-  float* res_val_pin = nullptr;   // pinned: top-k results of the step
+  uint32_t* token_pin = nullptr;  // pinned: the token of the step (read by the graph's first kernel)
+  float* res_val_pin = nullptr;   // pinned: top-k results of the step (written by the graph's last kernel)
   uint32_t* res_idx_pin = nullptr;
 };
 
@@ -462,7 +462,7 @@ void drop_step_graphs(bp_model* m) {
   drop_step_graph(m->fill);
 }
 
-// The whole step (token copy, embed, layers, output norm, LM head, top-k of TOPK_MAX, result copies) captured
+// The whole step (embed, layers, output norm, LM head, top-k of TOPK_MAX) captured
 // from the model's stream at position pos. The fill graph begins with the embedding (several of its launches are
 // queued, each behind its own token copy) and ends with the last layer.
 int capture_step_graph(bp_model* m, bp_model::StepGraph& g, uint32_t pos) {
@@ -473,14 +473,13 @@ int capture_step_graph(bp_model* m, bp_model::StepGraph& g, uint32_t pos) {
   g.attn.resize(c.n_layer);
   M_CUDA(m, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   int st = BP_OK;
-  cudaError_t e = suffix ? cudaMemcpyAsync(m->tokens_dev, m->token_pin, sizeof(uint32_t), cudaMemcpyHostToDevice, s) : cudaSuccess;
-  if (e == cudaSuccess) e = bp_q1_embed(true, s, m->embed, m->tokens_dev, 1, m->x);
+  // The step's token and results are words of pinned memory that the first and the last kernel read and write themselves:
+  // a copy node each cost more than the access (a step of the two-layer shape 72 -> 65 us).
+  cudaError_t e = bp_q1_embed(true, s, m->embed, suffix ? m->token_pin : m->tokens_dev, 1, m->x);
   for (uint32_t il = 0; e == cudaSuccess && st == BP_OK && il < c.n_layer; il++) st = decode_layer(m, il, pos, true, &g.attn[il]);
   if (suffix && e == cudaSuccess && st == BP_OK) e = bp_q1_rms_norm(true, s, m->x, m->x, m->output_norm, c.n_embd, 1, c.rms_eps);
   if (suffix && e == cudaSuccess && st == BP_OK) e = bp_q1_matvec(true, s, m->lm_head, m->x, m->logits, false);
-  if (suffix && e == cudaSuccess && st == BP_OK) e = bp_q1_topk(true, s, m->logits, c.n_vocab, TOPK_MAX, m->topk_val, m->topk_idx);
-  if (suffix && e == cudaSuccess && st == BP_OK) e = cudaMemcpyAsync(m->res_val_pin, m->topk_val, TOPK_MAX * sizeof(float), cudaMemcpyDeviceToHost, s);
-  if (suffix && e == cudaSuccess && st == BP_OK) e = cudaMemcpyAsync(m->res_idx_pin, m->topk_idx, TOPK_MAX * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+  if (suffix && e == cudaSuccess && st == BP_OK) e = bp_q1_topk(true, s, m->logits, c.n_vocab, TOPK_MAX, m->res_val_pin, m->res_idx_pin);
   const cudaError_t e_end = cudaStreamEndCapture(s, &g.graph);  // always: the stream must leave capture mode
   if (st != BP_OK) return st;
   M_CUDA(m, e);
