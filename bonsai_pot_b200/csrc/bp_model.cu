@@ -382,22 +382,18 @@ cudaError_t attention_call(bp_model* m, uint32_t il, uint32_t pos) {
 
 // One layer of the one-token path: layer_pre_kv_in_pass, dispatch_kv_writeback_fused, layer_post_kv_in_pass
 // (src/forward.rs:608-631, 763-908). The three attention dispatches are one call of the attention library.
-// in_graph: the launches are being captured into the step's graph (attn_nodes then receives the attention
-// launches with their nodes); the choice of dependent launches differs between the two ways of launching.
-// Which launches carry programmatic stream serialization was measured per kernel on the 8B shape (us per layer,
-// stream launches / graph replay): all four matvecs 55.0 / 53.2, all but the down projection 48.8 / 44.8, gate + up
-// only 49.9 / 41.1, none 51.2 / 42.3. The down projection's CTAs, resident early, take the SM slots that the
-// second wave of the gate + up launch is waiting for. (Measured with the 8-lane matvecs; the warp-per-row kernels that
-// these launches now run at that shape come in one wave, and the combinations have not been measured again.)
-int decode_layer(bp_model* m, uint32_t il, uint32_t pos, bool in_graph = false, std::vector<bp_launch_record>* attn_nodes = nullptr) {
+// attn_nodes: the launches are being captured into the step's graph, and it receives the attention launches with their nodes.
+// Which launches carry programmatic stream serialization, us per step of the 8B shape as a graph, position 100 / 900: all
+// but Wo 1150 / 1233, all four matvecs 1152 / 1236, all but Wo and Q/K/V 1165 / 1260, gate + up only (the choice for the
+// 8-lane matvecs, whose second wave the down projection's early CTAs kept waiting) 1208 / 1302, none 1237 / 1328.
+int decode_layer(bp_model* m, uint32_t il, uint32_t pos, std::vector<bp_launch_record>* attn_nodes = nullptr) {
   const Config& c = m->cfg;
   const LayerTensors& lt = m->layers[il];
   cudaStream_t s = m->stream;
-  const bool pdl = !in_graph;
   {
     const bp_q1_tensor w[3] = {lt.wq, lt.wk, lt.wv};
     __half* const out[3] = {m->q, m->k_cur, m->v_cur};
-    M_CUDA(m, bp_q1_matvec_normed(pdl, s, w, out, 3, m->x, lt.attn_norm, c.rms_eps));
+    M_CUDA(m, bp_q1_matvec_normed(true, s, w, out, 3, m->x, lt.attn_norm, c.rms_eps));
   }
   if (attn_nodes != nullptr) {  // capturing: keep the nodes of the attention launches
     bp_launch_recorder rec;
@@ -418,13 +414,13 @@ int decode_layer(bp_model* m, uint32_t il, uint32_t pos, bool in_graph = false, 
       M_CUDA(m, cudaMemcpyAsync(m->attn_out, slot, static_cast<size_t>(c.q_dim) * 2, cudaMemcpyHostToDevice, s));
     }
   }
-  M_CUDA(m, bp_q1_matvec(pdl, s, lt.wo, m->attn_out, m->x, true));
+  M_CUDA(m, bp_q1_matvec(false, s, lt.wo, m->attn_out, m->x, true));
   // matvec_q1_0_fused_normed over (gate, up) and silu(gate) * up in one launch: a lane computes row i of both
   // tensors and writes the f16 value that feeds the down projection (the same values dispatch_matvec_q1_0_silu
   // stages; that shader as one kernel had each of the 256 CTAs of the 4096-row down tensor recompute all 12288
   // of them: 27.6 us against 8 for the plain matvec).
   M_CUDA(m, bp_q1_matvec_normed_silu(true, s, lt.wg, lt.wu, m->ffn_in, m->x, lt.ffn_norm, c.rms_eps));
-  M_CUDA(m, bp_q1_matvec(false, s, lt.wd, m->ffn_in, m->x, true));
+  M_CUDA(m, bp_q1_matvec(true, s, lt.wd, m->ffn_in, m->x, true));
   return BP_OK;
 }
 
@@ -476,7 +472,7 @@ int capture_step_graph(bp_model* m, bp_model::StepGraph& g, uint32_t pos) {
   // The step's token and results are words of pinned memory that the first and the last kernel read and write themselves:
   // a copy node each cost more than the access (a step of the two-layer shape 72 -> 65 us).
   cudaError_t e = bp_q1_embed(true, s, m->embed, suffix ? m->token_pin : m->tokens_dev, 1, m->x);
-  for (uint32_t il = 0; e == cudaSuccess && st == BP_OK && il < c.n_layer; il++) st = decode_layer(m, il, pos, true, &g.attn[il]);
+  for (uint32_t il = 0; e == cudaSuccess && st == BP_OK && il < c.n_layer; il++) st = decode_layer(m, il, pos, &g.attn[il]);
   if (suffix && e == cudaSuccess && st == BP_OK) e = bp_q1_rms_norm(true, s, m->x, m->x, m->output_norm, c.n_embd, 1, c.rms_eps);
   if (suffix && e == cudaSuccess && st == BP_OK) e = bp_q1_matvec(true, s, m->lm_head, m->x, m->logits, false);
   if (suffix && e == cudaSuccess && st == BP_OK) e = bp_q1_topk(true, s, m->logits, c.n_vocab, TOPK_MAX, m->res_val_pin, m->res_idx_pin);
