@@ -67,6 +67,7 @@ struct UmmaParams {
   uint32_t n_px, px_off;
   __half* const* px_out;  // in device memory: the parameter block stays small (a larger one costs about 1 % per launch)
   uint32_t merge;       // 1: the CTAs of a head group merge its splits themselves (merge_unit)
+  uint32_t row_step;    // launch of several layers: cache rows of a layer
   uint2* ll;            // tagged partials [split][head][BP_LL_STRIDE]: (value bits, tag of the launch)
   uint32_t* epochs;     // per head group (grid y): the tag of the last merged launch
   uint32_t fused;
@@ -312,7 +313,10 @@ __device__ __forceinline__ void merge_part(const UmmaParams& p, uint32_t lane, u
 // few percent with the sheer amount of code around their loops; measured on one GPU, per call at
 // ctx 4096 / 32768: both codes in one kernel 8.09 / 20.45 us, one instance per mode 8.29 / 19.90 us.
 // Hence this pairing.
-template <uint32_t HPC, uint32_t MODE>
+// ALL: the fused steps of grid z layers in one launch (bp_launch_decode_layers). q, out, k_cur and v_cur hold a row
+// per layer, the cache pointers and row_base belong to the first one; for the activations, the outputs and the merge a
+// layer's heads follow the previous layer's (n_head is the head count of them all).
+template <uint32_t HPC, uint32_t MODE, bool ALL = false>
 __global__ void __launch_bounds__(U_THREADS, 1)
 decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__ UmmaParams p) {
   // tensor maps in device memory (written by the host before any launch that reads them): K quants, K scales, V quants, V scales
@@ -339,6 +343,9 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
   if (threadIdx.x == 0) pdl_launch_dependents();
   const uint32_t ns = p.nk, nv = p.nv;  // ns: K stages
   const uint32_t g0 = blockIdx.y * HPC;
+  const uint32_t layer = ALL ? blockIdx.z : 0u;
+  const uint32_t hg0 = g0 + layer * p.n_kv_head, group = blockIdx.y + layer * gridDim.y;  // over the launch's layers
+  const uint32_t row0 = p.row_base + (ALL ? layer * p.row_step : 0u);
   const uint32_t split = blockIdx.x, n_splits = gridDim.x;
   const uint32_t tok_begin = split * p.tps;
   const uint32_t tok_end = min(tok_begin + p.tps, p.cur_pos);
@@ -364,7 +371,7 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
   auto issue_stage = [&](uint32_t it, uint32_t s) {
     const uint32_t bar = smem_u32(bar2(full_bar, it, ns));
     const uint32_t stage = smem_base + s * L::KSTAGE_B;
-    const int row = static_cast<int>(p.row_base + tok_begin + it * UT);
+    const int row = static_cast<int>(row0 + tok_begin + it * UT);
     // Older rows were written by launches that have long completed; rows from fresh_from on (the
     // newest token's, when a separate kernel wrote it just before this one) only by the time the
     // dependency wait returns. In the fused step this CTA writes the newest row itself and patches
@@ -380,7 +387,7 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
   // their own: who patches the row in has not followed the slot's phases, and one phase looks like the next but one.
   auto issue_v = [&](uint32_t j) {
     const uint32_t v = j % nv, bar = smem_u32(new_row && j / HPC == n_iter - 1 ? &v_last : bar2(v_full, j, nv));
-    const int row = static_cast<int>(p.row_base + tok_begin + (j / HPC) * UT);
+    const int row = static_cast<int>(row0 + tok_begin + (j / HPC) * UT);
     mbar_arrive_expect_tx(bar, L::VSLOT_B);
     tma_load_3d(v_ring + v * L::VSLOT_B, &map_vq, bar, 0, static_cast<int>(g0 + j % HPC), row);
   };
@@ -474,14 +481,14 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
       prefetch_l2(p.w_k + 4 * lane);
     }
     pdl_wait();  // q is written by the kernel before this one
-    if (p.merge && n_splits > 1) epoch = ld_relaxed_u32(p.epochs + blockIdx.y);  // used in the epilogue
+    if (p.merge && n_splits > 1) epoch = ld_relaxed_u32(p.epochs + group);  // used in the epilogue
 
     // lane l holds dims 4l .. 4l+3 of one head: a Q8_0 block is 8 lanes. One 8-byte load, three
     // shuffles for the block maximum, two 4-byte stores: short straight-line code, because this sits
     // on the critical path of every launch (the first Q K^T waits for it) and runs cold.
     for (uint32_t hl = aw; hl < HPC * p.qpg; hl += 4) {
       const uint32_t g = hl / p.qpg, hq = hl % p.qpg, b = lane >> 3;
-      const size_t q_off = (static_cast<size_t>(g0 + g) * p.qpg + hq) * BP_HEAD_DIM;
+      const size_t q_off = (static_cast<size_t>(hg0 + g) * p.qpg + hq) * BP_HEAD_DIM;
       uint2 raw;
       if (p.fused) {
         // q_norm_rope of this head, rounded to f16 exactly as the stand-alone kernel stores it
@@ -541,10 +548,11 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
     float dk[HPC], dv[HPC];
     if (new_row) {
       pdl_wait();  // k_cur / v_cur come from the kernel before this one
-      const uint32_t pos = p.cur_pos - 1, kv_dim = p.n_kv_head * BP_HEAD_DIM;
+      const uint32_t kv_dim = p.n_kv_head * BP_HEAD_DIM;
+      const size_t row = static_cast<size_t>(p.cur_pos - 1) + (ALL ? static_cast<size_t>(layer) * p.row_step : 0u);
 #pragma unroll
       for (uint32_t g = 0; g < HPC; g++) {
-        const size_t src = static_cast<size_t>(g0 + g) * BP_HEAD_DIM;
+        const size_t src = static_cast<size_t>(hg0 + g) * BP_HEAD_DIM;
         const Rot4 kp = norm_rope(p.k_cur + src, p.w_k, p.rope_row, p.eps, static_cast<int>(lane));
         const uint2 vr = *reinterpret_cast<const uint2*>(p.v_cur + src + 4 * lane);
         const float2 v01 = __half22float2(*reinterpret_cast<const __half2*>(&vr.x));
@@ -552,11 +560,11 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
         const float vraw[4] = {v01.x, v01.y, v23.x, v23.y};
         pk[g] = quant4(kp.v, &dk[g]);
         pv[g] = quant4(vraw, &dv[g]);
-        const size_t word = (static_cast<size_t>(pos) * kv_dim + src) / 4 + lane;
+        const size_t word = (row * kv_dim + static_cast<size_t>(g0 + g) * BP_HEAD_DIM) / 4 + lane;
         p.k_qs[word] = pk[g];
         p.v_qs[word] = pv[g];
         if ((lane & 7) == 0) {
-          const size_t blk = static_cast<size_t>(pos) * (kv_dim / BP_QK8) + (g0 + g) * 4 + (lane >> 3);
+          const size_t blk = row * (kv_dim / BP_QK8) + (g0 + g) * 4 + (lane >> 3);
           p.k_d[blk] = dk[g];
           p.v_d[blk] = dv[g];
         }
@@ -861,7 +869,7 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
 #pragma unroll
         for (uint32_t w = g; w < NGRP; w += HPC) acc += o[w][hq] * ex2(misc->mfin[w][hq] - m);
         acc_h[g * 4 + hq] = acc;
-        const uint32_t h = (g0 + g) * p.qpg + hq;
+        const uint32_t h = (hg0 + g) * p.qpg + hq;
         if (n_splits == 1) {
           put(h, dim, acc * (1.0f / l));
         } else if (MODE != 1 && merger) {  // stays in the CTA
@@ -897,7 +905,7 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
         }
         const uint32_t n_oth = n_splits - 1;
         const uint32_t mine = quad < n_oth ? (n_oth - quad + 3) / 4 : 0;  // other splits quad, quad + 4, ...
-        merge_part<10>(p, lane, quad, 4, mine, split, g0 * p.qpg + hl, qd * 32 + lane, tag, &abort_s, m_r, l_r, o_r);
+        merge_part<10>(p, lane, quad, 4, mine, split, hg0 * p.qpg + hl, qd * 32 + lane, tag, &abort_s, m_r, l_r, o_r);
         misc->xo[quad][lane] = o_r;
         if (lane == 0) {
           misc->xm[quad] = m_r;
@@ -914,10 +922,10 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
             o_all = fmaf(misc->xo[w][lane], e, o_all);
             l_all = fmaf(misc->xl[w], e, l_all);
           }
-          put(g0 * p.qpg + hl, qd * 32 + lane, o_all * (1.0f / l_all));
+          put(hg0 * p.qpg + hl, qd * 32 + lane, o_all * (1.0f / l_all));
           // The next launch's tag. Safe to advance once unit 0 is merged: its warps have seen every split's
           // tag, so every CTA of the group has read the epoch.
-          if (u == 0 && lane == 0) *reinterpret_cast<volatile uint32_t*>(p.epochs + blockIdx.y) = tag;
+          if (u == 0 && lane == 0) *reinterpret_cast<volatile uint32_t*>(p.epochs + group) = tag;
         }
         if (u + n_splits < HPC * 16) named_bar_sync(SHARE_BAR, 128);  // the exchange area is reused
       }
@@ -939,8 +947,8 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
       const uint32_t hl = u >> 2, d = (u & 3) * 32 + lane;
       float m, l;
       head_ml(hl / 4, hl % 4, m, l);
-      merge_unit<15>(p, lane, n_splits, split, g0 * p.qpg + hl, d, own_part()[hl * BP_HEAD_DIM + d], m, l, tag, &abort_s);
-      if (u == 0 && lane == 0) *reinterpret_cast<volatile uint32_t*>(p.epochs + blockIdx.y) = tag;  // as in mode 1
+      merge_unit<15>(p, lane, n_splits, split, hg0 * p.qpg + hl, d, own_part()[hl * BP_HEAD_DIM + d], m, l, tag, &abort_s);
+      if (u == 0 && lane == 0) *reinterpret_cast<volatile uint32_t*>(p.epochs + group) = tag;  // as in mode 1
     }
   }
 
@@ -972,6 +980,8 @@ cudaError_t bp_decode_umma_init(bp_attn_ctx* c) {
   cudaError_t e = umma_attr<1>();
   if (e != cudaSuccess) return e;
   e = umma_attr<2>();
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(decode_umma_kernel<1, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(U_SMEM_BUDGET));
   if (e != cudaSuccess) return e;
   // The in-kernel merge makes the CTAs of a head group wait for one another, so a launch may never
   // have more CTAs than the device holds at once: ask the runtime instead of assuming one per SM.
@@ -1043,46 +1053,29 @@ static cudaError_t launch_umma(bp_attn_ctx* c, cudaStream_t s, UmmaParams& p, ui
   return bp_launch(c->opt_pdl != 0, decode_umma_kernel<HPC, 1>, grid, dim3(U_THREADS), smem, s, c->umaps_dev, p);
 }
 
-cudaError_t bp_launch_decode_umma(bp_attn_ctx* c, cudaStream_t s, uint32_t layer, const __half* q, __half* out,
-                                  uint32_t cur_pos, uint32_t* n_splits_out, const bp_fused_step* fs) {
-  const uint32_t spp = umma_spp(c, cur_pos);
-  const uint32_t n_splits = bp_decode_umma_splits(c, cur_pos);
-  UmmaParams p;
+// What a launch of layer `layer` (or of several from it on) has in common.
+static UmmaParams umma_params(bp_attn_ctx* c, uint32_t layer, const __half* q, __half* out, uint32_t cur_pos, const bp_fused_step* fs) {
+  UmmaParams p = {};
   p.q = q;
   p.out = out;
   p.partials = c->partials;
   p.err = c->err_dev;
   p.row_base = layer * c->cfg.max_seq;
   p.cur_pos = cur_pos;
-  p.tps = spp * UT;
   p.nk = p.nv = 1;
   p.n_head = c->cfg.n_head;
   p.qpg = c->qpg;
   p.sm_scale_log2 = (1.0f / sqrtf(static_cast<float>(BP_HEAD_DIM))) * 1.4426950408889634f;
   p.dbg = c->dbg_on ? c->dbg_dev : nullptr;
-  p.n_px = c->n_px;
-  p.px_off = layer * c->cfg.n_shards * c->q_dim + c->cfg.shard * c->q_dim;
-  p.px_out = c->px_dev;
-  // The in-kernel merge makes CTAs wait for one another: all of them must be resident at once,
-  // which only a caller with the device to itself can promise (option exclusive_device). The
-  // exchange lives in the in-kernel merge.
-  p.merge = (c->opt_umerge && c->opt_exclusive) || c->n_px > 0;
   p.wait_limit = c->opt_wait_limit;
   p.poll_limit = c->opt_poll_limit;
   p.v_pre_all = c->opt_vpre;
-  p.fresh_from = bp_fresh_from(c, layer);
-  const uint32_t px_slot = c->n_px > 0 && c->opt_px_meet && layer > 0 ? (layer - 1) % 64 : NO_SLOT;
-  p.px_meet = px_slot | c->cfg.shard << 8;
-  p.px_tab = c->pxf_dev;
   p.ll = c->ll;
   p.epochs = c->epochs;
   p.fused = fs != nullptr ? 1u : 0u;
   p.eps = c->cfg.rms_eps;
   p.n_kv_head = c->cfg.n_kv_head;
-  p.q_roped = nullptr;
-  p.w_q = p.w_k = p.k_cur = p.v_cur = p.rope_row = nullptr;
-  p.k_d = p.v_d = nullptr;
-  p.k_qs = p.v_qs = nullptr;
+  p.px_meet = NO_SLOT;
   if (fs != nullptr) {
     p.q_roped = fs->q_roped;
     p.w_q = fs->w_q;
@@ -1095,8 +1088,84 @@ cudaError_t bp_launch_decode_umma(bp_attn_ctx* c, cudaStream_t s, uint32_t layer
     p.k_qs = reinterpret_cast<uint32_t*>(c->kv[0] + bp_qs_off(c, layer));
     p.v_qs = reinterpret_cast<uint32_t*>(c->kv[1] + bp_qs_off(c, layer));
   }
+  return p;
+}
+
+cudaError_t bp_launch_decode_umma(bp_attn_ctx* c, cudaStream_t s, uint32_t layer, const __half* q, __half* out,
+                                  uint32_t cur_pos, uint32_t* n_splits_out, const bp_fused_step* fs) {
+  const uint32_t spp = umma_spp(c, cur_pos);
+  const uint32_t n_splits = bp_decode_umma_splits(c, cur_pos);
+  UmmaParams p = umma_params(c, layer, q, out, cur_pos, fs);
+  p.tps = spp * UT;
+  p.n_px = c->n_px;
+  p.px_off = layer * c->cfg.n_shards * c->q_dim + c->cfg.shard * c->q_dim;
+  p.px_out = c->px_dev;
+  // The in-kernel merge makes CTAs wait for one another: all of them must be resident at once,
+  // which only a caller with the device to itself can promise (option exclusive_device). The
+  // exchange lives in the in-kernel merge.
+  p.merge = (c->opt_umerge && c->opt_exclusive) || c->n_px > 0;
+  p.fresh_from = bp_fresh_from(c, layer);
+  const uint32_t px_slot = c->n_px > 0 && c->opt_px_meet && layer > 0 ? (layer - 1) % 64 : NO_SLOT;
+  p.px_meet = px_slot | c->cfg.shard << 8;
+  p.px_tab = c->pxf_dev;
   *n_splits_out = p.merge ? 1 : n_splits;  // nothing left to merge for the caller
   if (fs != nullptr) bp_note_row_write(c, layer, cur_pos - 1);
   bp_note_sm_launch(c, n_splits * (c->cfg.n_kv_head / c->opt_uhpc));
   return c->opt_uhpc == 2 ? launch_umma<2>(c, s, p, spp, n_splits) : launch_umma<1>(c, s, p, spp, n_splits);
+}
+
+// The fused steps of ALL layers as one launch or two, for activations that are all there before the first layer
+// (bp_decode_token_host): a call per layer is a chain of 36 kernels whose two ends, about 7 us, stream nothing; a launch
+// over the layers' (layer, KV head) pairs streams through them (36 layers at 4096 keys, call from and to pinned host
+// memory: 360 us as a chain in a graph, 122 here). Pairs that fill the device are not split at all; those that are left
+// over, or all of a small shard's, are split as far as every CTA is resident (the merge makes them wait for one another).
+// Plain launches: the cache is settled, so every row is requested at once.
+bool bp_decode_layers_batched(const bp_attn_ctx* c) {
+  return bp_use_umma(c) && c->opt_uhpc == 1 && c->n_px == 0 && c->opt_umerge && c->opt_exclusive &&
+         c->cfg.n_layer * c->cfg.n_kv_head >= BP_BATCHED_PAIRS && c->cfg.n_kv_head <= c->umma_resident;
+}
+cudaError_t bp_launch_decode_layers(bp_attn_ctx* c, cudaStream_t s, const __half* q, __half* out, uint32_t cur_pos, const bp_fused_step& fs,
+                                    uint32_t* launches) {
+  const uint32_t groups = c->cfg.n_kv_head, fit = c->umma_resident, n_st = (cur_pos + UT - 1) / UT;
+  const size_t ll_units = static_cast<size_t>(fit) * c->qpg * BP_LL_STRIDE;  // a tagged partial of every head of every CTA
+  if (c->ll_layers == nullptr) {
+    cudaError_t e = cudaMalloc(&c->ll_layers, ll_units * sizeof(uint2) + fit * sizeof(uint32_t));
+    if (e != cudaSuccess) return e;
+    e = cudaMemsetAsync(c->ll_layers, 0, ll_units * sizeof(uint2) + fit * sizeof(uint32_t), s);
+    if (e != cudaSuccess) return e;
+  }
+  for (uint32_t il = 0; il < c->cfg.n_layer;) {
+    uint32_t layers = c->cfg.n_layer - il, splits = 1;
+    const uint32_t ctas = layers * groups, tail = ctas % fit;
+    if (ctas <= fit) {
+      splits = fit / ctas;
+      if (splits > (n_st + 1) / 2) splits = (n_st + 1) / 2;  // two stages are one split, as in umma_spp
+    } else if (tail != 0 && tail * 4 < fit * 3) {
+      layers = (ctas - tail) / groups;  // whole waves; the rest is split over the device in the next launch
+    }
+    const uint32_t spp = (n_st + splits - 1) / splits;
+    splits = (n_st + spp - 1) / spp;
+    bp_fused_step f = fs;
+    f.k_cur += static_cast<size_t>(il) * c->kv_dim;
+    f.v_cur += static_cast<size_t>(il) * c->kv_dim;
+    UmmaParams p = umma_params(c, il, q + static_cast<size_t>(il) * c->q_dim, out + static_cast<size_t>(il) * c->q_dim, cur_pos, &f);
+    p.tps = spp * UT;
+    p.merge = 1;
+    p.row_step = c->cfg.max_seq;
+    p.n_head = c->cfg.n_head * layers;
+    p.fresh_from = UINT32_MAX;
+    p.ll = c->ll_layers;
+    p.epochs = reinterpret_cast<uint32_t*>(c->ll_layers + ll_units);
+    const uint32_t cap = umma_max_stages<1>();
+    p.nk = spp < cap ? spp : cap;
+    p.nv = p.nk;
+    for (uint32_t i = 0; i < layers; i++) bp_note_row_write(c, il + i, cur_pos - 1);
+    bp_note_sm_launch(c, splits * groups * layers);
+    *launches += 1;
+    cudaError_t e = bp_launch(false, decode_umma_kernel<1, 1, true>, dim3(splits, groups, layers), dim3(U_THREADS), ULayout<1>::total(p.nk, p.nv), s,
+                              c->umaps_dev, p);
+    if (e != cudaSuccess) return e;
+    il += layers;
+  }
+  return cudaSuccess;
 }

@@ -27,6 +27,7 @@ struct bp_attn_ctx {
   float* partials;   // device: split-KV scratch [max_splits][n_head][BP_PART_STRIDE]
   uint2* ll;         // device: tagged split partials of the in-kernel merge [max_splits][n_head][BP_LL_STRIDE] (value, tag)
   uint32_t* epochs;  // device: per head group, the tag of the last merged launch (64 words)
+  uint2* ll_layers;  // device, or null: the same two for launches over several layers (bp_launch_decode_layers)
   uint32_t* err_host; // pinned, mapped: kernels store a non-zero code here when a bounded wait gives up
   uint32_t* err_dev;  // device alias of err_host
   uint32_t max_splits;
@@ -224,4 +225,11 @@ cudaError_t bp_launch_decode_umma(bp_attn_ctx* c, cudaStream_t s, uint32_t layer
 cudaError_t bp_launch_decode_fused(bp_attn_ctx* c, cudaStream_t s, uint32_t layer, const __half* q_raw, __half* q_roped,
                                    const __half* w_q, const __half* k_cur, const __half* v_cur, const __half* w_k,
                                    uint32_t pos, __half* out, uint32_t* launches);
+// The fused steps of every layer at row cur_pos - 1 in as few launches as the device allows; q, out, fs.k_cur and fs.v_cur
+// hold a row per layer. Worth it from BP_BATCHED_PAIRS (layer, KV head) pairs on: with fewer, a launch leaves most of the
+// device idle or splits every head as the calls per layer do.
+constexpr uint32_t BP_BATCHED_PAIRS = 32;
+bool bp_decode_layers_batched(const bp_attn_ctx* c);
+cudaError_t bp_launch_decode_layers(bp_attn_ctx* c, cudaStream_t s, const __half* q, __half* out, uint32_t cur_pos, const bp_fused_step& fs,
+                                    uint32_t* launches);
 inline bool bp_use_umma(const bp_attn_ctx* c) { return c->variant == 0 && c->qpg == 4 && c->have_umaps; }

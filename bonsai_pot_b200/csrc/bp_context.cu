@@ -375,6 +375,7 @@ void bp_attn_destroy(bp_attn_ctx* c) {
   cudaFree(c->umaps_dev);
   cudaFree(c->pmaps_dev);
   cudaFree(c->ll);
+  cudaFree(c->ll_layers);
   cudaFree(c->epochs);
   cudaFree(c->px_epoch);
   cudaFree(c->pxf_dev);
@@ -711,7 +712,10 @@ int bp_decode_token_host(bp_attn_ctx* c, const void* q, const void* k, const voi
   uint32_t launches = 0;
   if (c->variant == 0 && bp_use_umma(c)) {
     // fused layer steps: the decode kernel normalises q and writes the new cache row itself
-    if (c->opt_token_graph) {
+    if (c->opt_token_graph && bp_decode_layers_batched(c)) {
+      BP_CUDA(c, bp_launch_decode_layers(c, st, c->stage_q, c->stage_out, pos + 1,
+                                         bp_fused_step{nullptr, c->stage_wq, c->stage_wk, c->stage_k, c->stage_v}, &launches));
+    } else if (c->opt_token_graph) {
       if (int s = token_graph_launch(c, st, pos, &launches)) return s;
     } else {
       for (uint32_t il = 0; il < nl; il++) BP_CUDA(c, token_layer_call(c, st, il, pos, &launches));

@@ -189,7 +189,10 @@ int bp_decode_step_host(bp_attn_ctx* ctx, uint32_t layer, const void* q_host, co
  * one `Session::step` (src/forward.rs:578-672), which the reference submits as
  * a single command buffer per token. q_host, out_host: f16 [n_layer][n_head*128];
  * k_host, v_host: f16 [n_layer][n_kv_head*128]. One host-to-device copy per
- * input, the kernels of every layer in order, one copy back, one synchronise. */
+ * input, the layers' kernels, one copy back, one synchronise. With 32 (layer, KV head)
+ * pairs and more the layers' steps run together in one launch or two: no layer reads
+ * what another wrote. That splits a head's tokens otherwise than a call per layer, so
+ * the outputs agree with it to rounding; the cache rows are the same bits. */
 int bp_decode_token_host(bp_attn_ctx* ctx, const void* q_host, const void* k_host, const void* v_host,
                          const void* w_q_norm_host, const void* w_k_norm_host, uint32_t pos,
                          void* out_host);
@@ -261,9 +264,10 @@ int bp_set_variant(bp_attn_ctx* ctx, uint32_t variant);
  * tile, two CTAs per SM; 0 = chosen by batch size: 3 when there are more work
  * items than SMs, else 1). Launch structure: "dependent_launch" (1 = kernels are
  * launched with programmatic stream serialization, the default), "token_graph" (1 = the
- * layers' launches of bp_decode_token_host go to the device as one CUDA graph launch, its
- * nodes given the new position's launch arguments before every token, the default; 0 =
- * stream launches), "decode_in_kernel_merge"
+ * layers of bp_decode_token_host run together, or, with few (layer, KV head) pairs, a peer
+ * exchange, two heads per CTA or without the in-kernel merge, their launches go to the
+ * device as one CUDA graph launch, its nodes given the new position's launch arguments
+ * before every token, the default; 0 = a stream launch per layer), "decode_in_kernel_merge"
  * (1 = the tcgen05 decode kernel merges its splits itself, the default; 0 = a
  * second kernel does), "decode_ring" (K stages * 16 + V slots of the tcgen05
  * decode kernel, 0 = as many as fit), "decode_v_preload" (1 = the first round of

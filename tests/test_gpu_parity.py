@@ -542,6 +542,43 @@ def test_token_host_graph_launch_is_identical_to_stream_launches():
             assert np.array_equal(da.view(np.uint32), db.view(np.uint32)) and np.array_equal(qa, qb)
 
 
+@pytest.mark.parametrize("n_layer,n_kv,launches", [(4, 8, 1), (5, 8, 1), (36, 1, 1), (18, 8, 1), (20, 8, 2), (36, 8, 1)])
+def test_token_host_over_all_layers_agrees_with_a_call_per_layer(n_layer, n_kv, launches):
+    """From 32 (layer, KV head) pairs on bp_decode_token_host takes the layers together: pairs that fill the device are
+    not split, the others by what is resident (4 x 8 pairs: 4 splits, 36 x 1: 4, 20 x 8: 18 layers whole and 2 with 9
+    splits). Short, stage-edge and longer contexts, back and forth: the cache rows bit for bit, the outputs as far as
+    the order of the sums goes (f16 outputs of FP32 sums: half an ulp either way, 2^-10 of the value, and 1e-4 where
+    values cancel)."""
+    sh = O.Shape(n_layer=n_layer, max_seq=1300, n_head=4 * n_kv, n_kv_head=n_kv)
+    rng = np.random.default_rng(31)
+    w = synth.ones_weight()
+    positions = [0, 1, 127, 128, 255, 256, 1290, 300, 1299]
+    seq = [[rng.standard_normal(n_layer * d).astype(np.float16) for d in (sh.q_dim, sh.kv_dim, sh.kv_dim)] for _ in positions]
+    results = []
+    for graph in (1, 0):
+        with make_ctx(sh) as ctx:
+            ctx.set_option("token_graph", graph)
+            fill = np.random.default_rng(32)
+            for il in range(n_layer):
+                for kind in range(2):
+                    ctx.kv_import(kind, il, 0, 1300, (fill.random((1300, sh.nb), dtype=np.float32) * 0.05 + 0.001))
+                    ctx.kv_import(kind, il, 1, 1300, fill.integers(-127, 128, (1300, sh.kv_dim), dtype=np.int8))
+            outs = []
+            for (q, k, v), pos in zip(seq, positions):
+                out = np.zeros((n_layer, sh.q_dim), dtype=np.float16)
+                ctx.decode_token_host(q, k, v, w, w, pos, out)
+                outs.append(out.astype(np.float32))
+                sms = torch.cuda.get_device_properties(0).multi_processor_count
+                assert ctx.last_launch_count() == (n_layer if not graph else launches) or sms != 148
+            assert not ctx.status()
+            results.append((outs, [read_cache(ctx, sh, il, 1300) for il in range(n_layer)]))
+    for a, b in zip(results[0][0], results[1][0]):
+        assert (np.abs(a - b) <= 1e-4 + 2.0 ** -10 * np.abs(b)).all()
+    for ra, rb in zip(results[0][1], results[1][1]):
+        for (da, qa), (db, qb) in zip(ra, rb):
+            assert np.array_equal(da.view(np.uint32), db.view(np.uint32)) and np.array_equal(qa, qb)
+
+
 @pytest.mark.parametrize("warps,hpc", [(16, 8), (8, 4), (8, 2), (16, 1), (8, 1)])
 def test_decode_tuning_options_do_not_change_results(warps, hpc):
     sh = O.Shape(n_layer=2, max_seq=4096)
