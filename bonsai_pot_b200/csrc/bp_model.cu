@@ -560,14 +560,15 @@ int quantize_and_matmul(bp_model* m, const __half* act, uint32_t k, uint32_t mt,
   uint32_t* err = m->attn->err_dev;
   const uint32_t limit = m->attn->opt_mm_wait_limit;
   if (bp_q1_matmul_is_tiled(mt)) {
+    const uint32_t nt = bp_q1_tile_tokens(w, n_w, mt);
     if (norm != nullptr) {
-      M_CUDA(m, bp_q1_rms_quantize_tiled(true, s, act, norm, m->cfg.rms_eps, k, mt, m->a_tiled, m->a_tiled_d));
+      M_CUDA(m, bp_q1_rms_quantize_tiled(true, s, act, norm, m->cfg.rms_eps, k, mt, nt, m->a_tiled, m->a_tiled_d));
     } else if (up != nullptr) {
-      M_CUDA(m, bp_q1_silu_quantize_tiled(true, s, act, up, k, mt, m->a_tiled, m->a_tiled_d));
+      M_CUDA(m, bp_q1_silu_quantize_tiled(true, s, act, up, k, mt, nt, m->a_tiled, m->a_tiled_d));
     } else {
-      M_CUDA(m, bp_q1_quantize_tiled(true, s, act, k, mt, m->a_tiled, m->a_tiled_d));
+      M_CUDA(m, bp_q1_quantize_tiled(true, s, act, k, mt, nt, m->a_tiled, m->a_tiled_d));
     }
-    M_CUDA(m, bp_q1_matmul_tiled(true, s, w, out, n_w, mt, m->a_tiled, m->a_tiled_d, accumulate, err, limit));
+    M_CUDA(m, bp_q1_matmul_tiled(true, s, w, out, n_w, mt, nt, m->a_tiled, m->a_tiled_d, accumulate, err, limit));
     return BP_OK;
   }
   if (int st = untiled_buffers(m)) return st;

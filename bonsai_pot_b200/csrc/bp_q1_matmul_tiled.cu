@@ -13,7 +13,11 @@
 //     which changes the bits);
 //   - the sign bits of a sub-block are one 32-bit word w, and word g of its 32 bytes is (w << g) & 0x80808080
 //     xor 0xB8B8B8B8 (e4m3 +-1): two instructions per four weights. That puts input 8 j + 7 - g of a sub-block
-//     at byte 4 g + j, and the quantiser writes the activations in the same order.
+//     at byte 4 g + j, and the quantiser writes the activations in the same order;
+//   - the weights are the rows of a tile and the tokens its columns, so a batch pays for its tokens in steps of 16.
+//     (With the tokens on the 128 TMEM lanes and a tile of up to 128 weight rows a batch of 21 tokens paid for 128, one of
+//     173 for 256. A block of 128 inputs took a tile of 128 x 112 outputs 1.79 us with the staging in the worker warps; here
+//     128 x 128 outputs take 1.74, 128 x 64 1.15, 128 x 16 0.85.)
 #include <cuda_fp16.h>
 
 #include "bp_common.cuh"
@@ -25,16 +29,14 @@ namespace {
 
 using namespace bp;
 
-constexpr uint32_t TT_M = 128;                    // tokens of a tile = TMEM lanes
-constexpr uint32_t TT_PART = TT_M * 128;          // one part (16 rint(q / 16), or the remainder) of a tile's block of 128 inputs
-constexpr uint32_t TT_WORKERS = 16;               // worker warps: 4 quarters of the TMEM lanes x 4 groups of columns
-constexpr uint32_t TT_THREADS = (1 + TT_WORKERS) * 32;
-constexpr uint32_t TT_STAGES = 4;
+constexpr uint32_t TT_M = 128;                       // weight rows of a tile = TMEM lanes
+constexpr uint32_t TT_A = TT_M * 128;                // a block of 128 inputs of a tile's weights: one byte per weight
+constexpr uint32_t TT_RAW = TT_M * 16, TT_RAWS = 8;  // sign bits of a block of a tile, and blocks of them on their way
 
 // ---- activations -------------------------------------------------------------------------------------------
-// Tiled activations of a batch: per tile of 128 tokens and block of 128 inputs, 2 x 16 KB: part 0 and part 1 as
-// [128 tokens][128 bytes], a token's 16-byte chunks xor-ed with (token mod 8): the layout the MMA reads
-// (K-major, 128-byte swizzle), so a stage is ONE bulk copy. Scales: [tile][block][128 tokens][4 sub-blocks].
+// Tiled activations of a batch: per tile of N tokens and block of 128 inputs, part 0 (16 rint(q / 16)) and then part 1
+// (the remainder) as [N tokens][128 bytes], a token's 16-byte chunks xor-ed with (token mod 8): the layout the MMA reads
+// (K-major, 128-byte swizzle), so a stage is ONE bulk copy. Scales: [tile][block][4 sub-blocks][N tokens].
 enum { SRC_PLAIN = 0, SRC_RMS = 1, SRC_SILU = 2 };
 
 // quantize_q8_0.wgsl after nothing, after rms_norm.wgsl:41-85, or after silu_mul.wgsl:18-27: the producing
@@ -42,7 +44,8 @@ enum { SRC_PLAIN = 0, SRC_RMS = 1, SRC_SILU = 2 };
 // invocation count: its sum is per invocation). Four lanes share a sub-block: lane t takes the inputs of output
 // words 2 t and 2 t + 1, which are the pairs 8 j + 6 - 2 t, 8 j + 7 - 2 t.
 template <int SRC>
-__global__ void __launch_bounds__(512) quantize_tiled_kernel(const __half* x, const __half* aux, uint32_t k, float eps, uint8_t* a_t, float* a_d) {
+__global__ void __launch_bounds__(512) quantize_tiled_kernel(const __half* x, const __half* aux, uint32_t k, float eps, uint32_t n_tok, uint8_t* a_t,
+                                                             float* a_d) {
   __shared__ float part[32];
   pdl_launch_dependents();
   pdl_wait();
@@ -58,8 +61,8 @@ __global__ void __launch_bounds__(512) quantize_tiled_kernel(const __half* x, co
     const float total = workgroup_sum<16>(s, part);
     inv2 = __half2half2(__float2half_rn(__frsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(k)), eps))));
   }
-  const uint32_t r = row % TT_M, t = tid & 3u;
-  const size_t tile0 = static_cast<size_t>(row / TT_M) * nb1;
+  const uint32_t r = row % n_tok, t = tid & 3u, part_b = n_tok * 128u;
+  const size_t tile0 = static_cast<size_t>(row / n_tok) * nb1;
   for (uint32_t u = tid; u < k / 8u; u += 512) {  // (k / 8 is a multiple of 16: the four lanes of a sub-block stay together)
     const uint32_t sub = u >> 2;
     float v[8];
@@ -101,20 +104,20 @@ __global__ void __launch_bounds__(512) quantize_tiled_kernel(const __half* x, co
       lo[w] = b01 | (static_cast<uint32_t>(b23) << 16);
     }
     const uint32_t kb = sub >> 2, s = sub & 3u;
-    uint8_t* dst = a_t + (tile0 + kb) * (2u * TT_PART) + r * 128u + (((2u * s + (t >> 1)) ^ (r & 7u)) << 4) + 8u * (t & 1u);
+    uint8_t* dst = a_t + (tile0 + kb) * (2u * part_b) + r * 128u + (((2u * s + (t >> 1)) ^ (r & 7u)) << 4) + 8u * (t & 1u);
     *reinterpret_cast<uint2*>(dst) = make_uint2(hi[0], hi[1]);
-    *reinterpret_cast<uint2*>(dst + TT_PART) = make_uint2(lo[0], lo[1]);
-    if (t == 0) a_d[((tile0 + kb) * TT_M + r) * 4u + s] = d;
+    *reinterpret_cast<uint2*>(dst + part_b) = make_uint2(lo[0], lo[1]);
+    if (t == 0) a_d[((tile0 + kb) * 4u + s) * n_tok + r] = d;
   }
 }
 
 // ---- product -----------------------------------------------------------------------------------------------
-struct TiledTensors {  // up to three weight tensors over the same activations: column tile blockIdx.x belongs to one of them
+struct TiledTensors {  // up to three weight tensors over the same activations: row tile blockIdx.x belongs to one of them
   const __half* w_d[3];
   const uint8_t* w_qs[3];
   __half* y[3];
   uint32_t n[3];
-  uint32_t tile_end[3];  // running total of column tiles
+  uint32_t tile_end[3];  // running total of row tiles
 };
 
 __device__ __forceinline__ void umma_f8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
@@ -128,17 +131,25 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
                : "memory");
 }
-__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t* r) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
+// 16-byte global -> shared copy; cp_async_arrive: this thread's copies so far arrive (once) on the mbarrier when they have landed
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
-template <uint32_t W>
-__device__ __forceinline__ void tmem_ld_w(uint32_t taddr, uint32_t (&r)[16]) {
-  static_assert(W == 8 || W == 12 || W == 16, "widths of a load");
-  if constexpr (W == 16) {
-    tmem_ld16(taddr, r);
+__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+}
+// 16 TMEM lanes x 8 GROUPS columns: the thread gets, per group of 8 columns, columns 2 (lane mod 4) + {0, 1} of row
+// lane / 4 (r[0], r[1]) and of row lane / 4 + 8 (r[2], r[3]).
+template <uint32_t GROUPS>
+__device__ __forceinline__ void tmem_ld_rows16(uint32_t taddr, uint32_t* r) {
+  static_assert(GROUPS == 1 || GROUPS == 2, "groups of a load");
+  if constexpr (GROUPS == 1) {
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
   } else {
-    tmem_ld8(taddr, reinterpret_cast<uint32_t(&)[8]>(r));
-    if constexpr (W == 12) tmem_ld4(taddr + 8, r + 8);
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
   }
 }
 __device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
@@ -158,34 +169,55 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
   return v;
 }
 
-// A CTA owns 128 tokens x 4 NC weight rows and runs alone on its SM.
-//   worker warps      stage a block of 128 inputs two blocks ahead (thread = one sub-block of one weight row: a word
-//                     of signs -> 32 bytes; one thread requests the activations), then take finished sub-blocks out
-//                     of TMEM: thread = token = TMEM lane, NC weight rows, sums in registers over all blocks
-//   warp 0, lane 0    issues the MMAs, G sub-blocks per hand-over, into one of two sets of G TMEM buffers
-// What bounds it (128 x 112 tile, cycles per sub-block, stamps in the kernel): 855, of them 510 the scaling and adding
-// (336 if only the FMA pipe counted), 220 the staging (its proxy fence above all), 120 waiting for the MMAs; the
-// tensor pipe is 13 % busy, the issue slots 58 % (gate + up of 512 tokens under ncu). A pass of 512 tokens at the Bonsai-8B shape: 37.9 ms with the
-// mma.sync kernel, 29.2 now; 21 tokens: 53 ms with the CUDA-core kernel, 11.8 now. Slower (ms per 512-token pass): four
-// sets of one sub-block 32.6, the staging in four warps of its own 30.4, two issuing threads with the next
-// hand-over's first load before the last piece is added 30.8, scalar instead of packed sums and products: no change.
+// A CTA owns 128 weight rows x N tokens and runs alone on its SM. The weights are the A operand (their rows are
+// the TMEM lanes), the tokens the columns, so a batch costs by its tokens in steps of 16.
+//   loader warp       sign bits (asynchronous copies) and scales TT_RAWS blocks ahead; one lane requests the activations
+//                     and their scales for a free stage
+//   stager warps      a block's 128 x 128 sign bits -> one byte per weight
+//   issuer warp       one thread issues the MMAs, G sub-blocks per hand-over, into one of BUFS sets of G TMEM buffers
+//   worker warps      take finished sub-blocks out of TMEM, scale and add them: sums in registers over all blocks
 // Every wait is bounded; a wait that gives up stores a code in the error word and the CTA winds down: it ends only
 // when its own copies have landed and its own MMAs are complete (waits of TT_DRAIN polls, whatever the caller's limit:
 // what is waited for there always comes), because the next CTA on the SM gets the same shared memory and TMEM.
 constexpr uint32_t TT_DRAIN = 1u << 20;
-template <uint32_t NC>
-__global__ void __launch_bounds__(TT_THREADS, 1) matmul_q1_tiled_kernel(const TiledTensors tensors, uint32_t k, uint32_t m, const uint8_t* __restrict__ a_t,
+
+template <uint32_t V>
+struct Num {  // a constant as an argument
+  static constexpr uint32_t value = V;
+};
+
+template <uint32_t N_>
+struct TtLayout {
+  static constexpr uint32_t N = N_;
+  // Worker warps: 4 quarters of the TMEM lanes x CG groups of NC tokens. Stager warps: as many as leave the workers
+  // their registers (a scheduler's 16384 are shared by a quarter of the warps: up to 20 warps have 96 each).
+  static constexpr uint32_t CG = N == 16 ? 2 : N == 48 ? 3 : 4, NC = N / CG, WORKERS = 4 * CG;
+  static constexpr uint32_t STAGERS = N > 64 ? 2 : 4;
+  static constexpr uint32_t LOADER = WORKERS + STAGERS, ISSUER = LOADER + 1;  // the warps that request copies and issue MMAs
+  static constexpr uint32_t THREADS = (ISSUER + 1) * 32;
+  static constexpr uint32_t B = 2 * N * 128, AD = N * 16, WD = TT_M * 4;
+  static constexpr uint32_t STAGE = TT_A + B;                         // operands: a multiple of 1024
+  static constexpr uint32_t STAGES = N > 64 ? 4 : N == 64 ? 6 : N == 48 ? 7 : 8;
+  static constexpr uint32_t OFF_AD = STAGES * STAGE, OFF_WD = OFF_AD + STAGES * AD;
+  static constexpr uint32_t OFF_RAW = OFF_WD + STAGES * WD;           // sign bits as they are in memory: [128 rows][16 bytes] per block
+  static constexpr uint32_t SMEM = OFF_RAW + TT_RAWS * TT_RAW + 1024;
+  static constexpr uint32_t G = N > 64 ? 2 : 4, STEPS = 4 / G;        // sub-blocks per hand-over, hand-overs per block
+  static constexpr uint32_t COLS = N > 64 ? 128 : N > 32 ? 64 : N;    // TMEM columns of one buffer
+  static constexpr uint32_t BUFS = N > 32 ? 2 : 4;                    // sets of G TMEM buffers
+  // a piece is what is loaded from TMEM at a time: up to 16 values of a thread, PS sub-blocks or 1 / PPS of one
+  static constexpr uint32_t PS = NC == 8 ? 2 : 1, PPS = NC > 16 ? 2 : 1, Q = G * PPS / PS;
+  static_assert(BUFS * G * COLS <= 512 && N % 16 == 0 && NC % 8 == 0 && SMEM <= 227 * 1024 - 1024, "limits of an SM");
+};
+
+template <uint32_t N>
+__global__ void __launch_bounds__(TtLayout<N>::THREADS, 1) matmul_q1_tiled_kernel(const TiledTensors tensors, uint32_t k, uint32_t m, const uint8_t* __restrict__ a_t,
                                                                         const float* __restrict__ a_d, uint32_t accumulate, float one, uint32_t* err,
                                                                         uint32_t wait_limit, uint32_t poll_ns) {
-  constexpr uint32_t N = 4 * NC, STAGE_B = 2 * TT_PART + N * 128;
-  constexpr uint32_t G = NC > 16 ? 2 : 4, STEPS = 4 / G;      // sub-blocks per hand-over, hand-overs per block
-  constexpr uint32_t BUFS = 2;                                                             // sets of G TMEM buffers
-  constexpr uint32_t COLS = N > 64 ? 128 : N;                 // TMEM columns of one buffer
-  constexpr uint32_t W0 = NC < 16 ? NC : 16, W1 = NC - W0, PIECES = W1 != 0 ? 2 : 1;  // columns of a TMEM load
-  static_assert(BUFS * G * COLS <= 512, "TMEM has 512 columns");
+  using L = TtLayout<N>;
+  constexpr uint32_t NC = L::NC, G = L::G, STEPS = L::STEPS, BUFS = L::BUFS, COLS = L::COLS, STAGES = L::STAGES;
   extern __shared__ uint8_t tt_raw[];
-  __shared__ __align__(8) uint64_t full[TT_STAGES], a_full[TT_STAGES], empty[TT_STAGES], d_full[BUFS], d_empty[BUFS], drained;
-  __shared__ __align__(16) float s_wd[TT_WORKERS][2][32];
+  __shared__ __align__(8) uint64_t full[STAGES], a_full[STAGES], empty[STAGES], d_full[BUFS], d_empty[BUFS], drained;
+  __shared__ __align__(8) uint64_t raw_full[TT_RAWS], raw_empty[TT_RAWS];
   __shared__ uint32_t tmem_base_s;
   __shared__ volatile uint32_t abort_s;
   const uint32_t smem_base = (smem_u32(tt_raw) + 1023u) & ~1023u;
@@ -196,23 +228,27 @@ __global__ void __launch_bounds__(TT_THREADS, 1) matmul_q1_tiled_kernel(const Ti
   // (selects: an indexed parameter array would be copied to local memory)
   auto pick = [&](const auto* v) { return which == 0 ? v[0] : which == 1 ? v[1] : v[2]; };
   const uint32_t n = pick(tensors.n);
-  const uint32_t n_base = (tile - (which == 0 ? 0u : which == 1 ? tensors.tile_end[0] : tensors.tile_end[1])) * N, m_base = blockIdx.y * TT_M;
+  const uint32_t n_base = (tile - (which == 0 ? 0u : which == 1 ? tensors.tile_end[0] : tensors.tile_end[1])) * TT_M, m_base = blockIdx.y * N;
   const uint32_t nb1 = k / 128u;
   if (tid == 0) {
-    for (uint32_t i = 0; i < TT_STAGES; i++) {
-      mbar_init(smem_u32(&full[i]), TT_WORKERS);
+    for (uint32_t i = 0; i < STAGES; i++) {
+      mbar_init(smem_u32(&full[i]), 2);  // stager and loader
       mbar_init(smem_u32(&a_full[i]), 1);
-      mbar_init(smem_u32(&empty[i]), 1);
+      mbar_init(smem_u32(&empty[i]), 1 + L::WORKERS);
     }
     for (uint32_t i = 0; i < BUFS; i++) {
       mbar_init(smem_u32(&d_full[i]), 1);
-      mbar_init(smem_u32(&d_empty[i]), TT_WORKERS);
+      mbar_init(smem_u32(&d_empty[i]), L::WORKERS);
+    }
+    for (uint32_t i = 0; i < TT_RAWS; i++) {
+      mbar_init(smem_u32(&raw_full[i]), 32);
+      mbar_init(smem_u32(&raw_empty[i]), 1);
     }
     mbar_init(smem_u32(&drained), 1);
     abort_s = 0;
     fence_barrier_init();
   }
-  if (warp == 0) tmem_alloc(smem_u32(&tmem_base_s), 512);
+  if (warp == L::ISSUER) tmem_alloc(smem_u32(&tmem_base_s), 512);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -245,17 +281,17 @@ __global__ void __launch_bounds__(TT_THREADS, 1) matmul_q1_tiled_kernel(const Ti
     atomicExch(err, 6u);
   };
 
-  if (warp == 0) {
+  if (warp == L::ISSUER) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    pdl_wait();  // the polls below count from here: the time of the kernel before this one is not theirs
+    if (elect_one()) {
       constexpr uint32_t IDESC = umma_idesc(1, 0, 0, 0, 0, TT_M, N);  // f32 = e4m3 (K-major) x e4m3 (K-major)
       const uint64_t dk = umma_desc_sw128(0, 16, 1024);
-      pdl_wait();  // the polls below count from here: the time of the kernel before this one is not theirs
       for (uint32_t b = 0; b < nb1; b++) {
-        const uint32_t slot = b % TT_STAGES;
-        waitb(&a_full[slot], (b / TT_STAGES) & 1u, poll_ns);
-        waitb(&full[slot], (b / TT_STAGES) & 1u);
-        const uint64_t ad = dk + ((smem_base + slot * STAGE_B) >> 4), bd = ad + (2u * TT_PART >> 4);
+        const uint32_t slot = b % STAGES;
+        waitb(&a_full[slot], (b / STAGES) & 1u, poll_ns);
+        waitb(&full[slot], (b / STAGES) & 1u);
+        const uint64_t ad = dk + ((smem_base + slot * L::STAGE) >> 4), bd = ad + (TT_A >> 4);
 #pragma unroll
         for (uint32_t h = 0; h < STEPS; h++) {
           const uint32_t j = b * STEPS + h, pb = j % BUFS;
@@ -266,149 +302,194 @@ __global__ void __launch_bounds__(TT_THREADS, 1) matmul_q1_tiled_kernel(const Ti
           for (uint32_t g = 0; g < G; g++)
 #pragma unroll
             for (uint32_t part = 0; part < 2; part++)  // a sub-block: 32 bytes along the row
-              umma_f8(tmem + (pb * G + g) * COLS, ad + part * (TT_PART >> 4) + (h * G + g) * 2u, bd + (h * G + g) * 2u, IDESC, part);
+              umma_f8(tmem + (pb * G + g) * COLS, ad + (h * G + g) * 2u, bd + part * (N * 128u >> 4) + (h * G + g) * 2u, IDESC, part);
           umma_commit(smem_u32(&d_full[pb]));
         }
         if (dead) break;  // no slot is given back any more: a copy into it could meet the previous one
-        umma_commit(smem_u32(&empty[slot]));
+        if (b + STAGES < nb1) umma_commit(smem_u32(&empty[slot]));  // (no arrival that nobody waits for: it could outlive the CTA)
       }
     }
-  } else {
-    // ---------------- workers ----------------
-    const __half* __restrict__ w_d = pick(tensors.w_d);
-    const uint8_t* __restrict__ w_qs = pick(tensors.w_qs);
-    const uint32_t wt = tid - 32u, srow = wt >> 2, ssub = wt & 3u;  // staging: sub-block ssub of weight row srow
-    const bool b_stage = srow < N, b_ok = b_stage && n_base + srow < n;
-    const uint8_t* b_src = w_qs + static_cast<size_t>(n_base + srow) * nb1 * 16u + 4u * ssub;
-    const uint8_t* a_src = a_t + static_cast<size_t>(blockIdx.y) * nb1 * (2u * TT_PART);
-    uint32_t rb = 0, rb2 = 0;  // the signs of the block to be staged next, and of the one after it
-    uint32_t copies = 0;       // blocks of activations requested (one thread)
-    auto fetch = [&](uint32_t b) {
-      rb = rb2;
-      rb2 = b_ok && b < nb1 ? __ldg(reinterpret_cast<const uint32_t*>(b_src + 16u * b)) : 0u;
-    };
-    auto store = [&](uint32_t b) {
-      const uint32_t slot = b % TT_STAGES;
-      if (b >= TT_STAGES) waitb(&empty[slot], ((b / TT_STAGES) - 1u) & 1u);
-      if (wt == 0 && !dead) {
-        mbar_arrive_expect_tx(smem_u32(&a_full[slot]), 2u * TT_PART);
-        bulk_load(smem_base + slot * STAGE_B, a_src + static_cast<size_t>(b) * (2u * TT_PART), 2u * TT_PART, smem_u32(&a_full[slot]));
-        copies = b + 1;
-      }
-      if (b_stage) {
-        uint8_t* brow = smem_gen + slot * STAGE_B + 2u * TT_PART + srow * 128u;
-        uint32_t o[8];
+  } else if (warp == L::LOADER) {
+    // ---------------- loader ----------------
+    constexpr uint32_t RL = TT_M / 32;  // weight rows of a lane: lane, lane + 32, ..
+    const uint8_t* w_qs = pick(tensors.w_qs);
+    const __half* w_d = pick(tensors.w_d);
+    const uint8_t* a_src = a_t + static_cast<size_t>(blockIdx.y) * nb1 * L::B;
+    const float* ad_src = a_d + static_cast<size_t>(blockIdx.y) * nb1 * (4u * N);
+    uint32_t at[RL];  // the lane's rows (one beyond the tensor repeats the last: nobody reads its results)
 #pragma unroll
-        for (uint32_t g = 0; g < 8; g++) o[g] = ((rb << g) & 0x80808080u) ^ 0xB8B8B8B8u;  // bit set: +1 (0x38), clear: -1 (0xB8)
-        *reinterpret_cast<uint4*>(brow + (((2u * ssub) ^ (srow & 7u)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
-        *reinterpret_cast<uint4*>(brow + (((2u * ssub + 1u) ^ (srow & 7u)) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
+    for (uint32_t r = 0; r < RL; r++) at[r] = min(n_base + lane + 32u * r, n - 1u);
+    __half scale[TT_RAWS][RL];
+    uint32_t copies = 0;  // blocks of activations requested (one lane)
+    bool before = true;   // the kernel before this one may still run: the weights are constants, the activations are its results
+    for (uint32_t t0 = 0; t0 < nb1 + TT_RAWS; t0 += TT_RAWS) {
+#pragma unroll
+      for (uint32_t i = 0; i < TT_RAWS; i++) {
+        const uint32_t t = t0 + i;
+        if (t >= TT_RAWS && t - TT_RAWS < nb1) {  // block t - TT_RAWS into its stage
+          const uint32_t b = t - TT_RAWS, slot = b % STAGES;
+          if (before) {
+            pdl_wait();
+            before = false;
+          }
+          if (b >= STAGES) waitb(&empty[slot], ((b / STAGES) - 1u) & 1u);
+          if (lane == 0 && !dead) {
+            mbar_arrive_expect_tx(smem_u32(&a_full[slot]), L::B + L::AD);
+            bulk_load(smem_base + slot * L::STAGE + TT_A, a_src + static_cast<size_t>(b) * L::B, L::B, smem_u32(&a_full[slot]));
+            bulk_load(smem_base + L::OFF_AD + slot * L::AD, ad_src + static_cast<size_t>(b) * (4u * N), L::AD, smem_u32(&a_full[slot]));
+            copies = b + 1;
+          }
+          float* wd = reinterpret_cast<float*>(smem_gen + L::OFF_WD + slot * L::WD);
+#pragma unroll
+          for (uint32_t r = 0; r < RL; r++) wd[lane + 32u * r] = __half2float(scale[i][r]);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&full[slot]));
+        }
+        if (t < nb1) {  // block t requested
+          if (t >= TT_RAWS) waitb(&raw_empty[i], ((t / TT_RAWS) - 1u) & 1u);
+#pragma unroll
+          for (uint32_t r = 0; r < RL; r++) {
+            const size_t blk = static_cast<size_t>(at[r]) * nb1 + t;
+            cp_async16(smem_base + L::OFF_RAW + i * TT_RAW + (lane + 32u * r) * 16u, w_qs + blk * 16u);
+            scale[i][r] = __ldg(w_d + blk);
+          }
+          cp_async_arrive(smem_u32(&raw_full[i]));
+        }
+      }
+    }
+    // no copy may still be on its way when the CTA ends (all have landed unless a wait gave up)
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    if (lane == 0)
+      for (uint32_t b = copies > STAGES ? copies - STAGES : 0; b < copies; b++) (void)mbar_wait(smem_u32(&a_full[b % STAGES]), (b / STAGES) & 1u, TT_DRAIN);
+  } else if (warp >= L::WORKERS) {
+    // ---------------- stagers ----------------
+    // The sign bits of a sub-block are one 32-bit word w, and word g of its 32 bytes is (w << g) & 0x80808080 xor
+    // 0xB8B8B8B8 (e4m3 +-1). A warp takes whole blocks, every STAGERS-th. (A stage is waited for by different stagers in
+    // turn, but none is ever two uses behind: a stager at block b has seen block b - STAGERS - STAGES released, and
+    // stages are released in order.)
+    static_assert(L::STAGERS <= STAGES && TT_RAWS % L::STAGERS == 0, "phases that a stager has to follow");
+    for (uint32_t b = warp - L::WORKERS; b < nb1; b += L::STAGERS) {
+      const uint32_t slot = b % STAGES, rs = b % TT_RAWS;
+      waitb(&raw_full[rs], (b / TT_RAWS) & 1u);
+      uint4 sign[4];
+#pragma unroll
+      for (uint32_t r = 0; r < 4; r++) sign[r] = *reinterpret_cast<const uint4*>(smem_gen + L::OFF_RAW + rs * TT_RAW + (lane + 32u * r) * 16u);
+      __syncwarp();
+      if (lane == 0 && b + TT_RAWS < nb1) mbar_arrive(smem_u32(&raw_empty[rs]));
+      if (b >= STAGES) waitb(&empty[slot], ((b / STAGES) - 1u) & 1u);
+#pragma unroll
+      for (uint32_t r = 0; r < 4; r++) {
+        uint8_t* row = smem_gen + slot * L::STAGE + (lane + 32u * r) * 128u;
+        const uint32_t w[4] = {sign[r].x, sign[r].y, sign[r].z, sign[r].w};
+#pragma unroll
+        for (uint32_t s = 0; s < 4; s++) {
+          uint32_t o[8];
+#pragma unroll
+          for (uint32_t g = 0; g < 8; g++) o[g] = ((w[s] << g) & 0x80808080u) ^ 0xB8B8B8B8u;  // bit set: +1 (0x38), clear: -1 (0xB8)
+          *reinterpret_cast<uint4*>(row + (((2u * s) ^ (lane & 7u)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+          *reinterpret_cast<uint4*>(row + (((2u * s + 1u) ^ (lane & 7u)) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
+        }
       }
       fence_proxy_async();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&full[slot]));
-    };
-    const uint32_t quad = warp & 3u, ew = warp - 1u, cg = ew >> 2;  // TMEM lane quarter; columns NC cg ..
-    const uint32_t row = quad * 32u + lane, mi = m_base + row;
+    }
+  } else {
+    // ---------------- workers ----------------
+    // thread: rows lane / 4 + {0, 8, 16, 24} of its quarter, token pairs 2 (lane mod 4) + {0, 1} of every 8: a scale that
+    // it reads from shared memory serves four rows.
+    const uint32_t quad = warp & 3u, cg = warp >> 2, r0 = quad * 32u + (lane >> 2), c2 = 2u * (lane & 3u);
     const uint32_t t_addr = tmem + ((quad * 32u) << 16) + cg * NC;
-    const bool row_ok = mi < m;
-    const uint32_t my_col = n_base + cg * NC + lane;  // the weight row whose scale this lane fetches for its warp
-    const bool col_ok = lane < NC && my_col < n;
-    const float4* ad_src = reinterpret_cast<const float4*>(a_d) + static_cast<size_t>(blockIdx.y) * nb1 * TT_M + row;
-    const __half* wd_src = w_d + static_cast<size_t>(my_col) * nb1;
-    unsigned long long acc[NC / 2];
+    unsigned long long acc[NC / 8][4];  // [token pair][row]
 #pragma unroll
-    for (uint32_t c = 0; c < NC / 2; c++) acc[c] = 0ull;
+    for (uint32_t c = 0; c < NC / 8; c++)
+#pragma unroll
+      for (uint32_t r = 0; r < 4; r++) acc[c][r] = 0ull;
     const unsigned long long ones = pack2(one, one);
-    // fetch(b) requests block b and makes block b - 1, requested one call earlier, the one that store() writes. The
-    // weights are constants: the first ones are requested before the kernel waits for its predecessor.
-    fetch(0);
-    fetch(1);
-    float wd_next = col_ok ? __half2float(wd_src[0]) : 0.0f;
     pdl_wait();
-    float4 ad_next = row_ok ? *ad_src : make_float4(0.f, 0.f, 0.f, 0.f);
-    store(0);
-    fetch(2);
-    if (nb1 > 1) store(1);
-    fetch(3);
     uint32_t d[2][16];
+    // GC groups of 8 tokens from TMEM column `at` on: [row half][group][4]
+    auto load_rows = [&](uint32_t at, auto gc, uint32_t* r) {
+      tmem_ld_rows16<decltype(gc)::value>(at, r);
+      tmem_ld_rows16<decltype(gc)::value>(at + (16u << 16), r + 4 * decltype(gc)::value);
+    };
     for (uint32_t b = 0; b < nb1; b++) {
-      if (b + 2 < nb1) {
-        store(b + 2);
-        fetch(b + 4);
-      }
-      const float adv[4] = {ad_next.x, ad_next.y, ad_next.z, ad_next.w};
-      float* wd_s = s_wd[ew][b & 1u];
-      wd_s[lane] = wd_next;
-      __syncwarp();
-      if (b + 1 < nb1) {
-        if (row_ok) ad_next = ad_src[static_cast<size_t>(b + 1u) * TT_M];
-        if (col_ok) wd_next = __half2float(wd_src[b + 1u]);
-      }
+      const uint32_t slot = b % STAGES;
+      waitb(&a_full[slot], (b / STAGES) & 1u);
+      waitb(&full[slot], (b / STAGES) & 1u);
+      const float* wd = reinterpret_cast<const float*>(smem_gen + L::OFF_WD + slot * L::WD) + r0;
+      unsigned long long wd2[4];
+#pragma unroll
+      for (uint32_t r = 0; r < 4; r++) wd2[r] = pack2(wd[8 * r], wd[8 * r]);
+      const float* ad_s = reinterpret_cast<const float*>(smem_gen + L::OFF_AD + slot * L::AD) + cg * NC + c2;
 #pragma unroll
       for (uint32_t h = 0; h < STEPS; h++) {
         const uint32_t j = b * STEPS + h, pb = j % BUFS;
         waitb(&d_full[pb], (j / BUFS) & 1u);
         tc_fence_after();
         // the pieces of the G sub-blocks, each load in flight while the previous piece is scaled and added
-        tmem_ld_w<W0>(t_addr + pb * G * COLS, d[0]);
+        auto load = [&](uint32_t q) {
+          uint32_t* r = d[q & 1u];
+          if constexpr (L::PPS == 2) {
+            const uint32_t at = t_addr + (pb * G + q / 2) * COLS;
+            if (q % 2 == 0) load_rows(at, Num<2>(), r);
+            else load_rows(at + 16, Num<(NC > 16 ? NC - 16 : 8) / 8>(), r);
+          } else {
 #pragma unroll
-        for (uint32_t q = 0; q < G * PIECES; q++) {
-          const uint32_t g = q / PIECES, piece = q % PIECES;
+            for (uint32_t i = 0; i < L::PS; i++) load_rows(t_addr + (pb * G + q * L::PS + i) * COLS, Num<(NC > 16 ? 16 : NC) / 8>(), r + i * NC);
+          }
+        };
+        load(0);
+#pragma unroll
+        for (uint32_t q = 0; q < L::Q; q++) {
           tmem_ld_wait();
-          if (q + 1 < G * PIECES) {
-            const uint32_t at = t_addr + (pb * G + (q + 1) / PIECES) * COLS;
-            if ((q + 1) % PIECES == 0) {
-              tmem_ld_w<W0>(at, d[(q + 1) & 1u]);
-            } else if constexpr (W1 != 0) {
-              tmem_ld_w<W1>(at + W0, d[(q + 1) & 1u]);
-            }
+          if (q + 1 < L::Q) {
+            load(q + 1);
           } else {  // the whole hand-over is in registers: its buffers may be overwritten
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&d_empty[pb]));
           }
-          const float ad_s = adv[h * G + g];
-          const unsigned long long ad2 = pack2(ad_s, ad_s);
-          const uint32_t c0 = piece * W0, width = piece == 0 ? W0 : W1;
 #pragma unroll
-          for (uint32_t c = 0; c < width; c += 4) {
-            const float4 w4 = *reinterpret_cast<const float4*>(wd_s + c0 + c);
-            const uint32_t* dq = d[q & 1u] + c;
-            const unsigned long long q01 = mul2(mul2(ad2, pack2(w4.x, w4.y)), pack2(__uint_as_float(dq[0]), __uint_as_float(dq[1])));
-            const unsigned long long q23 = mul2(mul2(ad2, pack2(w4.z, w4.w)), pack2(__uint_as_float(dq[2]), __uint_as_float(dq[3])));
-            acc[(c0 + c) / 2] = fma2(q01, ones, acc[(c0 + c) / 2]);
-            acc[(c0 + c) / 2 + 1] = fma2(q23, ones, acc[(c0 + c) / 2 + 1]);
+          for (uint32_t i = 0; i < L::PS; i++) {
+            const uint32_t g = L::PPS == 2 ? q / 2 : q * L::PS + i;
+            const uint32_t p0 = L::PPS == 2 ? (q % 2) * 2 : 0, groups = L::PPS == 2 ? (q % 2 == 0 ? 2 : (NC - 16) / 8) : NC / 8;
+#pragma unroll
+            for (uint32_t c = 0; c < groups; c++) {
+              const float2 a2 = *reinterpret_cast<const float2*>(ad_s + (h * G + g) * N + 8 * (p0 + c));
+              const unsigned long long ad2 = pack2(a2.x, a2.y);
+#pragma unroll
+              for (uint32_t r = 0; r < 4; r++) {  // rows of the first 16 lanes, then of the second
+                const uint32_t* dq = d[q & 1u] + i * NC + (r >> 1) * 4 * groups + 4 * c + 2 * (r & 1u);
+                const unsigned long long t = mul2(mul2(wd2[r], ad2), pack2(__uint_as_float(dq[0]), __uint_as_float(dq[1])));
+                acc[p0 + c][r] = fma2(t, ones, acc[p0 + c][r]);
+              }
+            }
           }
         }
       }
+      __syncwarp();
+      if (lane == 0 && b + STAGES < nb1) mbar_arrive(smem_u32(&empty[slot]));  // the block's scales are read
     }
-    // no copy may still be on its way when the CTA ends (all have landed unless a wait gave up)
-    if (wt == 0)
-      for (uint32_t b = copies > TT_STAGES ? copies - TT_STAGES : 0; b < copies; b++) (void)mbar_wait(smem_u32(&a_full[b % TT_STAGES]), (b / TT_STAGES) & 1u, TT_DRAIN);
-    __syncwarp();
-    if (row_ok && !dead) {
-      __half* y = pick(tensors.y);
-      __half* dst = y + static_cast<size_t>(mi) * n + n_base + cg * NC;
-      const bool vec = n % 4u == 0 && reinterpret_cast<uintptr_t>(y) % 8u == 0;
+    if (!dead) {
+      const uint32_t t0 = m_base + cg * NC + c2;
+      __half* const y = pick(tensors.y);
 #pragma unroll
-      for (uint32_t c = 0; c < NC; c += 4) {
-        float v[4];
-        unpack2(acc[c / 2], v[0], v[1]);
-        unpack2(acc[c / 2 + 1], v[2], v[3]);
-        const uint32_t col = n_base + cg * NC + c;
-        if (vec) {
-          if (col >= n) break;
-          __half o[4];
-          uint2 raw = make_uint2(0, 0);
-          if (accumulate) raw = *reinterpret_cast<const uint2*>(dst + c);
-          const __half* old = reinterpret_cast<const __half*>(&raw);
+      for (uint32_t c = 0; c < NC / 8; c++) {
 #pragma unroll
-          for (int e = 0; e < 4; e++) o[e] = __float2half_rn(accumulate ? __fadd_rn(__half2float(old[e]), v[e]) : v[e]);
-          *reinterpret_cast<uint2*>(dst + c) = *reinterpret_cast<const uint2*>(o);
-        } else {
+        for (uint32_t e = 0; e < 2; e++) {
+          const uint32_t t = t0 + 8 * c + e;
+          __half* dst = y + static_cast<size_t>(t) * n + n_base + r0;
+          __half old[4];
 #pragma unroll
-          for (uint32_t e = 0; e < 4; e++)
-            if (col + e < n) dst[c + e] = __float2half_rn(accumulate ? __fadd_rn(__half2float(dst[c + e]), v[e]) : v[e]);
+          for (uint32_t r = 0; r < 4; r++)
+            if (accumulate && t < m && n_base + r0 + 8 * r < n) old[r] = dst[8 * r];
+#pragma unroll
+          for (uint32_t r = 0; r < 4; r++) {
+            float v[2];
+            unpack2(acc[c][r], v[0], v[1]);
+            if (t < m && n_base + r0 + 8 * r < n) dst[8 * r] = __float2half_rn(accumulate ? __fadd_rn(__half2float(old[r]), v[e]) : v[e]);
+          }
         }
       }
     }
@@ -417,22 +498,19 @@ __global__ void __launch_bounds__(TT_THREADS, 1) matmul_q1_tiled_kernel(const Ti
   tc_fence_before();
   __syncthreads();
   if (abort_s) {  // the workers have not seen the last MMAs complete
-    if (tid == 0) {  // (the thread that issued them)
+    if (warp == L::ISSUER && elect_one()) {  // (the thread that issued them)
       umma_commit(smem_u32(&drained));
       (void)mbar_wait(smem_u32(&drained), 0, TT_DRAIN);
     }
     __syncthreads();
   }
-  if (warp == 0) {
+  if (warp == L::ISSUER) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);
   }
 }
 
-template <uint32_t NC>
-constexpr uint32_t tt_smem() { return TT_STAGES * (2 * TT_PART + 4 * NC * 128) + 1024; }
-
-template <uint32_t NC>
+template <uint32_t N>
 cudaError_t launch_tiled(bool pdl, cudaStream_t s, const bp_q1_tensor* w, __half* const* y, uint32_t n_w, uint32_t m, const uint8_t* a_t,
                          const float* a_d, bool accumulate, uint32_t* err, uint32_t wait_limit) {
   static bool configured[64] = {};
@@ -441,7 +519,7 @@ cudaError_t launch_tiled(bool pdl, cudaStream_t s, const bp_q1_tensor* w, __half
   if (e != cudaSuccess) return e;
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
   if (!configured[dev]) {
-    e = cudaFuncSetAttribute(matmul_q1_tiled_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(tt_smem<NC>()));
+    e = cudaFuncSetAttribute(matmul_q1_tiled_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(TtLayout<N>::SMEM));
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
@@ -453,56 +531,64 @@ cudaError_t launch_tiled(bool pdl, cudaStream_t s, const bp_q1_tensor* w, __half
     t.w_qs[i] = w[j].qs;
     t.y[i] = y[j];
     t.n[i] = w[j].n;
-    if (i < n_w) tiles += (w[i].n + 4 * NC - 1) / (4 * NC);
+    if (i < n_w) tiles += (w[i].n + TT_M - 1) / TT_M;
     t.tile_end[i] = tiles;
   }
   // (a limit of a few polls is short in time too: the MMA issuer's polls for a copy suspend it for as many ns at most)
-  return bp_launch(pdl, matmul_q1_tiled_kernel<NC>, dim3(tiles, (m + TT_M - 1) / TT_M), dim3(TT_THREADS), tt_smem<NC>(), s, t, w[0].k, m, a_t, a_d,
+  return bp_launch(pdl, matmul_q1_tiled_kernel<N>, dim3(tiles, (m + N - 1) / N), dim3(TtLayout<N>::THREADS), TtLayout<N>::SMEM, s, t, w[0].k, m, a_t, a_d,
                    accumulate ? 1u : 0u, 1.0f, err, wait_limit, wait_limit < 2000u ? wait_limit : 2000u);
 }
 
 }  // namespace
 
-size_t bp_q1_tiled_bytes(uint32_t m, uint32_t k) { return static_cast<size_t>((m + TT_M - 1) / TT_M) * (k / 128u) * 2u * TT_PART; }
-size_t bp_q1_tiled_scales(uint32_t m, uint32_t k) { return static_cast<size_t>((m + TT_M - 1) / TT_M) * (k / 128u) * TT_M * 4u; }
+// (a tile may be partly filled: at most 127 rows of no token, whatever its width)
+size_t bp_q1_tiled_bytes(uint32_t m, uint32_t k) { return static_cast<size_t>(m + 127u) * k * 2u; }
+size_t bp_q1_tiled_scales(uint32_t m, uint32_t k) { return static_cast<size_t>(m + 127u) * (k / 32u); }
 
-cudaError_t bp_q1_quantize_tiled(bool pdl, cudaStream_t s, const __half* x, uint32_t k, uint32_t m, uint8_t* a_t, float* a_d) {
-  return bp_launch(pdl, quantize_tiled_kernel<SRC_PLAIN>, dim3(m), dim3(512), 0, s, x, x, k, 0.0f, a_t, a_d);
+cudaError_t bp_q1_quantize_tiled(bool pdl, cudaStream_t s, const __half* x, uint32_t k, uint32_t m, uint32_t n_tok, uint8_t* a_t, float* a_d) {
+  return bp_launch(pdl, quantize_tiled_kernel<SRC_PLAIN>, dim3(m), dim3(512), 0, s, x, x, k, 0.0f, n_tok, a_t, a_d);
 }
-cudaError_t bp_q1_rms_quantize_tiled(bool pdl, cudaStream_t s, const __half* x, const __half* w, float eps, uint32_t k, uint32_t m, uint8_t* a_t, float* a_d) {
-  return bp_launch(pdl, quantize_tiled_kernel<SRC_RMS>, dim3(m), dim3(512), 0, s, x, w, k, eps, a_t, a_d);
+cudaError_t bp_q1_rms_quantize_tiled(bool pdl, cudaStream_t s, const __half* x, const __half* w, float eps, uint32_t k, uint32_t m, uint32_t n_tok,
+                                     uint8_t* a_t, float* a_d) {
+  return bp_launch(pdl, quantize_tiled_kernel<SRC_RMS>, dim3(m), dim3(512), 0, s, x, w, k, eps, n_tok, a_t, a_d);
 }
-cudaError_t bp_q1_silu_quantize_tiled(bool pdl, cudaStream_t s, const __half* gate, const __half* up, uint32_t k, uint32_t m, uint8_t* a_t, float* a_d) {
-  return bp_launch(pdl, quantize_tiled_kernel<SRC_SILU>, dim3(m), dim3(512), 0, s, gate, up, k, 0.0f, a_t, a_d);
+cudaError_t bp_q1_silu_quantize_tiled(bool pdl, cudaStream_t s, const __half* gate, const __half* up, uint32_t k, uint32_t m, uint32_t n_tok,
+                                      uint8_t* a_t, float* a_d) {
+  return bp_launch(pdl, quantize_tiled_kernel<SRC_SILU>, dim3(m), dim3(512), 0, s, gate, up, k, 0.0f, n_tok, a_t, a_d);
 }
 
-cudaError_t bp_q1_matmul_tiled(bool pdl, cudaStream_t s, const bp_q1_tensor* w, __half* const* y, uint32_t n_w, uint32_t m, const uint8_t* a_t,
-                               const float* a_d, bool accumulate, uint32_t* err, uint32_t wait_limit) {
-  if (n_w == 0 || n_w > 3) return cudaErrorInvalidValue;
+uint32_t bp_q1_tile_tokens(const bp_q1_tensor* w, uint32_t n_w, uint32_t m) {
+  if (bp_q1_tile_width() != 0) return bp_q1_tile_width();
   const uint32_t sms = bp_q1_sm_count();
-  // The width of a tile: waves of one CTA per SM, times what a block of a tile of that width takes: us, 512 tokens through
-  // the 8B shape's tensors, 96 blocks (down) to 32 (Q/K/V): 2.11 - 2.28, 1.79 - 1.96, 1.58 - 1.71, 1.23 - 1.36, 1.14 - 1.21.
-  // The choice was the fastest of the five widths for Q/K/V, Wo, gate + up and down at 21, 128, 173, 300 and 512 tokens.
-  const uint32_t widths[5] = {32, 28, 24, 16, 8};
-  const float cost[5] = {2.15f, 1.79f, 1.66f, 1.34f, 1.17f};
+  // Waves of one CTA per SM, times what a block of a tile of that width takes: us, gate + up of 512 tokens at the 8B shape
+  // (96 blocks take 6 % less per block, 32 blocks in one wave up to 10 % more).
+  const uint32_t widths[6] = {128, 96, 64, 48, 32, 16};
+  const float cost[6] = {1.74f, 1.44f, 1.15f, 1.01f, 0.93f, 0.85f};
+  uint32_t tiles = 0;
+  for (uint32_t i = 0; i < n_w; i++) tiles += (w[i].n + TT_M - 1) / TT_M;
   float best = 1e30f;
-  uint32_t nc = 32;
-  for (int c = 0; c < 5; c++) {
-    uint32_t tiles = 0;
-    for (uint32_t i = 0; i < n_w; i++) tiles += (w[i].n + 4 * widths[c] - 1) / (4 * widths[c]);
-    const uint32_t ctas = tiles * ((m + TT_M - 1) / TT_M);
+  uint32_t n_tok = 128;
+  for (int c = 0; c < 6; c++) {
+    const uint32_t ctas = tiles * ((m + widths[c] - 1) / widths[c]);
     const float t = cost[c] * static_cast<float>((ctas + sms - 1) / sms);
     if (t < best) {
       best = t;
-      nc = widths[c];
+      n_tok = widths[c];
     }
   }
-  if (bp_q1_tile_width() != 0) nc = bp_q1_tile_width() / 4;
-  switch (nc) {
+  return n_tok;
+}
+
+cudaError_t bp_q1_matmul_tiled(bool pdl, cudaStream_t s, const bp_q1_tensor* w, __half* const* y, uint32_t n_w, uint32_t m, uint32_t n_tok,
+                               const uint8_t* a_t, const float* a_d, bool accumulate, uint32_t* err, uint32_t wait_limit) {
+  if (n_w == 0 || n_w > 3) return cudaErrorInvalidValue;
+  switch (n_tok) {
+    case 128: return launch_tiled<128>(pdl, s, w, y, n_w, m, a_t, a_d, accumulate, err, wait_limit);
+    case 96: return launch_tiled<96>(pdl, s, w, y, n_w, m, a_t, a_d, accumulate, err, wait_limit);
+    case 64: return launch_tiled<64>(pdl, s, w, y, n_w, m, a_t, a_d, accumulate, err, wait_limit);
+    case 48: return launch_tiled<48>(pdl, s, w, y, n_w, m, a_t, a_d, accumulate, err, wait_limit);
     case 32: return launch_tiled<32>(pdl, s, w, y, n_w, m, a_t, a_d, accumulate, err, wait_limit);
-    case 28: return launch_tiled<28>(pdl, s, w, y, n_w, m, a_t, a_d, accumulate, err, wait_limit);
-    case 24: return launch_tiled<24>(pdl, s, w, y, n_w, m, a_t, a_d, accumulate, err, wait_limit);
     case 16: return launch_tiled<16>(pdl, s, w, y, n_w, m, a_t, a_d, accumulate, err, wait_limit);
-    default: return launch_tiled<8>(pdl, s, w, y, n_w, m, a_t, a_d, accumulate, err, wait_limit);
+    default: return cudaErrorInvalidValue;
   }
 }

@@ -1693,8 +1693,8 @@ cudaError_t bp_q1_quantize_q8(bool pdl, cudaStream_t s, const __half* x, uint32_
 }
 
 // 0 = the default: a model's batches through the tiled product, untiled activations by alignment (op_variant); 1 dp4a,
-// 2 mma.sync, 3 tcgen05; 4 / 5 = mma.sync with 64- / 128-token tiles only; 6 .. 10 = as 0, the tiled product with 128,
-// 112, 96, 64, 32 weight rows per tile
+// 2 mma.sync, 3 tcgen05; 4 / 5 = mma.sync with 64- / 128-token tiles only; 6 .. 11 = as 0, the tiled product with 128,
+// 48, 96, 64, 32, 16 tokens per tile
 static uint32_t g_matmul_variant = 0;
 
 // The kernel for the untiled activations of bp_op_quantize_q8_0: mma.sync wherever its 16-byte reads of a_d and a_qs
@@ -1752,11 +1752,11 @@ static cudaError_t launch_mma(bool pdl, cudaStream_t s, const bp_q1_tensor* w, _
 
 bool bp_q1_matmul_is_tiled(uint32_t m) { return m != 0 && (g_matmul_variant >= 6 || g_matmul_variant == 0); }
 uint32_t bp_q1_tile_width() {
-  constexpr uint32_t W[5] = {128, 112, 96, 64, 32};
+  constexpr uint32_t W[6] = {128, 48, 96, 64, 32, 16};
   return g_matmul_variant >= 6 ? W[g_matmul_variant - 6] : 0;
 }
 
-void bp_q1_set_matmul_variant(uint32_t v) { g_matmul_variant = v <= 10 ? v : 0; }
+void bp_q1_set_matmul_variant(uint32_t v) { g_matmul_variant = v <= 11 ? v : 0; }
 
 cudaError_t bp_q1_take_error(uint32_t* code) {
   cudaError_t e = cudaMemcpyFromSymbol(code, g_q1_err, sizeof(uint32_t));

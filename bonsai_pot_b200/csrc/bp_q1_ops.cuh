@@ -39,13 +39,15 @@ cudaError_t bp_q1_matmul_multi(bool pdl, cudaStream_t s, const bp_q1_tensor* w, 
 // kernel reads (sizes in bytes / floats for a batch of m tokens, k inputs).
 bool bp_q1_matmul_is_tiled(uint32_t m);
 uint32_t bp_q1_tile_width();  // tuning aid: 0 = by the number of tiles
+// Tokens of a tile (n_tok below) for the product of these weights with a batch of m tokens.
+uint32_t bp_q1_tile_tokens(const bp_q1_tensor* w, uint32_t n_w, uint32_t m);
 size_t bp_q1_tiled_bytes(uint32_t m, uint32_t k);
 size_t bp_q1_tiled_scales(uint32_t m, uint32_t k);
-cudaError_t bp_q1_quantize_tiled(bool pdl, cudaStream_t s, const __half* x, uint32_t k, uint32_t m, uint8_t* a_t, float* a_d);
-cudaError_t bp_q1_rms_quantize_tiled(bool pdl, cudaStream_t s, const __half* x, const __half* w, float eps, uint32_t k, uint32_t m, uint8_t* a_t, float* a_d);
-cudaError_t bp_q1_silu_quantize_tiled(bool pdl, cudaStream_t s, const __half* gate, const __half* up, uint32_t k, uint32_t m, uint8_t* a_t, float* a_d);
-cudaError_t bp_q1_matmul_tiled(bool pdl, cudaStream_t s, const bp_q1_tensor* w, __half* const* y, uint32_t n_w, uint32_t m, const uint8_t* a_t,
-                               const float* a_d, bool accumulate, uint32_t* err, uint32_t wait_limit);
+cudaError_t bp_q1_quantize_tiled(bool pdl, cudaStream_t s, const __half* x, uint32_t k, uint32_t m, uint32_t n_tok, uint8_t* a_t, float* a_d);
+cudaError_t bp_q1_rms_quantize_tiled(bool pdl, cudaStream_t s, const __half* x, const __half* w, float eps, uint32_t k, uint32_t m, uint32_t n_tok, uint8_t* a_t, float* a_d);
+cudaError_t bp_q1_silu_quantize_tiled(bool pdl, cudaStream_t s, const __half* gate, const __half* up, uint32_t k, uint32_t m, uint32_t n_tok, uint8_t* a_t, float* a_d);
+cudaError_t bp_q1_matmul_tiled(bool pdl, cudaStream_t s, const bp_q1_tensor* w, __half* const* y, uint32_t n_w, uint32_t m, uint32_t n_tok,
+                               const uint8_t* a_t, const float* a_d, bool accumulate, uint32_t* err, uint32_t wait_limit);
 void bp_q1_set_matmul_variant(uint32_t variant);  // tuning aid, see bp_op_set_matmul_variant
 cudaError_t bp_q1_take_error(uint32_t* code);     // synchronous; 0 = no wait gave up since the last call
 cudaError_t bp_q1_topk(bool pdl, cudaStream_t s, const __half* logits, uint32_t n, uint32_t k, float* out_val, uint32_t* out_idx);

@@ -61,8 +61,8 @@ int bp_op_matmul_q1_0_q8_0(void* stream, const void* d, const void* qs, uint32_t
 /* Tuning aid of the matmul: 0 = the default: a model's batches through the tiled tcgen05 product, this entry point
  * through mma.sync (through the CUDA cores if a_d or a_qs is not 16-byte aligned), 1 = CUDA cores (dp4a), 2 =
  * mma.sync (int8; tiles of 128 tokens, of 64, or whole waves of the former and the rest as the latter, whichever fills
- * the device's waves best), 3 = tcgen05 (f16 operands), 4 / 5 = mma.sync with tiles of 64 / 128 tokens only, 6 .. 10 = as 0
- * with 128, 112, 96, 64, 32 weight rows per tile of the tiled product. Results do not depend on it. Process-wide. */
+ * the device's waves best), 3 = tcgen05 (f16 operands), 4 / 5 = mma.sync with tiles of 64 / 128 tokens only, 6 .. 11 = as 0
+ * with 128, 48, 96, 64, 32, 16 tokens per tile of the tiled product. Results do not depend on it. Process-wide. */
 void bp_op_set_matmul_variant(uint32_t variant);
 /* The tcgen05 matmul waits on barriers, with a bound. Synchronizes the device and returns BP_ERR_TIMEOUT
  * if such a wait of a bp_op_matmul_q1_0_q8_0 launch gave up since the last call (its output is then
