@@ -621,10 +621,26 @@ cudaError_t bp_prefill_init(bp_attn_ctx* c) {
   return allow(prefill_umma_kernel<2, 1, true>, PLayout<2, 1>::SMEM);
 }
 
+static bool prefill_on_tensor_cores(const bp_attn_ctx* c) {
+  return c->variant != 1 && c->have_pmaps && (c->qpg & (c->qpg - 1)) == 0 && c->qpg <= BM;
+}
+static cudaError_t launch_prefill_umma(bp_attn_ctx* c, cudaStream_t s, const __half* q, __half* out, uint32_t m, uint32_t* launches);
+
+cudaError_t bp_launch_prefill_layer(bp_attn_ctx* c, cudaStream_t s, uint32_t layer, __half* q, const __half* w_q, const __half* k,
+                                    const __half* v, const __half* w_k, __half* out, uint32_t m, uint32_t* launches) {
+  cudaError_t e;
+  if (prefill_on_tensor_cores(c)) {
+    e = bp_launch_prefill_rows(c, s, layer, q, w_q, k, v, w_k, m, (m + BN - 1) / BN * BN, launches);
+    return e != cudaSuccess ? e : launch_prefill_umma(c, s, q, out, m, launches);
+  }
+  e = bp_launch_q_norm_rope(c, s, q, w_q, 0, m, launches);
+  if (e == cudaSuccess) e = bp_launch_kv_writeback(c, s, layer, k, v, w_k, 0, m, launches);
+  return e != cudaSuccess ? e : bp_launch_prefill(c, s, layer, q, out, m, launches);
+}
+
 cudaError_t bp_launch_prefill(bp_attn_ctx* c, cudaStream_t s, uint32_t layer, const __half* q,
                               __half* out, uint32_t m, uint32_t* launches) {
-  const bool pow2 = (c->qpg & (c->qpg - 1)) == 0 && c->qpg <= BM;
-  if (c->variant == 1 || !c->have_pmaps || !pow2) {
+  if (!prefill_on_tensor_cores(c)) {
     if (c->n_ppx != 0) return cudaErrorNotSupported;  // the exchange lives in the tensor-core kernel's epilogue
     return bp_launch_scalar_attention(c, s, layer, q, out, m, m, true, launches);
   }
@@ -638,6 +654,11 @@ cudaError_t bp_launch_prefill(bp_attn_ctx* c, cudaStream_t s, uint32_t layer, co
     *launches += 1;
     if (e != cudaSuccess) return e;
   }
+  return launch_prefill_umma(c, s, q, out, m, launches);
+}
+
+// The attention over the batch's expanded rows.
+static cudaError_t launch_prefill_umma(bp_attn_ctx* c, cudaStream_t s, const __half* q, __half* out, uint32_t m, uint32_t* launches) {
   PrefillParams p;
   p.q = q;
   p.out = out;

@@ -198,6 +198,12 @@ cudaError_t bp_launch_decode(bp_attn_ctx* c, cudaStream_t s, uint32_t layer, con
                              __half* out, uint32_t cur_pos, uint32_t* launches);
 cudaError_t bp_launch_prefill(bp_attn_ctx* c, cudaStream_t s, uint32_t layer, const __half* q,
                               __half* out, uint32_t m, uint32_t* launches);
+// The three launches above for a batch at positions 0 .. m - 1 of a layer: q is normalised and rotated in place, the cache
+// rows are written, out gets the attention outputs.
+cudaError_t bp_launch_prefill_layer(bp_attn_ctx* c, cudaStream_t s, uint32_t layer, __half* q, const __half* w_q, const __half* k,
+                                    const __half* v, const __half* w_k, __half* out, uint32_t m, uint32_t* launches);
+cudaError_t bp_launch_prefill_rows(bp_attn_ctx* c, cudaStream_t s, uint32_t layer, __half* q, const __half* w_q, const __half* k,
+                                   const __half* v, const __half* w_k, uint32_t m, uint32_t rows_pad, uint32_t* launches);
 // Meeting of the ranks of the peer exchange on counter `slot` (< 64): signal all, wait (bounded) for all.
 cudaError_t bp_launch_peer_sync(bp_attn_ctx* c, cudaStream_t s, uint32_t slot);
 // Book-keeping of the rule above. A launch that wrote rows [row0, ...) of `layer`; a launch of

@@ -603,9 +603,7 @@ static int layer_host(bp_attn_ctx* c, uint32_t layer, const void* q, const void*
   if (int e = upload_norm_weights(c, st, wq, wk)) return e;
   uint32_t launches = 0;
   if (prefill) {
-    BP_CUDA(c, bp_launch_q_norm_rope(c, st, c->stage_q, c->stage_wq, pos_base, m, &launches));
-    BP_CUDA(c, bp_launch_kv_writeback(c, st, layer, c->stage_k, c->stage_v, c->stage_wk, pos_base, m, &launches));
-    BP_CUDA(c, bp_launch_prefill(c, st, layer, c->stage_q, c->stage_out, m, &launches));
+    BP_CUDA(c, bp_launch_prefill_layer(c, st, layer, c->stage_q, c->stage_wq, c->stage_k, c->stage_v, c->stage_wk, c->stage_out, m, &launches));
   } else if (c->variant == 0 && bp_use_umma(c)) {
     BP_CUDA(c, bp_launch_decode_fused(c, st, layer, c->stage_q, nullptr, c->stage_wq, c->stage_k, c->stage_v, c->stage_wk,
                                       pos_base, c->stage_out, &launches));

@@ -928,9 +928,7 @@ int bp_model_prefill_topk(bp_model* m, const uint32_t* tokens, uint32_t n, uint3
       __half* const out[3] = {m->q, m->k_cur, m->v_cur};
       if (int st = quantize_and_matmul(m, m->x, c.n_embd, n, w, out, 3, false, lt.attn_norm)) return st;
     }
-    M_CUDA(m, bp_launch_q_norm_rope(m->attn, s, m->q, lt.q_norm, 0, n, &launches));
-    M_CUDA(m, bp_launch_kv_writeback(m->attn, s, il, m->k_cur, m->v_cur, lt.k_norm, 0, n, &launches));
-    M_CUDA(m, bp_launch_prefill(m->attn, s, il, m->q, m->attn_out, n, &launches));
+    M_CUDA(m, bp_launch_prefill_layer(m->attn, s, il, m->q, lt.q_norm, m->k_cur, m->v_cur, lt.k_norm, m->attn_out, n, &launches));
     {
       __half* const out[1] = {m->x};
       if (int st = quantize_and_matmul(m, m->attn_out, c.q_dim, n, &lt.wo, out, 1, true)) return st;

@@ -101,5 +101,11 @@ __device__ __forceinline__ uint32_t quant4(const float* x, float* d_out) {
   return packed;
 }
 
+// What the write-back leaves of a quantised row for the attention of the same batch: int8 * FP32 scale, rounded once to
+// f16, clamped to the finite range.
+__device__ __forceinline__ __half2 expand2(uint32_t packed, int i, float scale) {  // values i, i + 1 of the word
+  const float a = static_cast<float>(static_cast<int8_t>(packed >> (8 * i))) * scale, b = static_cast<float>(static_cast<int8_t>(packed >> (8 * i + 8))) * scale;
+  return __floats2half2_rn(fminf(fmaxf(a, -65504.f), 65504.f), fminf(fmaxf(b, -65504.f), 65504.f));
+}
 
 }  // namespace bp

@@ -97,6 +97,72 @@ q_norm_rope_kernel(__half* __restrict__ q, const __half* __restrict__ w_q_norm,
   }
 }
 
+// Both of the above for a batch at positions 0 .. m - 1, and the f16 rows that its attention reads (prefill_expand_kernel,
+// bp_attn_prefill.cu) while the quantised ones are still in registers: three launches of a layer in one, no row read back.
+// Warps: RQ query heads of a token, then RK KV heads of a token, then the padding rows m .. rows_pad - 1, which are zero.
+template <int RQ, int RK>
+__global__ void __launch_bounds__(256)
+prefill_rows_kernel(__half* __restrict__ q, const __half* __restrict__ w_q_norm, const __half* __restrict__ k_cur,
+                    const __half* __restrict__ v_cur, const __half* __restrict__ w_k_norm, const __half* __restrict__ rope,
+                    float* __restrict__ k_d, uint32_t* __restrict__ k_qs, float* __restrict__ v_d, uint32_t* __restrict__ v_qs,
+                    __half* __restrict__ k16, __half* __restrict__ v16, uint32_t* counter, uint32_t n_head, uint32_t n_kv_head, uint32_t m,
+                    uint32_t rows_pad, float eps) {
+  bp::pdl_launch_dependents();
+  bp::pdl_wait();  // q, k_cur, v_cur come from the previous kernel; the cache and the f16 rows may still be read by earlier ones
+  if (blockIdx.x == 0 && threadIdx.x == 0) *counter = 0;
+  const int lane = threadIdx.x & 31;
+  uint32_t unit = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const uint32_t nq = m * (n_head / RQ), nk = m * (n_kv_head / RK), kv_dim = n_kv_head * BP_HEAD_DIM;
+  if (unit < nq) {
+    const uint32_t tok = unit / (n_head / RQ);
+    __half* row = q + static_cast<size_t>(unit) * RQ * BP_HEAD_DIM;
+    Rot4 qp[RQ];
+    norm_rope_rows<RQ>(row, BP_HEAD_DIM, w_q_norm, rope + static_cast<size_t>(tok) * BP_HEAD_DIM, eps, lane, qp);
+#pragma unroll
+    for (int r = 0; r < RQ; r++) {
+      uint2 o;
+      __half2 lo = __floats2half2_rn(qp[r].v[0], qp[r].v[1]), hi = __floats2half2_rn(qp[r].v[2], qp[r].v[3]);
+      o.x = *reinterpret_cast<uint32_t*>(&lo);
+      o.y = *reinterpret_cast<uint32_t*>(&hi);
+      *reinterpret_cast<uint2*>(row + r * BP_HEAD_DIM + 4 * lane) = o;
+    }
+    return;
+  }
+  unit -= nq;
+  if (unit < nk) {
+    const uint32_t tok = unit / (n_kv_head / RK), head0 = (unit % (n_kv_head / RK)) * RK;
+    const size_t at = static_cast<size_t>(tok) * kv_dim + head0 * BP_HEAD_DIM;
+    Rot4 kp[RK];
+    norm_rope_rows<RK>(k_cur + at, BP_HEAD_DIM, w_k_norm, rope + static_cast<size_t>(tok) * BP_HEAD_DIM, eps, lane, kp);
+#pragma unroll
+    for (int r = 0; r < RK; r++) {
+      const size_t e = at + r * BP_HEAD_DIM + 4 * lane;
+      const uint2 vr = *reinterpret_cast<const uint2*>(v_cur + e);
+      const __half2* vh = reinterpret_cast<const __half2*>(&vr);
+      const float2 v01 = __half22float2(vh[0]), v23 = __half22float2(vh[1]);
+      const float vraw[4] = {v01.x, v01.y, v23.x, v23.y};
+      float d[2];
+      const uint32_t p[2] = {quant4(kp[r].v, &d[0]), quant4(vraw, &d[1])};
+      k_qs[e / 4] = p[0];
+      v_qs[e / 4] = p[1];
+      if ((lane & 7) == 0) {
+        k_d[e / BP_QK8] = d[0];
+        v_d[e / BP_QK8] = d[1];
+      }
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        const __half2 lo = bp::expand2(p[i], 0, d[i]), hi = bp::expand2(p[i], 2, d[i]);
+        *reinterpret_cast<uint2*>((i ? v16 : k16) + e) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+      }
+    }
+    return;
+  }
+  unit -= nk;
+  const uint32_t zeros = (rows_pad - m) * kv_dim / 8u, z = unit * 32u + lane;  // 16-byte words of K, then of V
+  if (z < 2 * zeros)
+    *reinterpret_cast<uint4*>((z < zeros ? k16 : v16) + static_cast<size_t>(m) * kv_dim + 8u * (z < zeros ? z : z - zeros)) = make_uint4(0, 0, 0, 0);
+}
+
 template <int R>
 cudaError_t launch_q(bp_attn_ctx* c, cudaStream_t s, __half* q, const __half* w, uint32_t pos, uint32_t rows, uint32_t pos_step) {
   const uint32_t units = rows * (c->cfg.n_head / R);
@@ -147,4 +213,24 @@ cudaError_t bp_launch_kv_writeback(bp_attn_ctx* c, cudaStream_t s, uint32_t laye
   if (static_cast<uint64_t>(m) * c->cfg.n_kv_head >= 4096 && c->cfg.n_kv_head % 2 == 0)
     return launch_kv<2>(c, s, layer, k, v, w, pos_base, m);
   return launch_kv<1>(c, s, layer, k, v, w, pos_base, m);
+}
+
+cudaError_t bp_launch_prefill_rows(bp_attn_ctx* c, cudaStream_t s, uint32_t layer, __half* q, const __half* w_q, const __half* k,
+                                   const __half* v, const __half* w_k, uint32_t m, uint32_t rows_pad, uint32_t* launches) {
+  *launches += 1;
+  bp_note_row_write(c, layer, 0);
+  float* k_d = reinterpret_cast<float*>(c->kv[0] + bp_d_off(c, layer));
+  float* v_d = reinterpret_cast<float*>(c->kv[1] + bp_d_off(c, layer));
+  uint32_t* k_qs = reinterpret_cast<uint32_t*>(c->kv[0] + bp_qs_off(c, layer));
+  uint32_t* v_qs = reinterpret_cast<uint32_t*>(c->kv[1] + bp_qs_off(c, layer));
+  __half* v16 = c->pf_kv16 + static_cast<size_t>(c->pf_rows) * c->kv_dim;
+  auto launch = [&](auto kernel, uint32_t rq, uint32_t rk) {
+    const uint32_t zeros = 2 * ((rows_pad - m) * c->kv_dim / 8u);
+    const uint32_t units = m * (c->cfg.n_head / rq) + m * (c->cfg.n_kv_head / rk) + (zeros + 31) / 32;
+    return bp_launch(c->opt_pdl != 0, kernel, dim3((units + 7) / 8), dim3(256), 0, s, q, w_q, k, v, w_k, c->rope, k_d, k_qs, v_d, v_qs, c->pf_kv16, v16,
+                     c->pf_counter, c->cfg.n_head, c->cfg.n_kv_head, m, rows_pad, c->cfg.rms_eps);
+  };
+  // several heads per warp from the sizes on where the launches of their own take them
+  const bool big = static_cast<uint64_t>(m) * c->cfg.n_head >= 8192 && c->cfg.n_head % 4 == 0 && c->cfg.n_kv_head % 2 == 0;
+  return big ? launch(prefill_rows_kernel<4, 2>, 4, 2) : launch(prefill_rows_kernel<1, 1>, 1, 1);
 }

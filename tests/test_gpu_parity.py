@@ -487,6 +487,30 @@ def test_host_entry_points_equal_the_device_path():
         assert within_tolerance(out_p, exact)[0]
 
 
+@pytest.mark.parametrize("n_head,n_kv,m", [(4, 1, 1), (4, 1, 65), (32, 8, 63), (32, 8, 64), (32, 8, 255), (32, 8, 256), (32, 8, 513), (8, 2, 700)])
+def test_prefill_layer_as_two_launches_is_identical_to_the_separate_dispatches(n_head, n_kv, m):
+    """The host entry point's rows kernel (Q norm + RoPE, write-back and f16 rows in one launch; several heads per warp from
+    8192 rows of q on where the head counts allow) against the three dispatches: outputs and cache rows bit for bit. The
+    rows behind a longer batch come from an earlier one: the padding of a shorter batch has to be zeroed."""
+    sh = O.Shape(n_layer=2, max_seq=1024, n_head=n_head, n_kv_head=n_kv)
+    rng = np.random.default_rng(m)
+    w = [(1 + 0.3 * rng.standard_normal(128)).astype(np.float16) for _ in range(2)]
+    with make_ctx(sh) as a, make_ctx(sh) as b:
+        for n in (m + 60, m):
+            q, k, v = (rng.standard_normal((n, d)).astype(np.float16) for d in (sh.q_dim, sh.kv_dim, sh.kv_dim))
+            v[0, 0] = np.inf if n != m else 3.0  # (what an earlier batch left must not reach a masked key's product)
+            out = np.zeros((n, sh.q_dim), dtype=np.float16)
+            a.prefill_layer_host(1, q, k, v, w[0], w[1], n, out)
+            qd, od = dev(q), torch.zeros(n, sh.q_dim, dtype=torch.float16, device="cuda")
+            b.dispatch_q_norm_rope_fused(qd, dev(w[0]), 0, n)
+            b.dispatch_kv_writeback_fused(1, dev(k), dev(v), dev(w[1]), 0, n)
+            b.dispatch_attention(1, qd, od, n)
+            torch.cuda.synchronize()
+        assert np.array_equal(out.view(np.uint16), od.cpu().numpy().view(np.uint16)) and np.isfinite(out.astype(np.float32)).all()
+        for x, y in zip(read_cache(a, sh, 1, m), read_cache(b, sh, 1, m)):
+            assert np.array_equal(x[0].view(np.uint32), y[0].view(np.uint32)) and np.array_equal(x[1], y[1])
+
+
 def test_token_host_entry_point_equals_per_layer_calls():
     sh = O.Shape(n_layer=3, max_seq=512)
     rng_cases = [build_decode_case(sh, seed=10, cfg_id=1, layer=il, n_past=300) for il in range(3)]
