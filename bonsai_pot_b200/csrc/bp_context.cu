@@ -581,6 +581,30 @@ static int upload_norm_weights(bp_attn_ctx* c, cudaStream_t st, const void* wq, 
   return BP_OK;
 }
 
+// The address under which kernels reach `bytes` of pinned host memory, or null: pageable, in part not pinned, or not
+// aligned to the 8 bytes that the kernels read at a time.
+static void* pinned_view(const void* p, size_t bytes) {
+  typedef CUresult (*attribute_fn)(void*, CUpointer_attribute, CUdeviceptr);
+  static const attribute_fn attribute = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    const cudaError_t e = cudaGetDriverEntryPoint("cuPointerGetAttribute", &fn, cudaEnableDefault, &found);
+    return e == cudaSuccess && found == cudaDriverEntryPointSuccess ? reinterpret_cast<attribute_fn>(fn) : nullptr;
+  }();
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return nullptr;
+  }
+  if (attribute == nullptr || at.type != cudaMemoryTypeHost || at.devicePointer == nullptr || reinterpret_cast<uintptr_t>(at.devicePointer) % 8u != 0) return nullptr;
+  CUdeviceptr start = 0;  // the pinned range that holds the first byte has to hold them all
+  size_t size = 0;
+  const CUdeviceptr first = reinterpret_cast<CUdeviceptr>(at.devicePointer);
+  if (attribute(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, first) != CUDA_SUCCESS || attribute(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, first) != CUDA_SUCCESS)
+    return nullptr;
+  return first >= start && first - start <= size && bytes <= size - (first - start) ? at.devicePointer : nullptr;
+}
+
 static int layer_host(bp_attn_ctx* c, uint32_t layer, const void* q, const void* k, const void* v, const void* wq,
                       const void* wk, uint32_t pos_base, uint32_t m, bool prefill, void* out) {
   if (int s = enter(c)) return s;
@@ -703,6 +727,24 @@ int bp_decode_token_host(bp_attn_ctx* c, const void* q, const void* k, const voi
   if (int s = ensure_stage(c, nl)) return s;  // one staging row per layer
   cudaStream_t st = c->host_stream;
   const size_t qb = static_cast<size_t>(nl) * c->q_dim * 2, kb = static_cast<size_t>(nl) * c->kv_dim * 2;
+  const bool batched = c->opt_token_graph && bp_decode_layers_batched(c);
+  if (batched) {
+    // Pinned activations are read, and pinned outputs written, by the kernel itself: every CTA takes the kilobyte of its
+    // heads under its first cache rows' latency, where the copies came one after the other before and behind it.
+    const void *dq = pinned_view(q, qb), *dk = pinned_view(k, kb), *dv = pinned_view(v, kb);
+    void* res = pinned_view(out, qb);
+    if (dq && dk && dv && res) {
+      if (int e = upload_norm_weights(c, st, wq, wk)) return e;
+      uint32_t launches = 0;
+      BP_CUDA(c, bp_launch_decode_layers(c, st, static_cast<const __half*>(dq), static_cast<__half*>(res), pos + 1,
+                                         bp_fused_step{nullptr, c->stage_wq, c->stage_wk, static_cast<const __half*>(dk), static_cast<const __half*>(dv)},
+                                         &launches));
+      BP_CUDA(c, cudaStreamSynchronize(st));
+      c->last_launches = launches;
+      if (*c->err_host) return enter(c);  // latches BP_ERR_TIMEOUT
+      return BP_OK;
+    }
+  }
   BP_CUDA(c, cudaMemcpyAsync(c->stage_q, q, qb, cudaMemcpyHostToDevice, st));
   BP_CUDA(c, cudaMemcpyAsync(c->stage_k, k, kb, cudaMemcpyHostToDevice, st));
   BP_CUDA(c, cudaMemcpyAsync(c->stage_v, v, kb, cudaMemcpyHostToDevice, st));
@@ -710,7 +752,7 @@ int bp_decode_token_host(bp_attn_ctx* c, const void* q, const void* k, const voi
   uint32_t launches = 0;
   if (c->variant == 0 && bp_use_umma(c)) {
     // fused layer steps: the decode kernel normalises q and writes the new cache row itself
-    if (c->opt_token_graph && bp_decode_layers_batched(c)) {
+    if (batched) {
       BP_CUDA(c, bp_launch_decode_layers(c, st, c->stage_q, c->stage_out, pos + 1,
                                          bp_fused_step{nullptr, c->stage_wq, c->stage_wk, c->stage_k, c->stage_v}, &launches));
     } else if (c->opt_token_graph) {

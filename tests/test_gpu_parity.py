@@ -579,7 +579,7 @@ def test_token_host_over_all_layers_agrees_with_a_call_per_layer(n_layer, n_kv, 
     positions = [0, 1, 127, 128, 255, 256, 1290, 300, 1299]
     seq = [[rng.standard_normal(n_layer * d).astype(np.float16) for d in (sh.q_dim, sh.kv_dim, sh.kv_dim)] for _ in positions]
     results = []
-    for graph in (1, 0):
+    for graph, pinned in ((1, False), (1, True), (0, False)):  # pinned: the kernel reads and writes host memory itself
         with make_ctx(sh) as ctx:
             ctx.set_option("token_graph", graph)
             fill = np.random.default_rng(32)
@@ -590,17 +590,22 @@ def test_token_host_over_all_layers_agrees_with_a_call_per_layer(n_layer, n_kv, 
             outs = []
             for (q, k, v), pos in zip(seq, positions):
                 out = np.zeros((n_layer, sh.q_dim), dtype=np.float16)
+                if pinned:
+                    q, k, v, out = (torch.from_numpy(a).pin_memory().numpy() for a in (q, k, v, out))
                 ctx.decode_token_host(q, k, v, w, w, pos, out)
                 outs.append(out.astype(np.float32))
                 sms = torch.cuda.get_device_properties(0).multi_processor_count
                 assert ctx.last_launch_count() == (n_layer if not graph else launches) or sms != 148
             assert not ctx.status()
             results.append((outs, [read_cache(ctx, sh, il, 1300) for il in range(n_layer)]))
+    for got in results[:2]:
+        for a, b in zip(got[0], results[2][0]):
+            assert (np.abs(a - b) <= 1e-4 + 2.0 ** -10 * np.abs(b)).all()
+        for ra, rb in zip(got[1], results[2][1]):
+            for (da, qa), (db, qb) in zip(ra, rb):
+                assert np.array_equal(da.view(np.uint32), db.view(np.uint32)) and np.array_equal(qa, qb)
     for a, b in zip(results[0][0], results[1][0]):
-        assert (np.abs(a - b) <= 1e-4 + 2.0 ** -10 * np.abs(b)).all()
-    for ra, rb in zip(results[0][1], results[1][1]):
-        for (da, qa), (db, qb) in zip(ra, rb):
-            assert np.array_equal(da.view(np.uint32), db.view(np.uint32)) and np.array_equal(qa, qb)
+        assert np.array_equal(a, b)
 
 
 @pytest.mark.parametrize("warps,hpc", [(16, 8), (8, 4), (8, 2), (16, 1), (8, 1)])
