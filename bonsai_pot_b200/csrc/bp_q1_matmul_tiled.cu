@@ -17,7 +17,7 @@
 //   - the weights are the rows of a tile and the tokens its columns, so a batch pays for its tokens in steps of 16.
 //     (With the tokens on the 128 TMEM lanes and a tile of up to 128 weight rows a batch of 21 tokens paid for 128, one of
 //     173 for 256. A block of 128 inputs took a tile of 128 x 112 outputs 1.79 us with the staging in the worker warps; here
-//     128 x 128 outputs take 1.74, 128 x 64 1.15, 128 x 16 0.85.)
+//     128 x 128 outputs take 1.52, 128 x 64 0.92, 128 x 16 0.59; the three operations alone would take 0.83 of the 1.52.)
 #include <cuda_fp16.h>
 
 #include "bp_common.cuh"
@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(TtLayout<N>::THREADS, 1) matmul_q1_tiled_kerne
       mbar_init(smem_u32(&empty[i]), 1 + L::WORKERS);
     }
     for (uint32_t i = 0; i < BUFS; i++) {
-      mbar_init(smem_u32(&d_full[i]), 1);
+      mbar_init(smem_u32(&d_full[i]), 2);  // the MMAs, and the thread that issued them
       mbar_init(smem_u32(&d_empty[i]), L::WORKERS);
     }
     for (uint32_t i = 0; i < TT_RAWS; i++) {
@@ -258,9 +258,12 @@ __global__ void __launch_bounds__(TtLayout<N>::THREADS, 1) matmul_q1_tiled_kerne
   // its loop without waiting, copying or writing results. (The flag is a register: a look at abort_s before every wait
   // and every MMA lengthened the chain from hand-over to hand-over by 7 % of the kernel.)
   bool dead = false;
+  // A phase that is complete already is found by a plain test: the poll that may suspend its thread costs some 350 cycles here
+  // even then, several times per block (128 x 128 outputs: 1.75 us with it alone, 1.62 with the test first; 128 x 16: 0.84, 0.63).
   auto waitb = [&](uint64_t* bar, uint32_t parity, uint32_t ns = 2000u) {  // ns: how long a poll may suspend its thread
     if (dead) return;
     const uint32_t addr = smem_u32(bar);
+    if (mbar_test(addr, parity)) return;
     for (uint32_t i = 0; i < wait_limit; i++) {
       uint32_t ok;
       asm volatile(
@@ -304,6 +307,7 @@ __global__ void __launch_bounds__(TtLayout<N>::THREADS, 1) matmul_q1_tiled_kerne
             for (uint32_t part = 0; part < 2; part++)  // a sub-block: 32 bytes along the row
               umma_f8(tmem + (pb * G + g) * COLS, ad + (h * G + g) * 2u, bd + part * (N * 128u >> 4) + (h * G + g) * 2u, IDESC, part);
           umma_commit(smem_u32(&d_full[pb]));
+          mbar_arrive(smem_u32(&d_full[pb]));  // passes on what this thread has waited for, the scales among it
         }
         if (dead) break;  // no slot is given back any more: a copy into it could meet the previous one
         if (b + STAGES < nb1) umma_commit(smem_u32(&empty[slot]));  // (no arrival that nobody waits for: it could outlive the CTA)
@@ -415,18 +419,18 @@ __global__ void __launch_bounds__(TtLayout<N>::THREADS, 1) matmul_q1_tiled_kerne
     };
     for (uint32_t b = 0; b < nb1; b++) {
       const uint32_t slot = b % STAGES;
-      waitb(&a_full[slot], (b / STAGES) & 1u);
-      waitb(&full[slot], (b / STAGES) & 1u);
       const float* wd = reinterpret_cast<const float*>(smem_gen + L::OFF_WD + slot * L::WD) + r0;
       unsigned long long wd2[4];
-#pragma unroll
-      for (uint32_t r = 0; r < 4; r++) wd2[r] = pack2(wd[8 * r], wd[8 * r]);
       const float* ad_s = reinterpret_cast<const float*>(smem_gen + L::OFF_AD + slot * L::AD) + cg * NC + c2;
 #pragma unroll
       for (uint32_t h = 0; h < STEPS; h++) {
         const uint32_t j = b * STEPS + h, pb = j % BUFS;
         waitb(&d_full[pb], (j / BUFS) & 1u);
         tc_fence_after();
+        if (h == 0) {  // (the scales are there: the issuer has waited for them and arrived on d_full since. Waiting for them here took 0.1 us)
+#pragma unroll
+          for (uint32_t r = 0; r < 4; r++) wd2[r] = pack2(wd[8 * r], wd[8 * r]);
+        }
         // the pieces of the G sub-blocks, each load in flight while the previous piece is scaled and added
         auto load = [&](uint32_t q) {
           uint32_t* r = d[q & 1u];
@@ -561,9 +565,9 @@ uint32_t bp_q1_tile_tokens(const bp_q1_tensor* w, uint32_t n_w, uint32_t m) {
   if (bp_q1_tile_width() != 0) return bp_q1_tile_width();
   const uint32_t sms = bp_q1_sm_count();
   // Waves of one CTA per SM, times what a block of a tile of that width takes: us, gate + up of 512 tokens at the 8B shape
-  // (96 blocks take 6 % less per block, 32 blocks in one wave up to 10 % more).
+  // (96 blocks take 7 % less per block, 32 blocks in one wave up to 6 % more, of 16 tokens 20 %).
   const uint32_t widths[6] = {128, 96, 64, 48, 32, 16};
-  const float cost[6] = {1.74f, 1.44f, 1.15f, 1.01f, 0.93f, 0.85f};
+  const float cost[6] = {1.52f, 1.22f, 0.92f, 0.77f, 0.69f, 0.59f};
   uint32_t tiles = 0;
   for (uint32_t i = 0; i < n_w; i++) tiles += (w[i].n + TT_M - 1) / TT_M;
   float best = 1e30f;
