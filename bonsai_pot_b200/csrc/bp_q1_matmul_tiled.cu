@@ -17,7 +17,7 @@
 //   - the weights are the rows of a tile and the tokens its columns, so a batch pays for its tokens in steps of 16.
 //     (With the tokens on the 128 TMEM lanes and a tile of up to 128 weight rows a batch of 21 tokens paid for 128, one of
 //     173 for 256. A block of 128 inputs took a tile of 128 x 112 outputs 1.79 us with the staging in the worker warps; here
-//     128 x 128 outputs take 1.52, 128 x 64 0.92, 128 x 16 0.59; the three operations alone would take 0.83 of the 1.52.)
+//     128 x 128 outputs take 1.50, 128 x 64 0.90, 128 x 16 0.59; the three operations alone would take 0.83 of the 1.50.)
 #include <cuda_fp16.h>
 
 #include "bp_common.cuh"
@@ -412,6 +412,7 @@ __global__ void __launch_bounds__(TtLayout<N>::THREADS, 1) matmul_q1_tiled_kerne
     const unsigned long long ones = pack2(one, one);
     pdl_wait();
     uint32_t d[2][16];
+    bool there = false;  // the next hand-over, seen while this one was worked on
     // GC groups of 8 tokens from TMEM column `at` on: [row half][group][4]
     auto load_rows = [&](uint32_t at, auto gc, uint32_t* r) {
       tmem_ld_rows16<decltype(gc)::value>(at, r);
@@ -425,7 +426,7 @@ __global__ void __launch_bounds__(TtLayout<N>::THREADS, 1) matmul_q1_tiled_kerne
 #pragma unroll
       for (uint32_t h = 0; h < STEPS; h++) {
         const uint32_t j = b * STEPS + h, pb = j % BUFS;
-        waitb(&d_full[pb], (j / BUFS) & 1u);
+        if (!there) waitb(&d_full[pb], (j / BUFS) & 1u);
         tc_fence_after();
         if (h == 0) {  // (the scales are there: the issuer has waited for them and arrived on d_full since. Waiting for them here took 0.1 us)
 #pragma unroll
@@ -453,6 +454,8 @@ __global__ void __launch_bounds__(TtLayout<N>::THREADS, 1) matmul_q1_tiled_kerne
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&d_empty[pb]));
+            // (the answer comes while the last piece is worked on: 128 x 96 outputs 1.22 -> 1.18 us, 128 x 128 1.52 -> 1.50)
+            there = mbar_test(smem_u32(&d_full[(j + 1) % BUFS]), ((j + 1) / BUFS) & 1u);
           }
 #pragma unroll
           for (uint32_t i = 0; i < L::PS; i++) {
@@ -567,7 +570,7 @@ uint32_t bp_q1_tile_tokens(const bp_q1_tensor* w, uint32_t n_w, uint32_t m) {
   // Waves of one CTA per SM, times what a block of a tile of that width takes: us, gate + up of 512 tokens at the 8B shape
   // (96 blocks take 7 % less per block, 32 blocks in one wave up to 6 % more, of 16 tokens 20 %).
   const uint32_t widths[6] = {128, 96, 64, 48, 32, 16};
-  const float cost[6] = {1.52f, 1.22f, 0.92f, 0.77f, 0.69f, 0.59f};
+  const float cost[6] = {1.50f, 1.18f, 0.90f, 0.76f, 0.70f, 0.59f};
   uint32_t tiles = 0;
   for (uint32_t i = 0; i < n_w; i++) tiles += (w[i].n + TT_M - 1) / TT_M;
   float best = 1e30f;
