@@ -186,13 +186,13 @@ struct Num {  // a constant as an argument
   static constexpr uint32_t value = V;
 };
 
-template <uint32_t N_>
+template <uint32_t N_, uint32_t STAGERS_ = (N_ > 64 ? 2 : 4)>
 struct TtLayout {
   static constexpr uint32_t N = N_;
   // Worker warps: 4 quarters of the TMEM lanes x CG groups of NC tokens. Stager warps: as many as leave the workers
   // their registers (a scheduler's 16384 are shared by a quarter of the warps: up to 20 warps have 96 each).
   static constexpr uint32_t CG = N == 16 ? 2 : N == 48 ? 3 : 4, NC = N / CG, WORKERS = 4 * CG;
-  static constexpr uint32_t STAGERS = N > 64 ? 2 : 4;
+  static constexpr uint32_t STAGERS = STAGERS_;
   static constexpr uint32_t LOADER = WORKERS + STAGERS, ISSUER = LOADER + 1;  // the warps that request copies and issue MMAs
   static constexpr uint32_t THREADS = (ISSUER + 1) * 32;
   static constexpr uint32_t B = 2 * N * 128, AD = N * 16, WD = TT_M * 4;
@@ -209,11 +209,15 @@ struct TtLayout {
   static_assert(BUFS * G * COLS <= 512 && N % 16 == 0 && NC % 8 == 0 && SMEM <= 227 * 1024 - 1024, "limits of an SM");
 };
 
-template <uint32_t N>
-__global__ void __launch_bounds__(TtLayout<N>::THREADS, 1) matmul_q1_tiled_kernel(const TiledTensors tensors, uint32_t k, uint32_t m, const uint8_t* __restrict__ a_t,
-                                                                        const float* __restrict__ a_d, uint32_t accumulate, float one, uint32_t* err,
-                                                                        uint32_t wait_limit, uint32_t poll_ns) {
-  using L = TtLayout<N>;
+// The outputs of weight row tile `tile` and of the L::N tokens from number `first` on of token tile `m_tile`, which has NL
+// tokens in the activations (first = 0 when L::N = NL). Tensors is a value or a reference: which of them leaves the compiler
+// the better code differs (gate + up in tiles of 128: three whole waves 143 / 149 us, five and a cut one 274 / 267).
+template <class L, uint32_t NL, class Tensors>
+__device__ __forceinline__ void tiled_tile(Tensors tensors, uint32_t k, uint32_t m, const uint8_t* __restrict__ a_t,
+                                           const float* __restrict__ a_d, uint32_t accumulate, float one, uint32_t* err, uint32_t wait_limit,
+                                           uint32_t poll_ns, uint32_t tile, uint32_t m_tile, uint32_t first) {
+  static_assert(NL % L::N == 0, "part of a tile");
+  constexpr uint32_t N = L::N;
   constexpr uint32_t NC = L::NC, G = L::G, STEPS = L::STEPS, BUFS = L::BUFS, COLS = L::COLS, STAGES = L::STAGES;
   extern __shared__ uint8_t tt_raw[];
   __shared__ __align__(8) uint64_t full[STAGES], a_full[STAGES], empty[STAGES], d_full[BUFS], d_empty[BUFS], drained;
@@ -223,12 +227,11 @@ __global__ void __launch_bounds__(TtLayout<N>::THREADS, 1) matmul_q1_tiled_kerne
   const uint32_t smem_base = (smem_u32(tt_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = tt_raw + (smem_base - smem_u32(tt_raw));
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t tile = blockIdx.x;
   const uint32_t which = tile < tensors.tile_end[0] ? 0u : tile < tensors.tile_end[1] ? 1u : 2u;
   // (selects: an indexed parameter array would be copied to local memory)
   auto pick = [&](const auto* v) { return which == 0 ? v[0] : which == 1 ? v[1] : v[2]; };
   const uint32_t n = pick(tensors.n);
-  const uint32_t n_base = (tile - (which == 0 ? 0u : which == 1 ? tensors.tile_end[0] : tensors.tile_end[1])) * TT_M, m_base = blockIdx.y * N;
+  const uint32_t n_base = (tile - (which == 0 ? 0u : which == 1 ? tensors.tile_end[0] : tensors.tile_end[1])) * TT_M, m_base = m_tile * NL + first;
   const uint32_t nb1 = k / 128u;
   if (tid == 0) {
     for (uint32_t i = 0; i < STAGES; i++) {
@@ -318,8 +321,8 @@ __global__ void __launch_bounds__(TtLayout<N>::THREADS, 1) matmul_q1_tiled_kerne
     constexpr uint32_t RL = TT_M / 32;  // weight rows of a lane: lane, lane + 32, ..
     const uint8_t* w_qs = pick(tensors.w_qs);
     const __half* w_d = pick(tensors.w_d);
-    const uint8_t* a_src = a_t + static_cast<size_t>(blockIdx.y) * nb1 * L::B;
-    const float* ad_src = a_d + static_cast<size_t>(blockIdx.y) * nb1 * (4u * N);
+    const uint8_t* a_src = a_t + static_cast<size_t>(m_tile) * nb1 * (2u * NL * 128u) + first * 128u;
+    const float* ad_src = a_d + static_cast<size_t>(m_tile) * nb1 * (4u * NL) + first;
     uint32_t at[RL];  // the lane's rows (one beyond the tensor repeats the last: nobody reads its results)
 #pragma unroll
     for (uint32_t r = 0; r < RL; r++) at[r] = min(n_base + lane + 32u * r, n - 1u);
@@ -339,8 +342,15 @@ __global__ void __launch_bounds__(TtLayout<N>::THREADS, 1) matmul_q1_tiled_kerne
           if (b >= STAGES) waitb(&empty[slot], ((b / STAGES) - 1u) & 1u);
           if (lane == 0 && !dead) {
             mbar_arrive_expect_tx(smem_u32(&a_full[slot]), L::B + L::AD);
-            bulk_load(smem_base + slot * L::STAGE + TT_A, a_src + static_cast<size_t>(b) * L::B, L::B, smem_u32(&a_full[slot]));
-            bulk_load(smem_base + L::OFF_AD + slot * L::AD, ad_src + static_cast<size_t>(b) * (4u * N), L::AD, smem_u32(&a_full[slot]));
+            constexpr uint32_t PARTS = N == NL ? 1 : 2, SCALES = N == NL ? 1 : 4;  // (what lies together when the tile is whole)
+#pragma unroll
+            for (uint32_t c = 0; c < PARTS; c++)
+              bulk_load(smem_base + slot * L::STAGE + TT_A + c * (N * 128u), a_src + (static_cast<size_t>(b) * 2u + c) * (NL * 128u), L::B / PARTS,
+                        smem_u32(&a_full[slot]));
+#pragma unroll
+            for (uint32_t c = 0; c < SCALES; c++)
+              bulk_load(smem_base + L::OFF_AD + slot * L::AD + c * (N * 4u), ad_src + (static_cast<size_t>(b) * 4u + c) * NL, L::AD / SCALES,
+                        smem_u32(&a_full[slot]));
             copies = b + 1;
           }
           float* wd = reinterpret_cast<float*>(smem_gen + L::OFF_WD + slot * L::WD);
@@ -518,6 +528,41 @@ __global__ void __launch_bounds__(TtLayout<N>::THREADS, 1) matmul_q1_tiled_kerne
 }
 
 template <uint32_t N>
+__global__ void __launch_bounds__(TtLayout<N>::THREADS, 1) matmul_q1_tiled_kernel(const TiledTensors tensors, uint32_t k, uint32_t m, const uint8_t* __restrict__ a_t,
+                                                                        const float* __restrict__ a_d, uint32_t accumulate, float one, uint32_t* err,
+                                                                        uint32_t wait_limit, uint32_t poll_ns) {
+  tiled_tile<TtLayout<N>, N, const TiledTensors>(tensors, k, m, a_t, a_d, accumulate, one, err, wait_limit, poll_ns, blockIdx.x, blockIdx.y, 0);
+}
+
+// The same with the tiles of the last wave cut into tiles of NS tokens: `whole` CTAs have a tile of N, then come the narrow
+// ones. A last wave of few tiles leaves most SMs idle for as long as a full one takes: gate + up of 512 tokens at the 8B
+// shape (768 tiles = 5 waves of 148 and 28) 288 -> 267 us, of 128 tokens (148 and 44; tiles of 64 before) 91 -> 82.
+template <uint32_t N, uint32_t NS>
+__global__ void __launch_bounds__(TtLayout<N>::THREADS, 1) matmul_q1_tiled_cut_kernel(const TiledTensors tensors, uint32_t k, uint32_t m,
+                                                                        const uint8_t* __restrict__ a_t, const float* __restrict__ a_d,
+                                                                        uint32_t accumulate, float one, uint32_t* err, uint32_t wait_limit,
+                                                                        uint32_t poll_ns, uint32_t whole) {
+  using Small = TtLayout<NS, TtLayout<N>::STAGERS>;
+  static_assert(Small::THREADS == TtLayout<N>::THREADS, "the same warps");
+  const uint32_t tiles = tensors.tile_end[2];
+  if (blockIdx.x < whole) {
+    tiled_tile<TtLayout<N>, N, const TiledTensors&>(tensors, k, m, a_t, a_d, accumulate, one, err, wait_limit, poll_ns, blockIdx.x % tiles, blockIdx.x / tiles, 0);
+  } else {
+    const uint32_t i = blockIdx.x - whole, at = whole + i / (N / NS), first = i % (N / NS) * NS;
+    if (at / tiles * N + first < m)
+      tiled_tile<Small, N, const TiledTensors&>(tensors, k, m, a_t, a_d, accumulate, one, err, wait_limit, poll_ns, at % tiles, at / tiles, first);
+  }
+}
+
+// Tokens of the tiles into which the last wave is cut: as narrow as lets them all run at once; n_tok: it is not cut. (Less
+// than one wave is not: plain tiles of that width are up to 7 % faster.)
+uint32_t last_wave_tokens(uint32_t n_tok, uint32_t ctas, uint32_t sms) {
+  const uint32_t rest = ctas % sms;
+  if (n_tok != 128 || ctas < sms || rest == 0) return n_tok;
+  return rest * 4 <= sms ? 32 : rest * 2 <= sms ? 64 : 128;
+}
+
+template <uint32_t N, uint32_t NS = N>
 cudaError_t launch_tiled(bool pdl, cudaStream_t s, const bp_q1_tensor* w, __half* const* y, uint32_t n_w, uint32_t m, const uint8_t* a_t,
                          const float* a_d, bool accumulate, uint32_t* err, uint32_t wait_limit) {
   static bool configured[64] = {};
@@ -525,11 +570,6 @@ cudaError_t launch_tiled(bool pdl, cudaStream_t s, const bp_q1_tensor* w, __half
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  if (!configured[dev]) {
-    e = cudaFuncSetAttribute(matmul_q1_tiled_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(TtLayout<N>::SMEM));
-    if (e != cudaSuccess) return e;
-    configured[dev] = true;
-  }
   TiledTensors t;
   uint32_t tiles = 0;
   for (uint32_t i = 0; i < 3; i++) {
@@ -541,9 +581,32 @@ cudaError_t launch_tiled(bool pdl, cudaStream_t s, const bp_q1_tensor* w, __half
     if (i < n_w) tiles += (w[i].n + TT_M - 1) / TT_M;
     t.tile_end[i] = tiles;
   }
+  const uint32_t m_tiles = (m + N - 1) / N, ctas = tiles * m_tiles, sms = bp_q1_sm_count();
+  if constexpr (N == 128 && NS == N) {
+    const uint32_t last = last_wave_tokens(N, ctas, sms);
+    if (last == 32) return launch_tiled<N, 32>(pdl, s, w, y, n_w, m, a_t, a_d, accumulate, err, wait_limit);
+    if (last == 64) return launch_tiled<N, 64>(pdl, s, w, y, n_w, m, a_t, a_d, accumulate, err, wait_limit);
+  }
+  using L = TtLayout<N>;
+  constexpr uint32_t SMALL = TtLayout<NS, L::STAGERS>::SMEM, SMEM = L::SMEM > SMALL ? L::SMEM : SMALL;
+  const void* kernel;
+  if constexpr (NS == N) kernel = reinterpret_cast<const void*>(matmul_q1_tiled_kernel<N>);
+  else kernel = reinterpret_cast<const void*>(matmul_q1_tiled_cut_kernel<N, NS>);
+  if (!configured[dev]) {
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SMEM));
+    if (e != cudaSuccess) return e;
+    configured[dev] = true;
+  }
   // (a limit of a few polls is short in time too: the MMA issuer's polls for a copy suspend it for as many ns at most)
-  return bp_launch(pdl, matmul_q1_tiled_kernel<N>, dim3(tiles, (m + N - 1) / N), dim3(TtLayout<N>::THREADS), TtLayout<N>::SMEM, s, t, w[0].k, m, a_t, a_d,
-                   accumulate ? 1u : 0u, 1.0f, err, wait_limit, wait_limit < 2000u ? wait_limit : 2000u);
+  const uint32_t acc = accumulate ? 1u : 0u, poll_ns = wait_limit < 2000u ? wait_limit : 2000u;
+  if constexpr (NS == N) {
+    return bp_launch(pdl, matmul_q1_tiled_kernel<N>, dim3(tiles, m_tiles), dim3(L::THREADS), SMEM, s, t, w[0].k, m, a_t, a_d, acc, 1.0f, err, wait_limit,
+                     poll_ns);
+  } else {
+    const uint32_t rest = ctas % sms, whole = ctas - rest;
+    return bp_launch(pdl, matmul_q1_tiled_cut_kernel<N, NS>, dim3(whole + rest * (N / NS)), dim3(L::THREADS), SMEM, s, t, w[0].k, m, a_t, a_d, acc, 1.0f,
+                     err, wait_limit, poll_ns, whole);
+  }
 }
 
 }  // namespace
@@ -577,7 +640,8 @@ uint32_t bp_q1_tile_tokens(const bp_q1_tensor* w, uint32_t n_w, uint32_t m) {
   uint32_t n_tok = 128;
   for (int c = 0; c < 6; c++) {
     const uint32_t ctas = tiles * ((m + widths[c] - 1) / widths[c]);
-    const float t = cost[c] * static_cast<float>((ctas + sms - 1) / sms);
+    const uint32_t last = last_wave_tokens(widths[c], ctas, sms);
+    const float t = cost[c] * static_cast<float>(ctas / sms) + (ctas % sms == 0 ? 0.0f : last == widths[c] ? cost[c] : last == 64 ? cost[2] : cost[4]);
     if (t < best) {
       best = t;
       n_tok = widths[c];

@@ -601,6 +601,20 @@ def test_tiled_product_is_identical_to_the_cuda_core_product(tmp_path, m):
             assert np.array_equal(a.view(np.uint8), b.view(np.uint8)), variant
 
 
+@pytest.mark.parametrize("n_ff,m", [(9600, 1), (9600, 33), (9600, 128), (12288, 65), (12288, 100), (6400, 300), (6400, 257)])
+def test_last_wave_of_the_tiled_product_is_identical_in_narrow_tiles(tmp_path, n_ff, m):
+    """Tiles of 128 tokens whose last wave on 148 SMs is cut into tiles of 32 (150 = 148 + 2 and 300 = 2 x 148 + 4 of
+    them) and of 64 (192 = 148 + 44), some with few tokens and some with none: as the dp4a path's."""
+    d = str(tmp_path / "m")
+    model_dir.write_synthetic_model(d, shape=dict(RAGGED, n_embd=256, n_ff=n_ff), seed=12)
+    prompt = [(13 * i + 5) % 500 for i in range(m)]
+    rows = sorted({0, m // 2, m - 1})
+    want = prefill_rows(d, prompt, 1, rows)
+    for variant in (0, 6):
+        for a, b in zip(want, prefill_rows(d, prompt, variant, rows)):
+            assert np.array_equal(a.view(np.uint8), b.view(np.uint8)), variant
+
+
 def edit_tensors(path, change):
     """Calls change(name, dtype, parts) for every tensor of a model directory and writes the arrays back: parts is
     (values,) of an F16 tensor, (scales [n][blocks], signs [n][blocks][16]) of a Q1_0 tensor."""
