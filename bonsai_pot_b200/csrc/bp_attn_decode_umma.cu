@@ -1117,8 +1117,9 @@ cudaError_t bp_launch_decode_umma(bp_attn_ctx* c, cudaStream_t s, uint32_t layer
 // The fused steps of ALL layers as one launch or two, for activations that are all there before the first layer
 // (bp_decode_token_host): a call per layer is a chain of 36 kernels whose two ends, about 7 us, stream nothing; a launch
 // over the layers' (layer, KV head) pairs streams through them (36 layers at 4096 keys, call from and to pinned host
-// memory: 360 us as a chain in a graph, 122 here). Pairs that fill the device are not split at all; those that are left
-// over, or all of a small shard's, are split as far as every CTA is resident (the merge makes them wait for one another).
+// memory: 360 us as a chain in a graph, 122 here, 98 with the buffers used in place). Pairs that fill the device are not
+// split at all; those that are left over, or all of a small shard's, are split as far as every CTA is resident (the merge
+// makes them wait for one another).
 // Plain launches: the cache is settled, so every row is requested at once.
 bool bp_decode_layers_batched(const bp_attn_ctx* c) {
   return bp_use_umma(c) && c->opt_uhpc == 1 && c->n_px == 0 && c->opt_umerge && c->opt_exclusive &&
