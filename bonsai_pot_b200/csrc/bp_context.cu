@@ -605,6 +605,17 @@ static void* pinned_view(const void* p, size_t bytes) {
   return first >= start && first - start <= size && bytes <= size - (first - start) ? at.devicePointer : nullptr;
 }
 
+// Whether a kernel that reads q, k and v while others of its CTAs already store outputs may store them at `out`: a CTA has
+// read its heads' q by then, but nobody else's q and no layer's k and v. (Copies to the device come before any output.)
+static bool may_store_in_place(const void* out, const void* q, const void* k, const void* v, size_t qb, size_t kb) {
+  const uintptr_t o = reinterpret_cast<uintptr_t>(out);
+  auto apart = [&](const void* in, size_t bytes) {
+    const uintptr_t i = reinterpret_cast<uintptr_t>(in);
+    return o + qb <= i || i + bytes <= o;
+  };
+  return (out == q || apart(q, qb)) && apart(k, kb) && apart(v, kb);
+}
+
 static int layer_host(bp_attn_ctx* c, uint32_t layer, const void* q, const void* k, const void* v, const void* wq,
                       const void* wk, uint32_t pos_base, uint32_t m, bool prefill, void* out) {
   if (int s = enter(c)) return s;
@@ -733,7 +744,7 @@ int bp_decode_token_host(bp_attn_ctx* c, const void* q, const void* k, const voi
     // heads under its first cache rows' latency, where the copies came one after the other before and behind it.
     const void *dq = pinned_view(q, qb), *dk = pinned_view(k, kb), *dv = pinned_view(v, kb);
     void* res = pinned_view(out, qb);
-    if (dq && dk && dv && res) {
+    if (dq && dk && dv && res && may_store_in_place(out, q, k, v, qb, kb)) {
       if (int e = upload_norm_weights(c, st, wq, wk)) return e;
       uint32_t launches = 0;
       BP_CUDA(c, bp_launch_decode_layers(c, st, static_cast<const __half*>(dq), static_cast<__half*>(res), pos + 1,

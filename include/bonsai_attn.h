@@ -193,7 +193,9 @@ int bp_decode_step_host(bp_attn_ctx* ctx, uint32_t layer, const void* q_host, co
  * pairs and more the layers' steps run together in one launch or two: no layer reads
  * what another wrote. That splits a head's tokens otherwise than a call per layer, so
  * the outputs agree with it to rounding; the cache rows are the same bits. If all four
- * buffers are pinned and 8-byte aligned, the kernel then reads and writes them itself. */
+ * buffers are pinned and 8-byte aligned, the kernel then reads and writes them itself,
+ * at any time until the call returns. The buffers may overlap: an out_host that overlaps
+ * k_host, v_host or another part of q_host than its own is written by a copy behind the kernels. */
 int bp_decode_token_host(bp_attn_ctx* ctx, const void* q_host, const void* k_host, const void* v_host,
                          const void* w_q_norm_host, const void* w_k_norm_host, uint32_t pos,
                          void* out_host);

@@ -608,6 +608,48 @@ def test_token_host_over_all_layers_agrees_with_a_call_per_layer(n_layer, n_kv, 
         assert np.array_equal(a, b)
 
 
+def test_token_host_takes_any_pinned_buffers_to_the_same_bits():
+    """Where q, k, v and out lie must not matter, overlapping (288 pairs: the first CTAs store outputs before the last
+    have read their inputs), off the kernel's 8-byte reads, or pinned only in part: as from separate pageable buffers."""
+    sh = O.Shape(n_layer=36, max_seq=700, n_head=32, n_kv_head=8)
+    nq, nk, pos = sh.n_layer * sh.q_dim, sh.n_layer * sh.kv_dim, 699
+    rng = np.random.default_rng(41)
+    w = synth.ones_weight()
+    given = [rng.standard_normal(n).astype(np.float16) for n in (nq, nk, nk)]
+    arena = torch.zeros(3 * nq, dtype=torch.float16).pin_memory().numpy()
+    away = nq + 2 * nk  # where out is clear of q at 0, k at nq and v at nq + nk
+    places = {  # offsets of q, k, v and out in the arena
+        "in place": (0, nq, nq + nk, away), "out on q": (0, nq, nq + nk, 0), "out on k": (0, nq, nq + nk, nq), "out on v": (0, nq, nq + nk, nq + nk),
+        "out a layer behind q": (0, nq + sh.q_dim, nq + sh.q_dim + nk, sh.q_dim), "out a head before q": (128, nq + 128, nq + 128 + nk, 0),
+        "out ends in k": (nq + 2 * nk, nq - 128, nq + nk, 0), "q off by 2 bytes": (1, nq + 4, nq + 4 + nk, away + 8),
+        "v off by 4 bytes": (0, nq, nq + nk + 2, away + 8), "out off by 6 bytes": (0, nq, nq + nk, away + 3)}
+    with make_ctx(sh) as ctx:
+        for il in range(sh.n_layer):
+            for kind in range(2):
+                ctx.kv_import(kind, il, 0, 700, (rng.random((700, sh.nb), dtype=np.float32) * 0.05 + 0.001))
+                ctx.kv_import(kind, il, 1, 700, rng.integers(-127, 128, (700, sh.kv_dim), dtype=np.int8))
+
+        def token(bufs, out):
+            for b, x in zip(bufs, given):
+                b[:] = x
+            ctx.decode_token_host(*bufs, w, w, pos, out)
+            return out.copy(), [[(d[pos], q[pos]) for d, q in read_cache(ctx, sh, il, 700)] for il in (0, 17, 35)]
+
+        want, rows = token([np.empty(n, np.float16) for n in (nq, nk, nk)], np.empty(nq, np.float16))
+        got = {name: token([arena[o:o + n] for o, n in zip(at, (nq, nk, nk))], arena[at[3]:at[3] + nq]) for name, at in places.items()}
+        for i in range(4):  # one of the four pageable
+            bufs = [np.empty(n, np.float16) if i == j else arena[o:o + n] for j, (o, n) in enumerate(zip(places["in place"], (nq, nk, nk, nq)))]
+            got["buffer %d pageable" % i] = token(bufs[:3], bufs[3])
+        wrong = []
+        for name, (out, fresh) in got.items():
+            same = np.array_equal(out.view(np.uint16), want.view(np.uint16))
+            for a, b in zip(fresh, rows):
+                for (da, qa), (db, qb) in zip(a, b):
+                    same &= np.array_equal(da.view(np.uint32), db.view(np.uint32)) and np.array_equal(qa, qb)
+            wrong += [] if same else [name]
+        assert not wrong
+
+
 @pytest.mark.parametrize("warps,hpc", [(16, 8), (8, 4), (8, 2), (16, 1), (8, 1)])
 def test_decode_tuning_options_do_not_change_results(warps, hpc):
     sh = O.Shape(n_layer=2, max_seq=4096)
