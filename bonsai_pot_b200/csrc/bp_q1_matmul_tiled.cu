@@ -382,8 +382,11 @@ __device__ __forceinline__ void tiled_tile(Tensors tensors, uint32_t k, uint32_t
     // turn, but none is ever two uses behind: a stager at block b has seen block b - STAGERS - STAGES released, and
     // stages are released in order.)
     static_assert(L::STAGERS <= STAGES && TT_RAWS % L::STAGERS == 0, "phases that a stager has to follow");
+    constexpr uint32_t AHEAD = STAGES < TT_RAWS ? STAGES : TT_RAWS;  // blocks that need nothing of the kernel before this one
     for (uint32_t b = warp - L::WORKERS; b < nb1; b += L::STAGERS) {
       const uint32_t slot = b % STAGES, rs = b % TT_RAWS;
+      // Further signs are requested, and stages given back, only behind that kernel: the polls count from its end.
+      if (b >= AHEAD && b < AHEAD + L::STAGERS) pdl_wait();
       waitb(&raw_full[rs], (b / TT_RAWS) & 1u);
       uint4 sign[4];
 #pragma unroll

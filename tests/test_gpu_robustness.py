@@ -304,6 +304,22 @@ def test_batched_product_whose_wait_runs_out_winds_down_and_latches(tmp_path, m)
         assert np.array_equal(a.view(np.uint16), b.view(np.uint16))
 
 
+def test_batched_product_does_not_count_the_time_of_the_kernels_before_it(tmp_path):
+    """The second layer's Q/K/V product (16 blocks, more than its stages) starts under the first layer's down product of 768
+    blocks, some 450 us. A limit of 48 polls, some 4 us each, is ample for what the product itself waits for (8 polls are
+    enough) and too short for that (96 were): no warp may begin to count before the dependency wait."""
+    d = str(tmp_path / "m")
+    model_dir.write_synthetic_model(d, shape=dict(n_layer=2, n_embd=2048, n_ff=98304, n_head=4, n_kv_head=1, head_dim=128, n_vocab=512), seed=6)
+    prompt = [(11 * i + 1) % 500 for i in range(16)]
+    with bp.Model(d, max_seq=64) as gm:
+        gm.prefill_topk(prompt)
+        want = gm.logits()
+        gm.attention().set_option("matmul_wait_limit", 48)
+        for _ in range(5):
+            gm.prefill_topk(prompt)
+            assert np.array_equal(gm.logits().view(np.uint16), want.view(np.uint16))
+
+
 @pytest.mark.parametrize("ring", [0, 0x33, 0x35, 0x53, 0x24])
 def test_rings_of_any_size_give_the_same_bits_at_every_repetition(ring):
     """Splits of 14 stages through rings of odd and even sizes, the loads of 144 CTAs competing for memory: a wait that
