@@ -115,6 +115,21 @@ struct ULayout {
   static constexpr uint32_t total(uint32_t nk, uint32_t nv) { return ring(nk, nv) + tail() + 1024; }
 };
 
+// Where an issuer stands in the two turns of a ring (see bar2). Counted along: divisions by the ring's size, which is not a
+// constant, stood before every wait of a job (us per layer, 36 layers: 4096 keys 8.53 -> 8.34, 200 keys 6.50 -> 6.19, 32768
+// keys 18.12 -> 17.69).
+struct Turn {
+  uint32_t i, phase;  // use mod twice the ring, and the phase of that barrier
+  __device__ __forceinline__ void step(uint32_t by, uint32_t ring) {  // by <= 2 ring
+    i += by;
+    if (i >= 2 * ring) {
+      i -= 2 * ring;
+      phase ^= 1u;
+    }
+  }
+  __device__ __forceinline__ uint32_t slot(uint32_t ring) const { return i < ring ? i : i - ring; }
+};
+
 struct Misc {            // small shared state, lives in the MISC_B region
   float sq[8][4][4];     // Q block scales [head][query head][block] (pre-multiplied by the softmax scale)
   int xchg[NGRP][2][4][8];  // [softmax group][job parity][warp]: 4 score maxima, 4 V-scale maxima
@@ -368,8 +383,8 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
   // chosen by the job modulo twice the ring every use that completes it is waited for by the same issuer, in order.
   auto bar2 = [](uint64_t* bars, uint32_t i, uint32_t ring) { return bars + i % (2 * ring); };
   auto phase2 = [](uint32_t i, uint32_t ring) { return (i / (2 * ring)) & 1u; };
-  auto issue_stage = [&](uint32_t it, uint32_t s) {
-    const uint32_t bar = smem_u32(bar2(full_bar, it, ns));
+  auto issue_stage = [&](uint32_t it, uint32_t s, uint64_t* full) {
+    const uint32_t bar = smem_u32(full);
     const uint32_t stage = smem_base + s * L::KSTAGE_B;
     const int row = static_cast<int>(row0 + tok_begin + it * UT);
     // Older rows were written by launches that have long completed; rows from fresh_from on (the
@@ -385,8 +400,8 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
   const bool new_row = p.fused && tok_end == p.cur_pos;  // this CTA's last stage holds the new token's row
   // The V tile of job j (stage j / HPC, head j % HPC) into V slot j % nv. The new row's tiles complete a barrier of
   // their own: who patches the row in has not followed the slot's phases, and one phase looks like the next but one.
-  auto issue_v = [&](uint32_t j) {
-    const uint32_t v = j % nv, bar = smem_u32(new_row && j / HPC == n_iter - 1 ? &v_last : bar2(v_full, j, nv));
+  auto issue_v = [&](uint32_t j, uint32_t v, uint64_t* full) {
+    const uint32_t bar = smem_u32(new_row && j / HPC == n_iter - 1 ? &v_last : full);
     const int row = static_cast<int>(row0 + tok_begin + (j / HPC) * UT);
     mbar_arrive_expect_tx(bar, L::VSLOT_B);
     tma_load_3d(v_ring + v * L::VSLOT_B, &map_vq, bar, 0, static_cast<int>(g0 + j % HPC), row);
@@ -405,7 +420,7 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
     prefetch_tensormap(&map_kq);
     prefetch_tensormap(&map_kd);
     prefetch_tensormap(&map_vd);
-    issue_stage(0, 0);
+    issue_stage(0, 0, full_bar);
     prefetch_tensormap(&map_vq);
   } else if (warp == 3) {
     if (lane >= 1 && lane < 2 * U_MAX_STAGES) mbar_init(smem_u32(&full_bar[lane]), 1);
@@ -536,10 +551,10 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
     if (lane == 0) {
       // the rest of the first round (stage 0 was requested during set-up)
       const uint32_t n_pre = n_iter < ns ? n_iter : ns;
-      for (uint32_t it = 1; it < n_pre; it++) issue_stage(it, it);
+      for (uint32_t it = 1; it < n_pre; it++) issue_stage(it, it, full_bar + it);
       // a launch whose V tiles all fit at once requests them here too (it should not wait for them);
       // otherwise the Q K^T issuers request every V tile when its job starts
-      for (uint32_t j = 0; j < v_pre; j++) issue_v(j);
+      for (uint32_t j = 0; j < v_pre; j++) issue_v(j, j, v_full + j);
     }
     __syncwarp();
     // Fused step, last split: the whole warp first quantises the new token's K / V rows of this
@@ -575,7 +590,7 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
       for (uint32_t it = ns; it < n_iter; it++) {
         wait(&k_empty[s], (use - 1) & 1);
         if (abort_s) break;
-        issue_stage(it, s);
+        issue_stage(it, s, full_bar + s + (use & 1u) * ns);
         if (++s == ns) { s = 0; use++; }
       }
     }
@@ -636,10 +651,11 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
       constexpr uint32_t IDESC_QK = umma_idesc(2, 1, 1, 0, 0, 128, 16);  // s32 = s8 (K-major) x s8
       const uint64_t dbase = umma_desc_sw128(0, 16, 1024);               // + (shared address >> 4)
       const uint32_t q = warp - 1;
+      Turn at_k = {q / HPC, 0}, at_v = {q, 0};
       wait(&q_bar, 0);
-      for (uint32_t j = q; j < n_jobs; j += NISS) {
-        const uint32_t it = j / HPC, g = j % HPC, bi = j % NGRP, k = j / NGRP, s = it % ns;
-        wait(bar2(full_bar, it, ns), phase2(it, ns));
+      for (uint32_t j = q; j < n_jobs; j += NISS, at_k.step(NISS / HPC, ns), at_v.step(NISS, nv)) {
+        const uint32_t it = j / HPC, g = j % HPC, bi = j % NGRP, k = j / NGRP, s = at_k.slot(ns);
+        wait(full_bar + at_k.i, at_k.phase);
         if (new_row && it == n_iter - 1) wait(&patched_bar, 0);  // the new row is in place
         if (k > 0) wait(&s_free[bi], (k - 1) & 1);
         tc_fence_after();
@@ -651,8 +667,8 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
         // Now request the job's V tile (unless set-up did): it arrives while the softmax group works,
         // and its slot is occupied for one load latency instead of the load latency plus the whole job.
         if (j >= v_pre) {
-          if (j >= nv) wait(bar2(v_empty, j - nv, nv), phase2(j - nv, nv));
-          if (!abort_s) issue_v(j);
+          if (j >= nv) wait(v_empty + (at_v.i < nv ? at_v.i + nv : at_v.i - nv), at_v.i < nv ? at_v.phase ^ 1u : at_v.phase);
+          if (!abort_s) issue_v(j, at_v.slot(nv), v_full + at_v.i);
         }
       }
     }
@@ -665,13 +681,14 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
       constexpr uint32_t IDESC_PV = umma_idesc(2, 1, 0, 1, 0, 128, 64);  // s32 += s8 (MN-major) x u8
       const uint64_t dbase = umma_desc_sw128(0, 16, 1024);
       const uint32_t q = warp - 1 - NISS;
-      for (uint32_t j = q; j < n_jobs; j += NISS) {
+      Turn at_v = {q, 0};
+      for (uint32_t j = q; j < n_jobs; j += NISS, at_v.step(NISS, nv)) {
         const uint32_t it = j / HPC, bi = j % NGRP, k = j / NGRP;
-        const uint32_t v = j % nv;
+        const uint32_t v = at_v.slot(nv);
         if (new_row && it == n_iter - 1) {
           wait(&patched_v, 0);  // the tile is there and the new row in it
         } else {
-          wait(bar2(v_full, j, nv), phase2(j, nv));
+          wait(v_full + at_v.i, at_v.phase);
         }
         wait(&p_ready[bi], k & 1);
         if (k > 0) wait(&o_free[bi], (k - 1) & 1);
@@ -683,7 +700,7 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
           umma_i8(tmem + NGRP * 64 + bi * 64, va + kk * (32 * 128 >> 4), pb + 2 * kk, IDESC_PV, kk);
         umma_commit(smem_u32(&o_ready[bi]));
         umma_commit(smem_u32(&p_free[bi]));
-        umma_commit(smem_u32(bar2(v_empty, j, nv)));  // the V slot is free once this P V has run
+        umma_commit(smem_u32(v_empty + at_v.i));  // the V slot is free once this P V has run
       }
     }
   }

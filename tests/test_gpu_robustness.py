@@ -350,3 +350,35 @@ def test_rings_of_any_size_give_the_same_bits_at_every_repetition(ring):
                 assert torch.equal(token(pos).view(torch.int16), ref.view(torch.int16))
         torch.cuda.synchronize()
         assert not ctx.status()
+
+
+@pytest.mark.parametrize("ring", [0x12, 0x13, 0x23, 0x25, 0x33])
+def test_rings_of_any_size_give_the_same_bits_with_two_heads_per_cta(ring):
+    """The same with both heads of a stage in one CTA: an issuer then steps through the K ring one stage at a time and
+    through the V ring two slots at a time, in the smallest rings from turn to turn with every job. 9 stages per split."""
+    n_layer, ctx_len, pos = 2, 42000, 41999
+    with bp.AttnContext(n_layer=n_layer, max_seq=ctx_len) as ctx:
+        g = torch.Generator(device="cuda").manual_seed(6)
+        w = torch.ones(128, dtype=torch.float16, device="cuda")
+        rand = lambda *shape: torch.randn(*shape, generator=g, device="cuda").half()
+        for il in range(n_layer):
+            for r0 in range(0, ctx_len, 8400):
+                ctx.dispatch_kv_writeback_fused(il, rand(8400, ctx.kv_dim), rand(8400, ctx.kv_dim), w, r0, 8400)
+        q, k, v = rand(n_layer, ctx.q_dim), rand(n_layer, ctx.kv_dim), rand(n_layer, ctx.kv_dim)
+        ctx.set_option("decode_umma_heads_per_cta", 2)
+
+        def token(at):
+            out = torch.zeros(n_layer, ctx.q_dim, dtype=torch.float16, device="cuda")
+            for il in range(n_layer):
+                ctx.decode_layer(il, q[il], w, k[il], v[il], w, at, out[il])
+            return out
+
+        for at in (pos - 200, pos):  # (a token writes its row)
+            token(at)
+        want = [token(at) for at in (pos, pos - 200)]
+        ctx.set_option("decode_ring", ring)
+        for _ in range(10):
+            for at, ref in zip((pos, pos - 200), want):
+                assert torch.equal(token(at).view(torch.int16), ref.view(torch.int16))
+        torch.cuda.synchronize()
+        assert not ctx.status()
