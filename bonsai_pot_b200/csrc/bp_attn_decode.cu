@@ -347,6 +347,7 @@ decode_mma_kernel(const __grid_constant__ CUtensorMap map_kq, const __grid_const
     fence_barrier_init();
   }
   __syncthreads();
+  uint32_t requested = 0;  // producer: stages
 
   if (warp == NW_) {
     // ---------------- producer ----------------
@@ -370,6 +371,7 @@ decode_mma_kernel(const __grid_constant__ CUtensorMap map_kq, const __grid_const
         tma_load_2d(stage + 2 * G::STAGE_QS + G::STAGE_D, &map_vd, bar, static_cast<int>(g0 * 16), row);
         for (uint32_t g = 0; g < hpc; g++)
           tma_load_3d(stage + G::STAGE_QS + g * (st_tok * 128), &map_vq, bar, 0, static_cast<int>(g0 + g), row);
+        requested = it + 1;
       }
       if (!ok) atomicExch(p.err, 1u);
     }
@@ -520,9 +522,9 @@ decode_mma_kernel(const __grid_constant__ CUtensorMap map_kq, const __grid_const
   // The producer drains its own copies before the CTA retires (all of them have
   // already completed unless a wait above gave up).
   if (warp == NW_ && lane == 0) {
-    const uint32_t first = n_iter > ns ? n_iter - ns : 0;
-    for (uint32_t it = first; it < n_iter; it++)
-      if (!mbar_wait(smem_u32(&full_bar[it % ns]), (it / ns) & 1, 1u << 20)) atomicExch(p.err, 2u);
+    const uint32_t first = requested > ns ? requested - ns : 0;
+    for (uint32_t it = first; it < requested; it++)
+      if (!mbar_wait(smem_u32(&full_bar[it % ns]), (it / ns) & 1, DRAIN_LIMIT)) atomicExch(p.err, 2u);
   }
 }
 

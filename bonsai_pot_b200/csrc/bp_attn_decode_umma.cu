@@ -160,6 +160,33 @@ __device__ __noinline__ void cta_wait(uint64_t* bar, uint32_t parity, volatile u
   }
 }
 
+// The end of a CTA whose waits gave up: its MMAs are complete and its copies have landed when it returns. All threads.
+__device__ __noinline__ void wind_down(bool issuer, uint64_t* drained, uint64_t* full_bar, uint32_t k_end, uint32_t ns, uint64_t* v_full,
+                                       const volatile uint32_t* v_end, uint32_t nv, uint32_t v_pre, uint32_t fresh, uint32_t n_jobs, uint64_t* v_last) {
+  if (threadIdx.x == 0) {
+    mbar_init(smem_u32(drained), 2 * NISS);
+    fence_barrier_init();
+  }
+  __syncthreads();
+  if (issuer && elect_one()) umma_commit(smem_u32(drained));  // (the threads that issued them)
+  if (threadIdx.x == 0) {
+    auto drain = [&](uint64_t* bar, uint32_t parity) { (void)mbar_wait(smem_u32(bar), parity, DRAIN_LIMIT); };
+    drain(drained, 0);
+    // The last load of each barrier: the one before it had landed when its stage or slot was given back.
+    for (uint32_t it = k_end > 2 * ns ? k_end - 2 * ns : 0; it < k_end; it++) drain(full_bar + it % (2 * ns), (it / (2 * ns)) & 1u);
+    auto requested = [&](uint32_t j) { return j < v_pre || j < v_end[j % NISS]; };
+    for (uint32_t x = 0; x < 2 * nv; x++) {
+      uint32_t uses = 0;
+      for (uint32_t j = x; j < fresh && requested(j); j += 2 * nv) uses++;
+      if (uses != 0) drain(v_full + x, (uses - 1) & 1u);
+    }
+    for (uint32_t j = fresh; j < n_jobs; j++)
+      if (!requested(j)) mbar_arrive(smem_u32(v_last));  // in place of a load that never was
+    if (fresh < n_jobs) drain(v_last, 0);
+  }
+  __syncthreads();
+}
+
 // One final output element: to this rank's output and, with a peer exchange, to every rank's gathered buffer.
 __device__ __forceinline__ void put_out(const UmmaParams& p, uint32_t h, uint32_t d, float v) {
   const __half hv = __float2half_rn(v);
@@ -340,9 +367,10 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[2 * U_MAX_STAGES], k_empty[U_MAX_STAGES], v_full[2 * U_MAX_STAGES], v_empty[2 * U_MAX_STAGES];
   __shared__ __align__(8) uint64_t s_ready[4], s_free[4], p_ready[4], p_free[4], o_ready[4], o_free[4];
-  __shared__ __align__(8) uint64_t q_bar, patched_bar, patched_v, v_last;
+  __shared__ __align__(8) uint64_t q_bar, patched_bar, patched_v, v_last, drained;
   __shared__ uint32_t tmem_base_s;
   __shared__ volatile uint32_t abort_s;
+  __shared__ volatile uint32_t k_end_s, v_end_s[NISS];  // stages, and an issuer's V tiles, are requested up to here
 
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -586,13 +614,14 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
       }
     }
     if (lane == 0) {
-      uint32_t s = 0, use = 1;
-      for (uint32_t it = ns; it < n_iter; it++) {
+      uint32_t s = 0, use = 1, it = n_iter < ns ? n_iter : ns;
+      for (; it < n_iter; it++) {
         wait(&k_empty[s], (use - 1) & 1);
         if (abort_s) break;
         issue_stage(it, s, full_bar + s + (use & 1u) * ns);
         if (++s == ns) { s = 0; use++; }
       }
+      k_end_s = it;
     }
     __syncwarp();
     if (new_row) {
@@ -653,7 +682,8 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
       const uint32_t q = warp - 1;
       Turn at_k = {q / HPC, 0}, at_v = {q, 0};
       wait(&q_bar, 0);
-      for (uint32_t j = q; j < n_jobs; j += NISS, at_k.step(NISS / HPC, ns), at_v.step(NISS, nv)) {
+      uint32_t j = q;
+      for (; j < n_jobs; j += NISS, at_k.step(NISS / HPC, ns), at_v.step(NISS, nv)) {
         const uint32_t it = j / HPC, g = j % HPC, bi = j % NGRP, k = j / NGRP, s = at_k.slot(ns);
         wait(full_bar + at_k.i, at_k.phase);
         if (new_row && it == n_iter - 1) wait(&patched_bar, 0);  // the new row is in place
@@ -668,9 +698,11 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
         // and its slot is occupied for one load latency instead of the load latency plus the whole job.
         if (j >= v_pre) {
           if (j >= nv) wait(v_empty + (at_v.i < nv ? at_v.i + nv : at_v.i - nv), at_v.i < nv ? at_v.phase ^ 1u : at_v.phase);
-          if (!abort_s) issue_v(j, at_v.slot(nv), v_full + at_v.i);
+          if (abort_s) break;
+          issue_v(j, at_v.slot(nv), v_full + at_v.i);
         }
       }
+      v_end_s[q] = j;
     }
   } else if (warp < 1 + 2 * NISS) {
     // ---------------- PV issuers: O^T[dim][(block, byte row, head)] (+)= V tile x P'^T ----------------
@@ -971,6 +1003,9 @@ decode_umma_kernel(const CUtensorMap* __restrict__ maps, const __grid_constant__
 
   tc_fence_before();
   __syncthreads();
+  if (abort_s) {  // (unless a wait gave up every copy has landed and every MMA is complete: the accumulate warps have seen the last)
+    wind_down(warp >= 1 && warp < 1 + 2 * NISS, &drained, full_bar, k_end_s, ns, v_full, v_end_s, nv, v_pre, new_row ? (n_iter - 1) * HPC : n_jobs, n_jobs, &v_last);
+  }
   if (warp == 1) tmem_dealloc(tmem, TMEM_COLS);
   if (p.dbg != nullptr && threadIdx.x == 0) {  // development aid: span of the launch in ns
     unsigned long long t_exit_ns;

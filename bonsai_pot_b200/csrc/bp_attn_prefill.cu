@@ -190,6 +190,24 @@ __global__ void __launch_bounds__(256) prefill_expand_kernel(const uint8_t* __re
   *reinterpret_cast<uint4*>(out) = w;
 }
 
+// The end of a CTA whose waits gave up: when it returns the MMAs of its first `issuers` warps are complete and its copies
+// have landed, which were the first k_end and v_end tiles. All threads.
+__device__ __noinline__ void wind_down(uint32_t issuers, uint64_t* drained, uint64_t* k_full, uint64_t* v_full, uint32_t slots, uint32_t k_end, uint32_t v_end) {
+  if (threadIdx.x == 0) {
+    mbar_init(smem_u32(drained), issuers);
+    fence_barrier_init();
+  }
+  __syncthreads();
+  if ((threadIdx.x >> 5) < issuers && elect_one()) umma_commit(smem_u32(drained));  // (the threads that issued them)
+  if (threadIdx.x == 0) {
+    (void)mbar_wait(smem_u32(drained), 0, DRAIN_LIMIT);
+    // the last tile of every slot: the one before it had landed when the slot was given back
+    for (uint32_t i = k_end > slots ? k_end - slots : 0; i < k_end; i++) (void)mbar_wait(smem_u32(&k_full[i % slots]), (i / slots) & 1, DRAIN_LIMIT);
+    for (uint32_t i = v_end > slots ? v_end - slots : 0; i < v_end; i++) (void)mbar_wait(smem_u32(&v_full[i % slots]), (i / slots) & 1, DRAIN_LIMIT);
+  }
+  __syncthreads();
+}
+
 template <uint32_t NQ, uint32_t CPS, bool PX>  // PX: with the peer exchange in the epilogue (an instance of its own: the plain one pays nothing)
 __global__ void __launch_bounds__(PLayout<NQ, CPS>::THREADS, CPS)
 prefill_umma_kernel(const CUtensorMap* __restrict__ maps, const PrefillParams p) {
@@ -200,8 +218,9 @@ prefill_umma_kernel(const CUtensorMap* __restrict__ maps, const PrefillParams p)
   __shared__ __align__(8) uint64_t k_full[L::KV_SLOTS], v_full[L::KV_SLOTS];
   __shared__ __align__(8) uint64_t k_empty[NQ][L::KV_SLOTS], v_empty[NQ][L::KV_SLOTS];  // per query tile: it is done with the slot
   __shared__ __align__(8) uint64_t s_ready[NQ][2], p_ready[NQ][2], p_free[NQ][2], o_done[NQ];
+  __shared__ __align__(8) uint64_t drained;
   __shared__ uint32_t tmem_base_s, item_s;
-  __shared__ volatile uint32_t abort_s;
+  __shared__ volatile uint32_t abort_s, k_end_s, v_end_s;  // a loader that gave up has requested tiles up to here, over all items
 
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -228,6 +247,7 @@ prefill_umma_kernel(const CUtensorMap* __restrict__ maps, const PrefillParams p)
       mbar_init(smem_u32(&o_done[x]), 1);
     }
     abort_s = 0;
+    k_end_s = v_end_s = UINT32_MAX;
     fence_barrier_init();
   }
   if (warp == 1) tmem_alloc(smem_u32(&tmem_base_s), L::TMEM_COLS);
@@ -343,7 +363,7 @@ prefill_umma_kernel(const CUtensorMap* __restrict__ maps, const PrefillParams p)
               }
             }
           }
-          if (!slot_free) return false;
+          if (!slot_free || abort_s) return false;  // (who gives up releases a slot whose tile may still be on its way)
           pend |= users;
           uint64_t* full = is_k ? &k_full[s] : &v_full[s];
           mbar_arrive_expect_tx(smem_u32(full), KV_TILE_B);
@@ -352,7 +372,7 @@ prefill_umma_kernel(const CUtensorMap* __restrict__ maps, const PrefillParams p)
           li++;
           return true;
         };
-        while ((lk < n_tiles || lv < n_tiles || ip < n_pv) && !abort_s) {
+        while (lk < n_tiles || lv < n_tiles || ip < n_pv) {
           bool progressed = false;
           if (lk < n_tiles) progressed |= try_load(true, lk, pend_k, phase_k);
           if (lv < n_tiles) progressed |= try_load(false, lv, pend_v, phase_v);
@@ -376,10 +396,16 @@ prefill_umma_kernel(const CUtensorMap* __restrict__ maps, const PrefillParams p)
           }
           if (progressed) {
             spins = 0;
+          } else if (abort_s) {
+            break;
           } else if (++spins > p.wait_limit) {  // bounded like every other wait (a round is a few dozen cycles)
             abort_s = 1;
             atomicExch(p.err, 5u);
           }
+        }
+        if (abort_s) {
+          if (do_k && k_end_s == UINT32_MAX) k_end_s = gkv + lk;
+          if (do_v && v_end_s == UINT32_MAX) v_end_s = gkv + lv;
         }
       }
     } else if (warp < L::FIRST_SM_WARP) {
@@ -571,6 +597,8 @@ prefill_umma_kernel(const CUtensorMap* __restrict__ maps, const PrefillParams p)
   }
   tc_fence_before();
   __syncthreads();
+  if (abort_s)  // (unless a wait gave up every tile has landed and every MMA is complete: o_done of the last item)
+    wind_down(L::FIRST_SM_WARP, &drained, k_full, v_full, L::KV_SLOTS, min(k_end_s, gkv), min(v_end_s, gkv));
   if (warp == 1) tmem_dealloc(tmem, L::TMEM_COLS);
 }
 

@@ -67,6 +67,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
   }
   return false;
 }
+// Polls for what a CTA that gives up still has on its way (its copies, its MMAs) before it ends: the next CTA on the SM
+// gets the same shared memory and TMEM. What is waited for there always comes, so the limit is not the caller's.
+constexpr uint32_t DRAIN_LIMIT = 1u << 20;
 
 // Tiled TMA loads global -> this CTA's shared memory, completion on an mbarrier.
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar,

@@ -382,3 +382,60 @@ def test_rings_of_any_size_give_the_same_bits_with_two_heads_per_cta(ring):
                 assert torch.equal(token(at).view(torch.int16), ref.view(torch.int16))
         torch.cuda.synchronize()
         assert not ctx.status()
+
+
+@pytest.mark.parametrize("call,rows,options", [
+    ("layer", 200, {}), ("layer", 4000, {}), ("layer", 30000, {}), ("layer", 30000, {"decode_umma_heads_per_cta": 2}), ("layer", 30000, {"decode_ring": 0x35}),
+    ("token", 300, {}), ("token", 30000, {}), ("prefill", 60, {}), ("prefill", 700, {"prefill_tiles_per_item": 2}), ("prefill", 2000, {"prefill_tiles_per_item": 1}),
+    ("prefill", 2000, {"prefill_tiles_per_item": 3})])
+def test_attention_whose_wait_runs_out_winds_down_and_latches(call, rows, options):
+    """One poll: CTAs of the tcgen05 attention kernels give up with their copies and MMAs in flight, and end only when
+    both are complete. The launches behind them find shared memory and TMEM free, the context reports BP_ERR_TIMEOUT
+    from then on, and a fresh one on the same device gives the bits of an undisturbed one."""
+    n_layer, max_seq = 5, 30000
+    g = torch.Generator(device="cuda").manual_seed(7)
+    rand = lambda *shape: torch.randn(*shape, generator=g, device="cuda").half()
+    w = torch.ones(128, dtype=torch.float16, device="cuda")
+    rows_kv = rand(2, 5000, 8 * 128)
+    new_q, new_k, new_v = rand(n_layer, 32 * 128), rand(n_layer, 8 * 128), rand(n_layer, 8 * 128)
+    batch_q = rand(rows, 32 * 128) if call == "prefill" else None
+    outs = []
+    for disturbed in (False, True, False):
+        with bp.AttnContext(n_layer=n_layer, max_seq=max_seq, max_prefill=2048) as ctx:
+            for il in range(n_layer):
+                for r0 in range(0, max_seq, 5000):
+                    ctx.dispatch_kv_writeback_fused(il, rows_kv[0], rows_kv[1], w, r0, 5000)
+            torch.cuda.synchronize()
+            for name, value in options.items():
+                ctx.set_option(name, value)
+            if disturbed:
+                ctx.set_option("wait_limit", 1)
+
+            def work():
+                if call == "layer":
+                    out = torch.zeros(n_layer, ctx.q_dim, dtype=torch.float16, device="cuda")
+                    for il in range(n_layer):
+                        ctx.decode_layer(il, new_q[il], w, new_k[il], new_v[il], w, rows - 1, out[il])
+                elif call == "token":
+                    out = torch.zeros(n_layer, ctx.q_dim, dtype=torch.float16).pin_memory()
+                    ctx.decode_token_host(*(host(x) for x in (new_q, new_k, new_v, w, w)), rows - 1, out.numpy())
+                else:
+                    out = torch.zeros(n_layer, rows, ctx.q_dim, dtype=torch.float16, device="cuda")
+                    for il in range(n_layer):
+                        ctx.dispatch_attention(il, batch_q, out[il], rows)
+                torch.cuda.synchronize()
+                return out
+
+            if disturbed:
+                try:  # the first call may return before the kernel has stored its code
+                    work()
+                except bp.DeviceTimeout:
+                    pass
+                assert ctx.status() == bp.errors.BP_ERR_TIMEOUT
+                with pytest.raises(bp.DeviceTimeout):
+                    work()
+            else:
+                outs.append(host(work().cuda()).view(np.uint16))
+                assert ctx.status() == 0
+    for out in outs[1:]:
+        assert np.array_equal(out, outs[0])
