@@ -889,7 +889,8 @@ __global__ void __launch_bounds__(MMA_THREADS, 1) matmul_q1_q8_mma_kernel(const 
 //                     reference's order, accumulated in registers over all blocks
 //   warp 0, lane 0    per sub-block two tcgen05.mma kind::f16 (M 128, N 128, K 16) into one of two TMEM
 //                     buffers of 2 x 128 columns, one step ahead of the workers
-// Every wait is bounded; a wait that gives up stores a code in the error word and the CTA winds down.
+// Every wait is bounded; a wait that gives up stores a code in the error word and the CTA winds down: it ends only when
+// its own MMAs are complete, because the next CTA on the SM gets the same shared memory and TMEM.
 constexpr uint32_t UM_STAGES = 4, UM_TILE_B = 16384, UM_STAGE_B = 2 * UM_TILE_B;
 constexpr uint32_t UM_EPI_WARPS = 16;
 constexpr uint32_t UM_THREADS = (1 + UM_EPI_WARPS) * 32;
@@ -901,7 +902,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1) matmul_q1_q8_umma_kernel(const 
                                                                           const int8_t* __restrict__ a_qs, __half* y, uint32_t accumulate,
                                                                           uint32_t* err, uint32_t wait_limit) {
   extern __shared__ uint8_t um_raw[];
-  __shared__ __align__(8) uint64_t full[UM_STAGES], empty[UM_STAGES], d_full[2], d_empty[2];
+  __shared__ __align__(8) uint64_t full[UM_STAGES], empty[UM_STAGES], d_full[2], d_empty[2], drained;
   __shared__ uint2 s_sign[16];
   __shared__ __align__(16) float s_wd[UM_EPI_WARPS][32];
   __shared__ uint32_t tmem_base_s;
@@ -939,6 +940,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1) matmul_q1_q8_umma_kernel(const 
   pdl_wait();
   // try_wait with a suspend-time hint: sixteen warps polling at full rate would take issue slots from
   // the warps that are computing
+  const uint32_t poll_ns = min(wait_limit, 2000u);  // (a limit of a few polls is short in time too)
   auto waitb = [&](uint64_t* bar, uint32_t parity) {
     if (abort_s) return;
     const uint32_t addr = smem_u32(bar);
@@ -949,7 +951,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1) matmul_q1_q8_umma_kernel(const 
           "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
           "selp.u32 %0, 1, 0, p;\n\t}"
           : "=r"(ok)
-          : "r"(addr), "r"(parity), "r"(2000u)
+          : "r"(addr), "r"(parity), "r"(poll_ns)
           : "memory");
       if (ok) return;
     }
@@ -1091,6 +1093,15 @@ __global__ void __launch_bounds__(UM_THREADS, 1) matmul_q1_q8_umma_kernel(const 
   }
   tc_fence_before();
   __syncthreads();
+  if (abort_s) {  // the workers have not seen the last MMAs complete: the thread that issued them waits for them
+    if (tid == 0) {
+      mbar_init(smem_u32(&drained), 1);
+      fence_barrier_init();
+      umma_commit(smem_u32(&drained));
+      (void)mbar_wait(smem_u32(&drained), 0, DRAIN_LIMIT);
+    }
+    __syncthreads();
+  }
   if (warp == 0) tmem_dealloc(tmem, 512);
 }
 

@@ -439,3 +439,31 @@ def test_attention_whose_wait_runs_out_winds_down_and_latches(call, rows, option
                 assert ctx.status() == 0
     for out in outs[1:]:
         assert np.array_equal(out, outs[0])
+
+
+@pytest.mark.parametrize("m", [1, 130, 512])
+def test_forced_tcgen05_product_whose_wait_runs_out_winds_down_and_latches(tmp_path, m):
+    """One poll of a nanosecond in the product of the untiled activations: its CTAs end only when their MMAs are
+    complete, the model reports BP_ERR_TIMEOUT, and a fresh one gives the bits of an undisturbed one."""
+    d = str(tmp_path / "m")
+    model_dir.write_synthetic_model(d, seed=4)
+    prompt = [(11 * i + 1) % 2000 for i in range(m)]
+    rows = []
+    lib = _lib.load()
+    lib.bp_op_set_matmul_variant(3)
+    try:
+        for disturbed in (False, True, False):
+            with bp.Model(d, max_seq=512) as gm:
+                if disturbed:
+                    gm.attention().set_option("matmul_wait_limit", 1)
+                    for _ in range(2):
+                        with pytest.raises(bp.DeviceTimeout):
+                            gm.prefill_topk(prompt)
+                    assert gm.attention().status() == bp.errors.BP_ERR_TIMEOUT
+                else:
+                    gm.prefill_topk(prompt)
+                    rows.append((gm.logits(), gm.hidden(0), gm.hidden(m - 1)))
+    finally:
+        lib.bp_op_set_matmul_variant(0)
+    for a, b in zip(*rows):
+        assert np.array_equal(a.view(np.uint16), b.view(np.uint16))
