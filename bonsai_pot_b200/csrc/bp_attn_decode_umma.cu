@@ -1170,8 +1170,12 @@ cudaError_t bp_launch_decode_umma(bp_attn_ctx* c, cudaStream_t s, uint32_t layer
 // (bp_decode_token_host): a call per layer is a chain of 36 kernels whose two ends, about 7 us, stream nothing; a launch
 // over the layers' (layer, KV head) pairs streams through them (36 layers at 4096 keys, call from and to pinned host
 // memory: 360 us as a chain in a graph, 122 here, 98 with the buffers used in place). Pairs that fill the device are not
-// split at all; those that are left over, or all of a small shard's, are split as far as every CTA is resident (the merge
-// makes them wait for one another).
+// split at all; all of a small shard's are split as far as every CTA is resident (the merge makes them wait for one
+// another). What whole waves of layers leave over is split in a launch of its own where two splits or more are resident:
+// us per call, 148 SMs x 8 KV heads, one launch / two: 20 layers (16 CTAs left) 214 / 162 at 16384 keys and 393 / 269 at
+// 32768, 27 layers (72 left) 220 / 210 and 405 / 350, though 87 / 94 and 91 / 105 at 4096. Left over in larger numbers they
+// would be split no further there and would only wait for the first launch: 28 layers (80 left) 93 / 102 at 4096, 220 / 234
+// at 16384, 415 / 430 at 32768.
 // Plain launches: the cache is settled, so every row is requested at once.
 bool bp_decode_layers_batched(const bp_attn_ctx* c) {
   return bp_use_umma(c) && c->opt_uhpc == 1 && c->n_px == 0 && c->opt_umerge && c->opt_exclusive &&
@@ -1189,12 +1193,12 @@ cudaError_t bp_launch_decode_layers(bp_attn_ctx* c, cudaStream_t s, const __half
   }
   for (uint32_t il = 0; il < c->cfg.n_layer;) {
     uint32_t layers = c->cfg.n_layer - il, splits = 1;
-    const uint32_t ctas = layers * groups, tail = ctas % fit;
+    const uint32_t ctas = layers * groups, whole = ctas / fit * fit / groups, rest = (layers - whole) * groups;
     if (ctas <= fit) {
       splits = fit / ctas;
       if (splits > (n_st + 1) / 2) splits = (n_st + 1) / 2;  // two stages are one split, as in umma_spp
-    } else if (tail != 0 && tail * 4 < fit * 3) {
-      layers = (ctas - tail) / groups;  // whole waves; the rest is split over the device in the next launch
+    } else if (rest != 0 && rest * 2 <= fit) {
+      layers = whole;  // the rest is split over the device in the next launch
     }
     const uint32_t spp = (n_st + splits - 1) / splits;
     splits = (n_st + spp - 1) / spp;

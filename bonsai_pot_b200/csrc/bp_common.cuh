@@ -232,8 +232,9 @@ cudaError_t bp_launch_decode_fused(bp_attn_ctx* c, cudaStream_t s, uint32_t laye
                                    const __half* w_q, const __half* k_cur, const __half* v_cur, const __half* w_k,
                                    uint32_t pos, __half* out, uint32_t* launches);
 // The fused steps of every layer at row cur_pos - 1 in as few launches as the device allows; q, out, fs.k_cur and fs.v_cur
-// hold a row per layer. Worth it from BP_BATCHED_PAIRS (layer, KV head) pairs on: with fewer, a launch leaves most of the
-// device idle or splits every head as the calls per layer do.
+// hold a row per layer. Taken from BP_BATCHED_PAIRS (layer, KV head) pairs on: at 32 pairs a call over 4096 keys takes 42 us
+// (4 layers of 8 heads) and 43 (32 of 1) where a graph of calls per layer takes 76 and 283. The line lies on the safe side:
+// with 8 pairs, too, it is 39 against 56 and 38 against 108.
 constexpr uint32_t BP_BATCHED_PAIRS = 32;
 bool bp_decode_layers_batched(const bp_attn_ctx* c);
 cudaError_t bp_launch_decode_layers(bp_attn_ctx* c, cudaStream_t s, const __half* q, __half* out, uint32_t cur_pos, const bp_fused_step& fs,

@@ -608,6 +608,13 @@ def test_token_host_over_all_layers_agrees_with_a_call_per_layer(n_layer, n_kv, 
         assert np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("n_layer,n_kv,launches", [(27, 8, 2), (28, 8, 1), (32, 8, 1), (40, 4, 2)])
+def test_token_host_splits_off_a_last_wave_only_where_its_pairs_can_be_split(n_layer, n_kv, launches):
+    """On 148 SMs: 18 whole layers and 72 pairs in two splits; 80 and 112 pairs, of which two splits would not be resident,
+    stay in the one launch; 37 layers of 4 heads and 12 pairs."""
+    test_token_host_over_all_layers_agrees_with_a_call_per_layer(n_layer, n_kv, launches)
+
+
 def test_token_host_takes_any_pinned_buffers_to_the_same_bits():
     """Where q, k, v and out lie must not matter, overlapping (288 pairs: the first CTAs store outputs before the last
     have read their inputs), off the kernel's 8-byte reads, or pinned only in part: as from separate pageable buffers."""
