@@ -1083,8 +1083,9 @@ uint32_t bp_decode_umma_splits(const bp_attn_ctx* c, uint32_t cur_pos) {
   return (n_st + spp - 1) / spp;
 }
 
+// The ring sizes of a launch with splits of up to spp stages; returns its dynamic shared memory.
 template <uint32_t HPC>
-static cudaError_t launch_umma(bp_attn_ctx* c, cudaStream_t s, UmmaParams& p, uint32_t spp, uint32_t n_splits) {
+static size_t umma_ring(const bp_attn_ctx* c, UmmaParams& p, uint32_t spp) {
   uint32_t cap = umma_max_stages<HPC>();
   uint32_t v_cap = cap * HPC > U_MAX_STAGES ? U_MAX_STAGES : cap * HPC;
   if (c->opt_uring != 0) {  // tuning override: K stages * 16 + V slots, accepted when it fits
@@ -1096,7 +1097,12 @@ static cudaError_t launch_umma(bp_attn_ctx* c, cudaStream_t s, UmmaParams& p, ui
   }
   p.nk = spp < cap ? spp : cap;
   p.nv = spp * HPC < v_cap ? spp * HPC : v_cap;
-  const size_t smem = ULayout<HPC>::total(p.nk, p.nv);
+  return ULayout<HPC>::total(p.nk, p.nv);
+}
+
+template <uint32_t HPC>
+static cudaError_t launch_umma(bp_attn_ctx* c, cudaStream_t s, UmmaParams& p, uint32_t spp, uint32_t n_splits) {
+  const size_t smem = umma_ring<HPC>(c, p, spp);
   dim3 grid(n_splits, c->cfg.n_kv_head / HPC);
   // Short launches (up to 16 splits of up to 4 stages) are merged by one CTA per head group, longer
   // ones by all CTAs of the group.
@@ -1213,14 +1219,11 @@ cudaError_t bp_launch_decode_layers(bp_attn_ctx* c, cudaStream_t s, const __half
     p.fresh_from = UINT32_MAX;
     p.ll = c->ll_layers;
     p.epochs = reinterpret_cast<uint32_t*>(c->ll_layers + ll_units);
-    const uint32_t cap = umma_max_stages<1>();
-    p.nk = spp < cap ? spp : cap;
-    p.nv = p.nk;
+    const size_t smem = umma_ring<1>(c, p, spp);
     for (uint32_t i = 0; i < layers; i++) bp_note_row_write(c, il + i, cur_pos - 1);
     bp_note_sm_launch(c, splits * groups * layers);
     *launches += 1;
-    cudaError_t e = bp_launch(false, decode_umma_kernel<1, 1, true>, dim3(splits, groups, layers), dim3(U_THREADS), ULayout<1>::total(p.nk, p.nv), s,
-                              c->umaps_dev, p);
+    cudaError_t e = bp_launch(false, decode_umma_kernel<1, 1, true>, dim3(splits, groups, layers), dim3(U_THREADS), smem, s, c->umaps_dev, p);
     if (e != cudaSuccess) return e;
     il += layers;
   }

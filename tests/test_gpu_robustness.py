@@ -384,6 +384,34 @@ def test_rings_of_any_size_give_the_same_bits_with_two_heads_per_cta(ring):
         assert not ctx.status()
 
 
+@pytest.mark.parametrize("n_layer,ctx_len", [(36, 8000), (8, 26000)])
+def test_all_layers_launch_takes_rings_of_any_size_to_the_same_bits(n_layer, ctx_len):
+    """Unsplit heads of 63 stages, two CTAs after the other on an SM, and heads in two splits of 102."""
+    with bp.AttnContext(n_layer=n_layer, max_seq=ctx_len) as ctx:
+        g = torch.Generator(device="cuda").manual_seed(8)
+        w = torch.ones(128, dtype=torch.float16, device="cuda")
+        rand = lambda *shape: torch.randn(*shape, generator=g, device="cuda").half()
+        for il in range(n_layer):
+            for r0 in range(0, ctx_len, 2000):
+                ctx.dispatch_kv_writeback_fused(il, rand(2000, ctx.kv_dim), rand(2000, ctx.kv_dim), w, r0, 2000)
+        bufs = [rand(n_layer, n).cpu().pin_memory().numpy() for n in (ctx.q_dim, ctx.kv_dim, ctx.kv_dim)]
+        out = torch.zeros(n_layer, ctx.q_dim, dtype=torch.float16).pin_memory().numpy()
+
+        def token(pos):
+            ctx.decode_token_host(*bufs, host(w), host(w), pos, out)
+            return out.view(np.uint16).copy()
+
+        for pos in (ctx_len - 200, ctx_len - 1):  # (a token writes its row)
+            token(pos)
+        want = [token(pos) for pos in (ctx_len - 1, ctx_len - 200)]
+        for ring in (0x11, 0x24, 0x33, 0x35, 0x53, 0x88):  # (the last does not fit: the default)
+            ctx.set_option("decode_ring", ring)
+            for _ in range(3):
+                for pos, ref in zip((ctx_len - 1, ctx_len - 200), want):
+                    assert np.array_equal(token(pos), ref), hex(ring)
+        assert not ctx.status()
+
+
 @pytest.mark.parametrize("call,rows,options", [
     ("layer", 200, {}), ("layer", 4000, {}), ("layer", 30000, {}), ("layer", 30000, {"decode_umma_heads_per_cta": 2}), ("layer", 30000, {"decode_ring": 0x35}),
     ("token", 300, {}), ("token", 30000, {}), ("prefill", 60, {}), ("prefill", 700, {"prefill_tiles_per_item": 2}), ("prefill", 2000, {"prefill_tiles_per_item": 1}),
