@@ -1088,9 +1088,11 @@ template <uint32_t HPC>
 static size_t umma_ring(const bp_attn_ctx* c, UmmaParams& p, uint32_t spp) {
   uint32_t cap = umma_max_stages<HPC>();
   uint32_t v_cap = cap * HPC > U_MAX_STAGES ? U_MAX_STAGES : cap * HPC;
-  if (c->opt_uring != 0) {  // tuning override: K stages * 16 + V slots, accepted when it fits
+  // tuning override: K stages * 16 + V slots, accepted when it fits (a fused step patches the new row into the V tiles of all
+  // HPC heads of the last stage: they are in their slots together)
+  if (c->opt_uring != 0) {
     const uint32_t k = c->opt_uring >> 4, v = c->opt_uring & 15;
-    if (k >= 1 && v >= 1 && k <= U_MAX_STAGES && v <= U_MAX_STAGES && ULayout<HPC>::total(k, v) <= U_SMEM_BUDGET) {
+    if (k >= 1 && v >= HPC && k <= U_MAX_STAGES && v <= U_MAX_STAGES && ULayout<HPC>::total(k, v) <= U_SMEM_BUDGET) {
       cap = k;
       v_cap = v;
     }

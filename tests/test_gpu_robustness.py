@@ -384,6 +384,13 @@ def test_rings_of_any_size_give_the_same_bits_with_two_heads_per_cta(ring):
         assert not ctx.status()
 
 
+@pytest.mark.parametrize("ring", [0x11, 0x41])
+def test_a_ring_of_one_v_slot_is_not_taken_for_two_heads_per_cta(ring):
+    """The last stage's V tiles of both heads have to be in their slots together before the new row is patched in: with
+    one slot the second was waited for without end, and the step gave up. The default ring runs instead."""
+    test_rings_of_any_size_give_the_same_bits_with_two_heads_per_cta(ring)
+
+
 @pytest.mark.parametrize("n_layer,ctx_len", [(36, 8000), (8, 26000)])
 def test_all_layers_launch_takes_rings_of_any_size_to_the_same_bits(n_layer, ctx_len):
     """Unsplit heads of 63 stages, two CTAs after the other on an SM, and heads in two splits of 102."""
