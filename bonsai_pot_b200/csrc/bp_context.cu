@@ -6,7 +6,6 @@
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
-#include <sys/mman.h>
 
 #include <algorithm>
 #include <mutex>
@@ -857,8 +856,8 @@ static cudaError_t shard_copy(void* host_row0, size_t pitch, size_t col, uint8_t
 // and two pinned buffers of SNAP_CHUNK, whose DMA runs under the host copy of the other buffer. A lane is made when a
 // snapshot first needs it and belongs to the context. Sharded contexts (strided rows) and the smallest payloads take
 // plain copies. 36 layers, capture / restore in us: 16 rows (1.3 MB) 607 / 590 (plain copies 1900 / 1800), 100 rows
-// 921 / 823, 512 rows (42 MB) 2575 / 1907; the capture 5800 before its fresh pages were asked for as huge ones. Eight
-// lanes: 512 rows 2206 / 1814, 100 rows 919 / 907.
+// 921 / 823, 512 rows (42 MB) 2575 / 1907 (a capture into fresh pages that are not huge ones 5800: who makes the buffer
+// asks for them). Eight lanes: 512 rows 2206 / 1814, 100 rows 919 / 907.
 constexpr uint32_t SNAP_LANES = 4;
 constexpr size_t SNAP_CHUNK = 1u << 20, SNAP_LANES_MIN = 64u << 10, SNAP_PER_LANE = 1u << 20;
 struct bp_snap_lanes {
@@ -957,11 +956,6 @@ static cudaError_t snap_transfer(bp_attn_ctx* c, uint8_t* payload, uint32_t pos,
   if (!l) return cudaSuccess;
   std::lock_guard<std::mutex> g(l->busy);
   if (!make_snap_lanes(l, lanes)) return cudaSuccess;
-  if (to_host) {  // a capture fills a fresh buffer: whole huge pages of it in one fault each (a wish: no matter if it fails)
-    constexpr uintptr_t HUGE = 2u << 20;
-    const uintptr_t from = (reinterpret_cast<uintptr_t>(payload) + HUGE - 1) & ~(HUGE - 1), to = (reinterpret_cast<uintptr_t>(payload) + bytes) & ~(HUGE - 1);
-    if (from < to) (void)madvise(reinterpret_cast<void*>(from), to - from, MADV_HUGEPAGE);
-  }
   // Ordered as a plain copy on the default stream is: behind what the blocking streams hold.
   cudaError_t e = cudaEventRecord(l->done[0][0], cudaStreamLegacy);
   if (e == cudaSuccess) e = cudaEventSynchronize(l->done[0][0]);

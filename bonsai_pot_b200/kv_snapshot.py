@@ -5,6 +5,7 @@ reference's value type around them."""
 from __future__ import annotations
 
 import ctypes as C
+import mmap
 import struct
 
 from . import _lib
@@ -28,13 +29,21 @@ def payload_offset(n_layer, kv_dim, pos, kind, il, sect):
 # Prototypes of this module's own: the attributes of `ctypes.pythonapi` are shared with everything else in the process.
 _bytes_new = C.PYFUNCTYPE(C.py_object, C.c_char_p, C.c_ssize_t)(("PyBytes_FromStringAndSize", C.pythonapi))
 _bytes_address = C.PYFUNCTYPE(C.c_void_p, C.py_object)(("PyBytes_AsString", C.pythonapi))
+_madvise = C.CFUNCTYPE(C.c_int, C.c_void_p, C.c_size_t, C.c_int)(("madvise", C.CDLL(None)))
+_HUGE_PAGE = 2 << 20
 
 
 def new_blob(size):
     """An uninitialised `bytes` object and the address of its bytes, for a call that fills it: a capture then
-    touches every page of the blob once (zeroing a buffer and copying it out took longer than the transfer)."""
+    touches every page of the blob once (zeroing a buffer and copying it out took longer than the transfer). Its whole
+    huge pages come in one fault each if the system grants the wish (a capture of 42 MB 5800 -> 2575 us); asked for here
+    because this memory is the blob's own, where a buffer handed to the C entry is its caller's."""
     blob = _bytes_new(None, size)
-    return blob, _bytes_address(blob)
+    address = _bytes_address(blob)
+    first, last = -(-address // _HUGE_PAGE) * _HUGE_PAGE, (address + size) // _HUGE_PAGE * _HUGE_PAGE
+    if first < last:
+        _madvise(first, last - first, mmap.MADV_HUGEPAGE)
+    return blob, address
 
 
 class KvSnapshot:

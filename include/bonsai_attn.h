@@ -227,9 +227,12 @@ uint64_t bp_snapshot_size(const bp_attn_ctx* ctx, uint32_t pos);
  * On a sharded context the blob is written in the GLOBAL row order: header
  * kv_dim = n_shards * local kv_dim, and only this shard's columns of each row
  * are touched, so n_shards calls on the same buffer assemble the full blob.
- * The first blob of 2 MB or more that an unsharded context captures or applies
- * makes four streams and 8 MB of pinned host memory that stay with the context
- * until it is destroyed (without them, plain copies); four threads then copy. */
+ * A payload of 64 KB or more of an unsharded context, captured or applied, goes
+ * through one to four lanes, one more per MB: each a stream and 2 MB of pinned host
+ * memory, made when first needed, that stay with the context until it is destroyed
+ * (plain copies where one cannot be made), and a thread while the call lasts. Most
+ * of a capture into fresh memory is the page faults of the blob: huge pages help,
+ * and are its caller's to ask for (madvise). */
 int bp_snapshot_capture(bp_attn_ctx* ctx, uint32_t pos, void* blob, uint64_t blob_bytes);
 /* `KvSnapshot::from_bytes` + `validate_against` + `kv_snapshot::apply`
  * (src/kv_snapshot.rs:104-140, 184-199, 312-372). Returns the restored `pos`

@@ -4,6 +4,7 @@ the one-token forward pass with the GPU's attention outputs fed to the CPU pass 
 the residual stream and the logits is exact while attention keeps its own tolerance); and the session
 behaviour the reference tests in tests/gpu_integration.rs."""
 import ctypes as C
+import mmap
 import os
 
 import numpy as np
@@ -540,6 +541,38 @@ def test_large_snapshots_hold_the_cache_rows(pos):
         assert snap.apply(other) == pos
         assert snap.payload == b"".join(sections(other))
         assert bp.KvSnapshot.from_bytes(snap.to_bytes()).clone().payload == snap.payload
+
+
+@pytest.mark.parametrize("pos", [14, 15, 227, 228, 682, 683])
+def test_snapshots_around_the_lines_between_one_and_more_lanes(pos):
+    """4608 bytes a row here: lanes from 64 KB (15 rows) on, one more from 1 MB (228 rows) and from 2 and 3 MB on."""
+    test_large_snapshots_hold_the_cache_rows(pos)
+
+
+def test_a_capture_leaves_the_callers_memory_as_it_was():
+    """The C entry fills a buffer that belongs to its caller: no advice on its pages stays behind (flag hg of the mapping)."""
+    with bp.AttnContext(n_layer=4, n_head=16, n_kv_head=4, max_seq=2048) as ctx, mmap.mmap(-1, 16 << 20, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS) as buf:
+        size = int(_lib.load().bp_snapshot_size(ctx._h, 2048))
+        assert 4 << 20 < size < 16 << 20
+        at = C.addressof(C.c_char.from_buffer(buf))
+
+        def flags():
+            with open("/proc/self/smaps") as f:
+                inside, found = False, []
+                for line in f:
+                    head = line.split()[0]
+                    if "-" in head and not head.endswith(":"):
+                        lo, hi = (int(x, 16) for x in head.split("-"))
+                        inside = lo < at + (16 << 20) and at < hi
+                    elif inside and head == "VmFlags:":
+                        found.append("hg" in line.split()[1:])
+                return found
+
+        assert flags() and not any(flags())
+        ctx._check(_lib.load().bp_snapshot_capture(ctx._h, 2048, at, size))
+        assert flags() and not any(flags())
+        assert buf[:8] == b"BONSAIKV"
+
 
 
 @pytest.mark.parametrize("k,n", [(3072, 17), (3200, 17), (4096, 4096), (4096 + 128, 600), (4096 + 128, 4096), (6272, 4096), (8192, 15),
