@@ -634,6 +634,21 @@ def test_tiled_product_is_identical_to_the_cuda_core_product(tmp_path, m):
             assert np.array_equal(a.view(np.uint8), b.view(np.uint8)), variant
 
 
+# (A tile of the product is 128 weight rows high, whatever its width, and widths are counted in tokens.)
+@pytest.mark.parametrize("m", [1, 15, 16, 17, 32, 47, 48, 49, 63, 64, 65, 95, 96, 97, 145, 512])
+def test_tiled_product_in_every_forced_token_width_at_its_edges(tmp_path, m):
+    """128, 48, 96, 64, 32 and 16 tokens per tile, each with counts one below, at and one above a whole tile of some
+    width: hidden rows of the first, a middle and the last token, and the logits, as the dp4a path's."""
+    d = str(tmp_path / "m")
+    model_dir.write_synthetic_model(d, shape=RAGGED, seed=14)
+    prompt = [(17 * i + 3) % 500 for i in range(m)]
+    rows = (0, m // 2, m - 1)
+    want = prefill_rows(d, prompt, 1, rows)
+    for variant in (6, 7, 8, 9, 10, 11):
+        for a, b in zip(want, prefill_rows(d, prompt, variant, rows)):
+            assert np.array_equal(a.view(np.uint16), b.view(np.uint16)), variant
+
+
 @pytest.mark.parametrize("n_ff,m", [(9600, 1), (9600, 33), (9600, 128), (12288, 65), (12288, 100), (6400, 300), (6400, 257)])
 def test_last_wave_of_the_tiled_product_is_identical_in_narrow_tiles(tmp_path, n_ff, m):
     """Tiles of 128 tokens whose last wave on 148 SMs is cut into tiles of 32 (150 = 148 + 2 and 300 = 2 x 148 + 4 of

@@ -304,6 +304,29 @@ def test_batched_product_whose_wait_runs_out_winds_down_and_latches(tmp_path, m)
         assert np.array_equal(a.view(np.uint16), b.view(np.uint16))
 
 
+@pytest.mark.parametrize("n_ff,m", [(9600, 128), (12288, 100)])
+def test_batched_product_with_a_cut_last_wave_winds_down_and_latches(tmp_path, n_ff, m):
+    """The same where the gate and up tiles of the last wave on 148 SMs are cut, into tiles of 32 and of 64 tokens: CTAs of
+    both widths of one kernel give up."""
+    d = str(tmp_path / "m")
+    model_dir.write_synthetic_model(d, shape=dict(n_layer=1, n_embd=256, n_ff=n_ff, n_head=4, n_kv_head=1, head_dim=128, n_vocab=512), seed=12)
+    prompt = [(13 * i + 5) % 500 for i in range(m)]
+    rows = []
+    for disturbed in (False, True, False):
+        with bp.Model(d, max_seq=512) as gm:
+            if disturbed:
+                gm.attention().set_option("matmul_wait_limit", 1)
+                for _ in range(2):
+                    with pytest.raises(bp.DeviceTimeout):
+                        gm.prefill_topk(prompt)
+                assert gm.attention().status() == bp.errors.BP_ERR_TIMEOUT
+            else:
+                gm.prefill_topk(prompt)
+                rows.append((gm.logits(), gm.hidden(0), gm.hidden(m - 1)))
+    for a, b in zip(*rows):
+        assert np.array_equal(a.view(np.uint16), b.view(np.uint16))
+
+
 def test_batched_product_does_not_count_the_time_of_the_kernels_before_it(tmp_path):
     """The second layer's Q/K/V product (16 blocks, more than its stages) starts under the first layer's down product of 768
     blocks, some 450 us. A limit of 48 polls, some 4 us each, is ample for what the product itself waits for (8 polls are
