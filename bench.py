@@ -517,8 +517,9 @@ def run_ours(args):
                 gh.copy_(out_full, non_blocking=True)
             stream.synchronize()
     if mode != "nccl":  # (the host entry point has no per-layer meeting kernel: the ranks meet once per token)
-        # Successive positions, as a generation loop asks for them, ending at the benchmark's context length
-        # (the library prepares its launches for the next position while the device works on the current one).
+        # Successive positions, as a generation loop asks for them, ending at the benchmark's context length.
+        # The call has every layer's activations before the first layer runs. From 32 (layer, KV head) pairs on, without
+        # a peer exchange, the library then runs the layers side by side: another work than `value`'s dependent layers.
         e_steps = max(5, args.steps)
         first = max(0, pos - (e_steps + 3 - 1))
         at = [min(pos, first + i) for i in range(e_steps + 3)]
@@ -537,6 +538,8 @@ def run_ours(args):
                        "ms_per_step": round(e_dt * 1e3, 4),
                        "positions": f"{at[3]} .. {at[-1]}",
                        "call": "bp_decode_token_host (pinned host activations in, f16 outputs back, one sync per token)" +
+                               ("" if use_px or N_LAYER * nkv_l < 32 else "; all layers' activations are given at once and the layers run "
+                                "side by side, not one after the other as in `value`") +
                                ("; then the meeting and the gathered rows back to the host, on every rank" if use_px else "")}
     if rank == 0 and world == 1:
         # ---- the other configurations, briefly ----

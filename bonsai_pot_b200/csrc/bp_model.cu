@@ -385,7 +385,9 @@ cudaError_t attention_call(bp_model* m, uint32_t il, uint32_t pos) {
 // attn_nodes: the launches are being captured into the step's graph, and it receives the attention launches with their nodes.
 // Which launches carry programmatic stream serialization, us per step of the 8B shape as a graph, position 100 / 900: all
 // but Wo 1150 / 1233, all four matvecs 1152 / 1236, all but Wo and Q/K/V 1165 / 1260, gate + up only (the choice for the
-// 8-lane matvecs, whose second wave the down projection's early CTAs kept waiting) 1208 / 1302, none 1237 / 1328.
+// 8-lane matvecs, whose second wave the down projection's early CTAs kept waiting) 1208 / 1302, none 1237 / 1328. As stream
+// launches (taps, no step graph): all but Wo 1275 / 1347, all but the down projection (the choice there before) 1316 / 1385,
+// all four 1208 / 1281, gate + up only 1455 / 1529, none 1567 / 1638.
 int decode_layer(bp_model* m, uint32_t il, uint32_t pos, std::vector<bp_launch_record>* attn_nodes = nullptr) {
   const Config& c = m->cfg;
   const LayerTensors& lt = m->layers[il];

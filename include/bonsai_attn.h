@@ -276,7 +276,8 @@ int bp_set_variant(bp_attn_ctx* ctx, uint32_t variant);
  * before every token, the default; 0 = a stream launch per layer), "decode_in_kernel_merge"
  * (1 = the tcgen05 decode kernel merges its splits itself, the default; 0 = a
  * second kernel does), "decode_ring" (K stages * 16 + V slots of the tcgen05
- * decode kernel, 0 = as many as fit), "decode_v_preload" (1 = the first round of
+ * decode kernel, 0 = as many as fit, also where the given numbers do not fit or there are
+ * fewer V slots than heads per CTA), "decode_v_preload" (1 = the first round of
  * V tiles is requested during set-up, the default), "tma_l2_promotion" (0 = 256 B,
  * the default, 1 = 128 B, 2 = 64 B, 3 = none). Results do not depend on any of
  * them beyond rounding. The in-kernel merge keeps per-context state on the device
