@@ -608,7 +608,7 @@ def test_warp_per_row_matvec_is_identical_to_eight_lanes_per_row(k, n):
         assert np.array_equal(a.view(np.uint16), b.view(np.uint16))
 
 
-# heights that no tile width divides (n_ff = 640: 128 + 112 + .. leave remainders; K and V have 128 rows)
+# heights of one to five row tiles (a tile of the product is 128 weight rows high and 16 to 128 tokens wide)
 RAGGED = dict(n_layer=1, n_embd=384, n_ff=640, n_head=4, n_kv_head=1, head_dim=128, n_vocab=512)
 
 
@@ -634,7 +634,6 @@ def test_tiled_product_is_identical_to_the_cuda_core_product(tmp_path, m):
             assert np.array_equal(a.view(np.uint8), b.view(np.uint8)), variant
 
 
-# (A tile of the product is 128 weight rows high, whatever its width, and widths are counted in tokens.)
 @pytest.mark.parametrize("m", [1, 15, 16, 17, 32, 47, 48, 49, 63, 64, 65, 95, 96, 97, 145, 512])
 def test_tiled_product_in_every_forced_token_width_at_its_edges(tmp_path, m):
     """128, 48, 96, 64, 32 and 16 tokens per tile, each with counts one below, at and one above a whole tile of some
